@@ -338,3 +338,102 @@ def tolerance(case):
     if kind == "step":
         return {"rel": 2.5e-2, "max": 0.55}
     return {"rel": 1e-4, "max": 3e-2, "differ": 1e-4}
+
+
+# ---------------------------------------------------------------------------- the same in 64 bits
+def exact(case, seed):
+    """What :func:`run` returns, in plain 64-bit torch: linear layers, attention and the double
+    quantisation's scales.  A training step has no such value (a whole model with its optimizer),
+    nor have whole codes and what hangs on the choice of one."""
+    if case["kind"] == "step":
+        return None
+    state = prepare(case, seed)
+    return {"linear": _exact_linear, "attention": _exact_attention, "nf4": _exact_nf4}[case["kind"]](case, state)
+
+
+def _keep_mask(rows, cols, p, seed):
+    """Philox4x32-7 with key ``seed`` over counters (row, column / 8, 0, 0): sixteen bits an element,
+    kept where they reach ``round(p * 65536)``."""
+    low = 0xFFFFFFFF
+    c = [rows[:, None].expand(-1, cols // 8), torch.arange(cols // 8, device=DEVICE)[None, :].expand(len(rows), -1)]
+    c += [torch.zeros_like(c[0]), torch.zeros_like(c[0])]
+    k0, k1 = seed & low, seed >> 32 & low
+    for _ in range(7):
+        p0, p1 = c[0] * 0xD2511F53, c[2] * 0xCD9E8D57
+        c = [p1 >> 32 & low ^ c[1] ^ k0, p1 & low, p0 >> 32 & low ^ c[3] ^ k1, p0 & low]
+        k0, k1 = (k0 + 0x9E3779B9) & low, (k1 + 0xBB67AE85) & low
+    lanes = torch.stack([c[j // 2] >> 16 * (j % 2) & 0xFFFF for j in range(8)], dim=-1)
+    return (lanes >= round(p * 65536)).reshape(len(rows), cols)
+
+
+def _nf4_values(q):
+    """64-bit values of a quantised weight: table value times the scale of its block of 64."""
+    table = torch.tensor([-1.0, -0.6961928009986877, -0.5250730514526367, -0.39491748809814453, -0.28444138169288635,
+                          -0.18477343022823334, -0.09105003625154495, 0.0, 0.07958029955625534, 0.16093020141124725,
+                          0.24611230194568634, 0.33791524171829224, 0.44070982933044434, 0.5626170039176941,
+                          0.7229568362236023, 1.0], dtype=torch.float64, device=DEVICE)
+    codes = torch.stack([q.packed >> 4, q.packed & 15], dim=-1).reshape(-1, 64)
+    nested = q.nested.double().repeat_interleave(256)[:len(codes)]
+    scales = q.code256.double()[q.absmax_q.long()] * nested + float(q.offset)
+    return (table[codes.long()] * scales[:, None]).reshape(q.shape)
+
+
+def _exact_linear(case, state):
+    seg, ranks, rates = _ints(case["segments"]), _ints(case["ranks"]), _floats(case["dropout"])
+    w = _nf4_values(state["w"]) if case["nf4"] else state["w"].double()
+    x = state["x"].detach().double()
+    y = x @ w.t()
+    if state["bias"] is not None:
+        y += state["bias"].double()
+    back = case["backward"]
+    if back:
+        dy = state["dy"].double()
+        dx, da, db = dy @ w, [], []
+    start = 0
+    for i, s in enumerate(seg):
+        rows = slice(start, start + (s if len(seg) == 1 else (s + TILE - 1) // TILE * TILE))
+        start, alpha, p = rows.stop, 32.0 / ranks[i], rates[i]
+        a, b = state["a"][i].detach().double(), state["b"][i].detach().double()
+        keep = 1.0
+        if p > 0:
+            keep = _keep_mask(torch.arange(rows.start, rows.stop, device=DEVICE), case["k"], p, state["seed"]) / (1.0 - p)
+        dropped = x[rows] * keep
+        low = alpha * (dropped @ a.t())
+        y[rows] += low @ b.t()
+        if back:
+            d_low = alpha * (dy[rows] @ b)
+            db.append(dy[rows].t() @ low)
+            da.append(d_low.t() @ dropped)
+            dx[rows] += (d_low @ a) * keep
+    return {"y": y, "grads": (dx, *da, *db)} if back else {"y": y}
+
+
+def _exact_attention(case, state):
+    heads, kv, d = case["heads"], case["kv_heads"], HEAD_DIM
+    qkv = state["qkv"].detach().double()
+    out = torch.empty(len(qkv), heads * d, dtype=torch.float64, device=DEVICE)
+    grad = torch.zeros_like(qkv)
+    start = 0
+    for n in _lengths(case["tokens"], case["median"], 1):
+        rows = slice(start, start + n)
+        start += n
+        above = torch.ones(n, n, dtype=torch.bool, device=DEVICE).triu(1)
+        for h in range(heads):
+            cols = [slice(c * d, (c + 1) * d) for c in (h, heads + h * kv // heads, heads + kv + h * kv // heads)]
+            q, k, v = (qkv[rows, c] for c in cols)
+            p = ((q @ k.t()) / math.sqrt(d)).masked_fill_(above, -math.inf).softmax(-1)
+            out[rows, cols[0]] = p @ v
+            if case["backward"]:
+                do = state["d_out"][rows, cols[0]].double()
+                grad[rows, cols[2]] += p.t() @ do
+                ds = p * (do @ v.t() - (do * out[rows, cols[0]]).sum(-1, keepdim=True)) / math.sqrt(d)
+                grad[rows, cols[0]] = ds @ k
+                grad[rows, cols[1]] += ds.t() @ q
+    return {"out": out, "grads": (grad,)} if case["backward"] else {"out": out}
+
+
+def _exact_nf4(case, state):
+    absmax = state["w"].double().reshape(-1, 64).abs().amax(1)
+    off = absmax - absmax.mean()
+    nested = torch.nn.functional.pad(off, (0, -len(off) % 256)).reshape(-1, 256).abs().amax(1)
+    return {"packed": None, "scales": None, "nested": nested.clamp_min(1e-12), "w": None}
