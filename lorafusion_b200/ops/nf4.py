@@ -15,6 +15,7 @@ A pure-PyTorch implementation of both directions is the CPU oracle.
 
 from __future__ import annotations
 
+import functools
 from dataclasses import dataclass
 from typing import Optional
 
@@ -96,7 +97,24 @@ def _nearest_code(x: torch.Tensor, code: torch.Tensor) -> torch.Tensor:
     return torch.bucketize(x, mids.to(x.device), right=False)
 
 
+@functools.lru_cache(maxsize=None)
+def _code_table(device: torch.device):
+    """The 256 second-level code values and the 255 midpoints between them, constants of a device."""
+    code = dynamic_code_8bit()
+    return code.to(device), ((code[:-1] + code[1:]) / 2).to(device)
+
+
 def _double_quantize(absmax: torch.Tensor):
+    if absmax.is_cuda and absmax.numel() > 0:
+        code, mids = _code_table(absmax.device)
+        n = absmax.numel()
+        q = torch.empty(n, dtype=torch.uint8, device=absmax.device)
+        nested = torch.empty(-(-n // NESTED_BLOCK), dtype=torch.float32, device=absmax.device)
+        scratch = torch.empty(149, dtype=torch.float64, device=absmax.device)   # 148 partial sums, the mean
+        mean = scratch[148:].view(torch.float32)[:1]
+        nv.call("lf_nf4_double_quantize", absmax.data_ptr(), n, scratch.data_ptr(), mids.data_ptr(), q.data_ptr(),
+                nested.data_ptr(), mean.data_ptr(), nv.current_stream_ptr())
+        return q, code, nested, float(mean)
     code = dynamic_code_8bit().to(absmax.device)
     offset = float(absmax.mean())
     centered = absmax - offset
