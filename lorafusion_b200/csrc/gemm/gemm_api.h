@@ -30,7 +30,7 @@ typedef struct LfGemmArgs {
   const void* b2;  // slab B operand
   int64_t b2_rows, b2_cols, b2_ld;
   const int32_t* tile_adapter;  // adapter id per 128-row M tile (dense mode), <0 = none; may be null
-  const int32_t* seg_tiles;     // segment mode: int4 {m0, k0, num_k_blocks, adapter} per tile
+  const int32_t* seg_tiles;     // lf_lora_skinny: int4 {adapter, first token, end token, 0} per segment
   void* out;
   int64_t ldo;
   int64_t out_adapter_stride;   // elements between adapters in `out` (F32_ACCUM)
@@ -108,6 +108,16 @@ int lf_gemm_nf4(const LfGemmArgs* args, const LfNf4Args* nf4);
 // Tensor-parallel fused variants reading an NF4 weight shard (see lf_gemm_tp and lf_gemm_nf4).
 int lf_gemm_tp_nf4(const LfGemmArgs* args, const LfTpArgs* tp, const LfNf4Args* nf4);
 
+// The rank-wide LoRA products (see lora_skinny.cu); `split` CTAs share the reduction of a tile.
+int lf_lora_skinny(const LfGemmArgs* args, int split);
+
 #ifdef __cplusplus
+}
+#endif
+
+#ifdef __cplusplus
+// Rows of eight or more bf16 columns are written 16 bytes at a time.
+inline bool gemm_out_aligned(const LfGemmArgs* a) {
+  return a->N < 8 || ((reinterpret_cast<uintptr_t>(a->out) & 15) == 0 && (a->M <= 1 || a->ldo % 8 == 0));
 }
 #endif

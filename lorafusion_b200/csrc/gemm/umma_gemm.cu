@@ -6,16 +6,14 @@
 //                                           over the rank dimension, adapter chosen per
 //                                           128-row tile)           -- reference K4/K5/K9
 //   * dX       dX = dY W + keep (.) (dS A_a) / (1 - p)              -- reference K6/K7/K10
-//   * the skinny LoRA products S' = a * drop(X) A_a^T, dS = a * dY B_a, dB, dA, with the
-//     dropout mask regenerated from Philox inside shared memory (never stored)
-//                                           -- reference K1-K3, K8, K11 and cuBLAS calls
+// (the rank-wide LoRA products live in lora_skinny.cu)
 // (file:line citations of the reference live in lorafusion_b200/ops/lora.py).
 //
 // Roles inside a CTA (1 CTA per SM, grid = min(#tiles, #SMs)):
 //   warp 0      : TMA producer (one elected lane)
 //   warp 1      : TMEM allocator + single-thread tcgen05.mma issuer
 //   warps 2..5  : epilogue (each warp owns one 32-lane TMEM quarter)
-//   warps 6..13 : only when MASK_A: apply the dropout mask to the A stage in place
+//   warps 6..13 : only with an NF4 weight: expand the B stage in place
 // Accumulators are double-buffered in TMEM so the epilogue of tile i overlaps the main loop
 // of tile i+1.
 #include <stdio.h>
@@ -31,24 +29,16 @@ namespace lf {
 
 constexpr int BM = 128;
 constexpr int BK = 64;
-constexpr int kNumMaskWarps = 8;
-// The dropout warps work in groups on DIFFERENT stages at the same time: one stage's rewrite is a
-// chain of latencies (barrier poll, shared-memory load, seven Philox rounds, store, proxy fence),
-// and eight warps on one stage at a time left the kernel bound by that chain, not by issue slots.
-constexpr int kMaskGroups = 4;
+constexpr int kNumExpandWarps = 8;
 
 struct GemmKParams {
   int M, N;
   int nkb_main, nkb2;
   int num_m_tiles, num_n_tiles, num_tiles, group_m;
   const int* tile_adapter;
-  const int4* seg_tiles;
-  int b_adapter_rows, b2_adapter_rows;
+  int b2_adapter_rows;
   void* out;
   long long ldo;
-  long long out_adapter_stride;
-  int out_transposed;
-  const float* adapter_scale;
   float scale;
   const __nv_bfloat16* bias;
   const uint32_t* adapter_thresh16;
@@ -57,7 +47,7 @@ struct GemmKParams {
   float inv_keep;
   uint32_t seed_lo, seed_hi, stream_id;
   int row_offset, col_offset;
-  int m_rotate;  // dense mode: M tiles are visited starting from this tile (wraps around)
+  int m_rotate;  // M tiles are visited starting from this tile (wraps around)
   int* err;
   // NF4 main loop: fp32 scale of every 64-element block of the [nf4_rows, 64 * blocks] weight
   const float* nf4_scales;
@@ -85,20 +75,11 @@ __constant__ float kNf4Values[16] = {
 //           with the GEMM, pull the partials of the rows this rank owns from every source with
 //           coalesced peer loads as their flags arrive and sum them in fp32 (+ residual).
 struct TileCoord {
-  int m0, n0, k0, nkb, adapter;
+  int m0, n_tile, adapter;
 };
 
 __device__ __forceinline__ TileCoord decode_tile(const GemmKParams& p, int idx) {
   TileCoord t;
-  if (p.seg_tiles != nullptr) {
-    const int4 s = p.seg_tiles[idx];
-    t.m0 = s.x;
-    t.n0 = 0;
-    t.k0 = s.y;
-    t.nkb = s.z;
-    t.adapter = s.w;
-    return t;
-  }
   const int per_group = p.group_m * p.num_n_tiles;
   const int g = idx / per_group;
   const int first_m = g * p.group_m;
@@ -109,9 +90,7 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmKParams& p, int idx) 
   m_tile += p.m_rotate;
   if (m_tile >= p.num_m_tiles) m_tile -= p.num_m_tiles;
   t.m0 = m_tile * BM;
-  t.n0 = n_tile;  // multiplied by BN by the caller (BN is a template constant there)
-  t.k0 = 0;
-  t.nkb = p.nkb_main;
+  t.n_tile = n_tile;
   t.adapter = (p.tile_adapter != nullptr) ? p.tile_adapter[m_tile] : 0;
   return t;
 }
@@ -123,29 +102,25 @@ struct SmemPlan {
   // NF4 variant: the packed 4-bit B tile lands behind the bf16 tile it is expanded into
   static constexpr int PACK_BYTES = NF4B ? BN * BK / 2 : 0;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES + PACK_BYTES;
-  static constexpr int STAGES = (BN == 256) ? 4 : (BN == 192 ? 5 : (BN == 128 ? 6 : 8));
+  static constexpr int STAGES = BN == 256 ? 4 : 6;
   static constexpr int BAR_BYTES = 512;
   static constexpr int TOTAL = STAGES * STAGE_BYTES + BAR_BYTES + 1024;  // + alignment slack
 };
 
 
-template <int BN, int NACC, bool A_MN, bool B_MN, bool B2_MN, int EPI, bool MASK_A, int TP = 0,
-          bool NF4B = false>
-__global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps : 0) +
+template <int BN, int NACC, bool B_MN, bool B2_MN, int EPI, int TP = 0, bool NF4B = false>
+__global__ void __launch_bounds__(192 + (NF4B ? 32 * kNumExpandWarps : 0) +
                                       (TP != 0 ? 32 * kNumCommWarps : 0), 1)
     umma_gemm_kernel(const GemmKParams p, const __grid_constant__ CUtensorMap tmA,
                      const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmA2,
                      const __grid_constant__ CUtensorMap tmB2, const TpParams tp) {
-  static_assert(!(MASK_A && TP != 0), "dropout-in-smem and TP fusion are not combined");
-  static_assert(!NF4B || (BN == 256 && !MASK_A && !A_MN),
-                "the NF4 main loop exists for 256-wide dense tiles only");
+  static_assert(!NF4B || BN == 256, "the NF4 main loop exists for 256-wide tiles only");
   // Thread layout: warp 0 TMA, warp 1 MMA, warps 2-5 epilogue, then (if any) the eight warps
-  // that rewrite a stage (dropout mask or NF4 expansion), then (if any) the four warps that
-  // move data between GPUs.  COMM_T0 = first thread of the latter.
-  constexpr int COMM_T0 = 192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps : 0);
+  // that expand an NF4 stage, then (if any) the four warps that move data between GPUs.
+  // COMM_T0 = first thread of the latter.
+  constexpr int COMM_T0 = 192 + (NF4B ? 32 * kNumExpandWarps : 0);
   using Plan = SmemPlan<BN, NF4B>;
-  constexpr bool XFORM = MASK_A || NF4B;  // extra warps rewrite a stage before the MMA reads it
   __shared__ float nf4_lut[16];
   if (NF4B && threadIdx.x < 16) nf4_lut[threadIdx.x] = kNf4Values[threadIdx.x];
   constexpr int STAGES = Plan::STAGES;
@@ -176,8 +151,7 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
-      // lane 0 of every warp that rewrites the stage reports for its warp
-      mbar_init(&ready[s], MASK_A ? kNumMaskWarps / kMaskGroups : kNumMaskWarps);
+      mbar_init(&ready[s], kNumExpandWarps);  // lane 0 of every expanding warp reports for its warp
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull[b], 1);
@@ -208,11 +182,10 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
       bool ok = true;
       for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
         TileCoord t = decode_tile(p, tile);
-        const int n0 = (p.seg_tiles != nullptr) ? 0 : t.n0 * BN;
+        const int n0 = t.n_tile * BN;
         const int nkb2 = (t.adapter >= 0) ? p.nkb2 : 0;
-        const int by = (t.adapter >= 0) ? t.adapter * p.b_adapter_rows : 0;
         const int by2 = (t.adapter >= 0) ? t.adapter * p.b2_adapter_rows : 0;
-        const int nkb = (t.adapter < 0 && p.b_adapter_rows > 0) ? 0 : t.nkb;
+        const int nkb = p.nkb_main;
         const int total = nkb + nkb2;
         if (TP == 1) {
           const int mt = t.m0 / BM;
@@ -238,13 +211,8 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
           mbar_expect_tx(&full[s], (NF4B && kb < nkb) ? Plan::A_BYTES + Plan::PACK_BYTES
                                                        : Plan::A_BYTES + Plan::B_BYTES);
           if (kb < nkb) {
-            const int kk = t.k0 + kb * BK;
-            if (!A_MN) {
-              tma_load_2d(sA, &tmA, &full[s], kk, t.m0);
-            } else {
-              tma_load_2d(sA, &tmA, &full[s], t.m0, kk);
-              tma_load_2d(sA + 8192, &tmA, &full[s], t.m0 + 64, kk);
-            }
+            const int kk = kb * BK;
+            tma_load_2d(sA, &tmA, &full[s], kk, t.m0);
             if (NF4B) {
               // packed bytes (two codes each): K-major W -> [256 rows x 32 B],
               // MN-major W -> [64 rows x 128 B]; tmB is a byte map here
@@ -252,11 +220,11 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
               if (!B_MN) tma_load_2d(sP, &tmB, &full[s], kk >> 1, n0);
               else tma_load_2d(sP, &tmB, &full[s], n0 >> 1, kk);
             } else if (!B_MN) {
-              tma_load_2d(sB, &tmB, &full[s], kk, by + n0);
+              tma_load_2d(sB, &tmB, &full[s], kk, n0);
             } else {
 #pragma unroll
               for (int h = 0; h < BN / 64; ++h)
-                tma_load_2d(sB + h * 8192, &tmB, &full[s], n0 + 64 * h, by + kk);
+                tma_load_2d(sB + h * 8192, &tmB, &full[s], n0 + 64 * h, kk);
             }
           } else {
             const int kk2 = (kb - nkb) * BK;
@@ -275,7 +243,7 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
     if (lane == 0) {
-      constexpr uint32_t IDESC_MAIN = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      constexpr uint32_t IDESC_MAIN = make_idesc_bf16(BM, BN, 0, B_MN ? 1 : 0);
       constexpr uint32_t IDESC_SLAB = make_idesc_bf16(BM, BN, 0, B2_MN ? 1 : 0);
       int it = 0;
       int tile_iter = 0;
@@ -283,7 +251,7 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
       for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x, ++tile_iter) {
         TileCoord t = decode_tile(p, tile);
         const int nkb2 = (t.adapter >= 0) ? p.nkb2 : 0;
-        const int nkb = (t.adapter < 0 && p.b_adapter_rows > 0) ? 0 : t.nkb;
+        const int nkb = p.nkb_main;
         const int total = nkb + nkb2;
         const int buf = tile_iter % NBUF;
         const uint32_t bph = (tile_iter / NBUF) & 1;
@@ -297,8 +265,8 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
         for (int kb = 0; kb < total; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(XFORM ? &ready[s] : &full[s], ph, ctx,
-                         XFORM ? ERR_WAIT_READY : ERR_WAIT_FULL)) {
+          if (!mbar_wait(NF4B ? &ready[s] : &full[s], ph, ctx,
+                         NF4B ? ERR_WAIT_READY : ERR_WAIT_FULL)) {
             ok = false;
             break;
           }
@@ -306,13 +274,11 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
           const uint32_t sA = smem_u32(smem + s * Plan::STAGE_BYTES);
           const uint32_t sB = sA + Plan::A_BYTES;
           const bool slab = kb >= nkb;
-          const bool a_mn = slab ? false : A_MN;
           const bool b_mn = slab ? B2_MN : B_MN;
           const uint32_t d = (NACC == 2 && slab) ? acc1 : acc0;
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = a_mn ? make_smem_desc_sw128(sA + kk * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(sA + kk * 32, 16, 1024);
+            const uint64_t da = make_smem_desc_sw128(sA + kk * 32, 16, 1024);
             const uint64_t db = b_mn ? make_smem_desc_sw128(sB + kk * 2048, 8192, 1024)
                                      : make_smem_desc_sw128(sB + kk * 32, 16, 1024);
             const uint32_t accum =
@@ -336,10 +302,9 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
     bool ok = true;
     for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x, ++tile_iter) {
       TileCoord t = decode_tile(p, tile);
-      const int n0 = (p.seg_tiles != nullptr) ? 0 : t.n0 * BN;
+      const int n0 = t.n_tile * BN;
       const int nkb2 = (t.adapter >= 0) ? p.nkb2 : 0;
-      const int nkb = (t.adapter < 0 && p.b_adapter_rows > 0) ? 0 : t.nkb;
-      const bool has_work = (nkb + nkb2) > 0;
+      const bool has_work = (p.nkb_main + nkb2) > 0;
       const bool has_slab = nkb2 > 0;
       const int buf = tile_iter % NBUF;
       const uint32_t bph = (tile_iter / NBUF) & 1;
@@ -358,11 +323,6 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
       const uint32_t acc0 = tmem_base + uint32_t(buf * BN * NACC) + lane_addr;
       const uint32_t acc1 = acc0 + BN;
 
-      float tile_scale = p.scale;
-      if (EPI == LF_EPI_BF16_ADAPTER_SCALE) {
-        tile_scale = (t.adapter >= 0 && p.adapter_scale != nullptr) ? p.adapter_scale[t.adapter]
-                                                                    : (t.adapter >= 0 ? p.scale : 0.f);
-      }
       uint32_t thresh = p.thresh16;
       float inv_keep = p.inv_keep;
       if (EPI == LF_EPI_BF16_DROPMIX && t.adapter >= 0 && p.adapter_thresh16 != nullptr) {
@@ -383,70 +343,54 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
           for (int j = 0; j < 32; ++j) r[j] = 0u;
         }
         const int col0 = n0 + c * 32;
-        if (EPI == LF_EPI_F32_ACCUM) {
-          if (has_work && row < p.M) {
-            float* out = reinterpret_cast<float*>(p.out) +
-                         (t.adapter >= 0 ? t.adapter * p.out_adapter_stride : 0);
+        float v[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int col = col0 + j;
-              if (col < p.N) {
-                float* dst = p.out_transposed ? (out + (long long)col * p.ldo + row)
-                                              : (out + (long long)row * p.ldo + col);
-                *dst += tile_scale * __uint_as_float(r[j]);
-              }
-            }
-          }
-        } else {
-          float v[32];
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.scale;
+        if (EPI == LF_EPI_BF16_DROPMIX) {
+          if (NACC == 2 && has_slab) {
+            if (thresh == 0) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * tile_scale;
-          if (EPI == LF_EPI_BF16_DROPMIX) {
-            if (NACC == 2 && has_slab) {
-              if (thresh == 0) {
+              for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(r2[j]);
+            } else {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(r2[j]);
-              } else {
+              for (int g = 0; g < 4; ++g) {
+                const uint32_t keep =
+                    dropout_keep8(uint32_t(row + p.row_offset),
+                                  uint32_t((col0 + p.col_offset) >> 3) + g, p.stream_id,
+                                  p.seed_lo, p.seed_hi, thresh);
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                  const uint32_t keep =
-                      dropout_keep8(uint32_t(row + p.row_offset),
-                                    uint32_t((col0 + p.col_offset) >> 3) + g, p.stream_id,
-                                    p.seed_lo, p.seed_hi, thresh);
-#pragma unroll
-                  for (int j = 0; j < 8; ++j)
-                    if ((keep >> j) & 1u) v[g * 8 + j] += inv_keep * __uint_as_float(r2[g * 8 + j]);
-                }
-              }
-            }
-          }
-          if (EPI == LF_EPI_BF16 && p.bias != nullptr) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int col = col0 + j;
-              if (col < p.N) v[j] += __bfloat162float(p.bias[col]);
-            }
-          }
-          if (row < p.M) {
-            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + (long long)row * p.ldo;
-            if (TP == 2) {
-              // partial tiles stay in THIS GPU's stage [M, N]; the owner of the rows pulls them
-              // (row-per-thread stores are merged in the local L2; pushed over NVLink they
-              // would travel as 16-byte writes)
-              out = tp.rs_peer_stage[tp.rank] + (long long)row * p.N;
-            }
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              const int col = col0 + g * 8;
-              if (col + 8 <= p.N) {
-                st_global_v4(out + col, pack_bf16x2(v[g * 8 + 0], v[g * 8 + 1]),
-                             pack_bf16x2(v[g * 8 + 2], v[g * 8 + 3]),
-                             pack_bf16x2(v[g * 8 + 4], v[g * 8 + 5]),
-                             pack_bf16x2(v[g * 8 + 6], v[g * 8 + 7]));
-              } else {
                 for (int j = 0; j < 8; ++j)
-                  if (col + j < p.N) out[col + j] = __float2bfloat16(v[g * 8 + j]);
+                  if ((keep >> j) & 1u) v[g * 8 + j] += inv_keep * __uint_as_float(r2[g * 8 + j]);
               }
+            }
+          }
+        }
+        if (EPI == LF_EPI_BF16 && p.bias != nullptr) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const int col = col0 + j;
+            if (col < p.N) v[j] += __bfloat162float(p.bias[col]);
+          }
+        }
+        if (row < p.M) {
+          __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + (long long)row * p.ldo;
+          if (TP == 2) {
+            // partial tiles stay in THIS GPU's stage [M, N]; the owner of the rows pulls them
+            // (row-per-thread stores are merged in the local L2; pushed over NVLink they
+            // would travel as 16-byte writes)
+            out = tp.rs_peer_stage[tp.rank] + (long long)row * p.N;
+          }
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            const int col = col0 + g * 8;
+            if (col + 8 <= p.N) {
+              st_global_v4(out + col, pack_bf16x2(v[g * 8 + 0], v[g * 8 + 1]),
+                           pack_bf16x2(v[g * 8 + 2], v[g * 8 + 3]),
+                           pack_bf16x2(v[g * 8 + 4], v[g * 8 + 5]),
+                           pack_bf16x2(v[g * 8 + 6], v[g * 8 + 7]));
+            } else {
+              for (int j = 0; j < 8; ++j)
+                if (col + j < p.N) out[col + j] = __float2bfloat16(v[g * 8 + j]);
             }
           }
         }
@@ -462,7 +406,7 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
           const int owner = mt / tp.tiles_per_shard;
           st_release_sys(tp.rs_peer_cnt[owner] +
                              (tp.rank * tp.tiles_per_shard + (mt - owner * tp.tiles_per_shard)) * p.num_n_tiles +
-                             t.n0,
+                             t.n_tile,
                          tp.epoch);
         }
       }
@@ -486,7 +430,7 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
       if (!ok) break;
       tp_reduce_item_any<BM, BN, !NF4B>(tp, et, lt, nt, p.N);
     }
-  } else if (TP == 1 && !MASK_A && int(threadIdx.x) >= COMM_T0) {
+  } else if (TP == 1 && int(threadIdx.x) >= COMM_T0) {
     // ------------- push this rank's token shard to every peer's gathered buffer -------------
     const int ct = threadIdx.x - COMM_T0;  // 0..127
     const int tps = tp.tiles_per_shard;
@@ -572,9 +516,9 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
     bool ok = true;
     for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
       TileCoord t = decode_tile(p, tile);
-      const int n0 = t.n0 * BN;
+      const int n0 = t.n_tile * BN;
       const int nkb2 = (t.adapter >= 0) ? p.nkb2 : 0;
-      const int nkb = t.nkb;
+      const int nkb = p.nkb_main;
       const int total = nkb + nkb2;
       for (int kb = 0; kb < total; ++kb, ++it) {
         const int s = it % STAGES;
@@ -636,73 +580,6 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
         if (lane == 0) mbar_arrive(&ready[s]);
       }
     }
-  } else if (MASK_A) {
-    // ------------------- dropout mask applied to the A stage in place -------------------
-    constexpr int NMT = 32 * kNumMaskWarps / kMaskGroups;  // threads that share one stage
-    const int grp = (threadIdx.x - 192) / NMT;             // this thread's group takes stages grp, grp + kMaskGroups, ...
-    const int mt = (threadIdx.x - 192) % NMT;
-    int it = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
-      TileCoord t = decode_tile(p, tile);
-      const int nkb2 = (t.adapter >= 0) ? p.nkb2 : 0;
-      const int nkb = (t.adapter < 0 && p.b_adapter_rows > 0) ? 0 : t.nkb;
-      const int total = nkb + nkb2;
-      uint32_t thresh = p.thresh16;
-      float inv_keep = p.inv_keep;
-      if (t.adapter >= 0 && p.adapter_thresh16 != nullptr) {
-        thresh = p.adapter_thresh16[t.adapter];
-        inv_keep = p.adapter_inv_keep[t.adapter];
-      }
-      for (int kb = 0; kb < total; ++kb, ++it) {
-        if (it % kMaskGroups != grp) continue;
-        const int s = it % STAGES;
-        const uint32_t ph = (it / STAGES) & 1;
-        // one answer per warp: its lanes meet again in __syncwarp below
-        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, ctx, ERR_WAIT_FULL))) {
-          ok = false;
-          break;
-        }
-        if (kb < nkb && thresh != 0) {
-          uint8_t* sA = smem + s * Plan::STAGE_BYTES;
-          const int kk = t.k0 + kb * BK;
-#pragma unroll
-          for (int i = 0; i < (Plan::A_BYTES / 16) / NMT; ++i) {
-            const int qd = mt + i * NMT;  // 16-byte chunk index inside the A stage
-            int token, feature;
-            if (!A_MN) {
-              const int r = qd >> 3;
-              const int c = (qd & 7) ^ (r & 7);
-              token = t.m0 + r;
-              feature = kk + 8 * c;
-            } else {
-              const int h = qd >> 9;
-              const int kr = (qd & 511) >> 3;
-              const int c = (qd & 7) ^ (kr & 7);
-              token = kk + kr;
-              feature = t.m0 + 64 * h + 8 * c;
-            }
-            const uint32_t keep =
-                dropout_keep8(uint32_t(token + p.row_offset), uint32_t((feature + p.col_offset) >> 3),
-                              p.stream_id, p.seed_lo, p.seed_hi, thresh);
-            uint4* ptr = reinterpret_cast<uint4*>(sA + qd * 16);
-            uint4 x = *ptr;
-            uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              float2 f = unpack_bf16x2(w[j]);
-              f.x = ((keep >> (2 * j)) & 1u) ? f.x * inv_keep : 0.f;
-              f.y = ((keep >> (2 * j + 1)) & 1u) ? f.y * inv_keep : 0.f;
-              w[j] = pack_bf16x2(f.x, f.y);
-            }
-            *ptr = make_uint4(w[0], w[1], w[2], w[3]);
-          }
-          fence_proxy_async_smem();
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ready[s]);
-      }
-    }
   }
 
   // ------------------------------ teardown ------------------------------
@@ -724,12 +601,11 @@ __global__ void __launch_bounds__(192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps :
 // ------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------
-template <int BN, int NACC, bool A_MN, bool B_MN, bool B2_MN, int EPI, bool MASK_A, int TP = 0,
-          bool NF4B = false>
+template <int BN, int NACC, bool B_MN, bool B2_MN, int EPI, int TP = 0, bool NF4B = false>
 static int launch_variant(const GemmKParams& kp, const CUtensorMap& tA, const CUtensorMap& tB,
                           const CUtensorMap& tA2, const CUtensorMap& tB2, int grid,
                           cudaStream_t stream, const TpParams& tp = TpParams()) {
-  auto kern = umma_gemm_kernel<BN, NACC, A_MN, B_MN, B2_MN, EPI, MASK_A, TP, NF4B>;
+  auto kern = umma_gemm_kernel<BN, NACC, B_MN, B2_MN, EPI, TP, NF4B>;
   constexpr int smem = SmemPlan<BN, NF4B>::TOTAL;
   static PerDeviceOnce configured;  // one per template instantiation
   {
@@ -739,7 +615,7 @@ static int launch_variant(const GemmKParams& kp, const CUtensorMap& tA, const CU
       return -10;
     }
   }
-  const int threads = 192 + ((MASK_A || NF4B) ? 32 * kNumMaskWarps : 0) + (TP != 0 ? 32 * kNumCommWarps : 0);
+  const int threads = 192 + (NF4B ? 32 * kNumExpandWarps : 0) + (TP != 0 ? 32 * kNumCommWarps : 0);
   kern<<<grid, threads, smem, stream>>>(kp, tA, tB, tA2, tB2, tp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -786,12 +662,14 @@ extern "C" int lf_gemm_tp_nf4(const LfGemmArgs* a, const LfTpArgs* t, const LfNf
 static int gemm_entry(const LfGemmArgs* a, const LfTpArgs* t, const LfNf4Args* q) {
   using namespace lf;
   if (a == nullptr || a->a == nullptr || a->b == nullptr || a->out == nullptr) return -1;
-  if (a->bn != 64 && a->bn != 128 && a->bn != 192 && a->bn != 256) return -2;
+  if (a->bn != 128 && a->bn != 256) return -2;
+  if (a->a_mn || a->mask_a || a->seg_tiles != nullptr || a->b_adapter_rows != 0) return -5;  // lf_lora_skinny
   if (a->K2 % BK != 0) return -3;
+  if (!gemm_out_aligned(a)) return -6;
   const int BN = a->bn;
   if (q != nullptr) {
-    // whole 64-code blocks per tile row, dense tiles, adapters only on the slab operand
-    if (BN != 256 || a->a_mn || a->mask_a || a->seg_tiles != nullptr || a->b_adapter_rows != 0) return -12;
+    // whole 64-code blocks per tile row
+    if (BN != 256) return -12;
     if (q->w_cols % 256 != 0 || q->w_rows % 64 != 0 || a->K % BK != 0) return -13;
     if (a->b_mn ? (a->N != q->w_cols || a->K != q->w_rows) : (a->N != q->w_rows || a->K != q->w_cols)) return -14;
     if (!a->b_mn && a->N % 256 != 0) return -13;
@@ -799,8 +677,8 @@ static int gemm_entry(const LfGemmArgs* a, const LfTpArgs* t, const LfNf4Args* q
 
   CUtensorMap tA, tB, tA2, tB2;
   int rc;
-  // A: K-major box = [128 rows x 64 cols]; MN-major box = [64 rows(k) x 64 cols(mn)]
-  rc = make_tmap_2d_b16(&tA, a->a, a->a_rows, a->a_cols, a->a_ld, a->a_mn ? 64 : BM, 64, true);
+  // K-major box = [128 (A) or BN (B) rows x 64 cols]; MN-major box = [64 rows(k) x 64 cols(mn)]
+  rc = make_tmap_2d_b16(&tA, a->a, a->a_rows, a->a_cols, a->a_ld, BM, 64, true);
   if (rc != 0) return -20 + rc;
   if (q == nullptr) {
     rc = make_tmap_2d_b16(&tB, a->b, a->b_rows, a->b_cols, a->b_ld, a->b_mn ? 64 : BN, 64, true);
@@ -829,17 +707,12 @@ static int gemm_entry(const LfGemmArgs* a, const LfTpArgs* t, const LfNf4Args* q
   kp.nkb2 = a->K2 / BK;
   kp.num_m_tiles = (a->M + BM - 1) / BM;
   kp.num_n_tiles = (a->N + BN - 1) / BN;
-  kp.seg_tiles = reinterpret_cast<const int4*>(a->seg_tiles);
-  kp.num_tiles = (a->seg_tiles != nullptr) ? a->num_seg_tiles : kp.num_m_tiles * kp.num_n_tiles;
+  kp.num_tiles = kp.num_m_tiles * kp.num_n_tiles;
   kp.group_m = a->group_m > 0 ? a->group_m : 8;
   kp.tile_adapter = a->tile_adapter;
-  kp.b_adapter_rows = a->b_adapter_rows;
   kp.b2_adapter_rows = a->b2_adapter_rows;
   kp.out = a->out;
   kp.ldo = a->ldo;
-  kp.out_adapter_stride = a->out_adapter_stride;
-  kp.out_transposed = a->out_transposed;
-  kp.adapter_scale = a->adapter_scale;
   kp.scale = a->scale;
   kp.bias = reinterpret_cast<const __nv_bfloat16*>(a->bias);
   kp.adapter_thresh16 = a->adapter_thresh16;
@@ -864,7 +737,6 @@ static int gemm_entry(const LfGemmArgs* a, const LfTpArgs* t, const LfNf4Args* q
   cudaStream_t st = reinterpret_cast<cudaStream_t>(a->stream);
 
   if (t != nullptr && t->mode != 0) {
-    if (a->seg_tiles != nullptr || a->mask_a) return -6;
     if (t->world < 1 || t->world > 8 || t->rank < 0 || t->rank >= t->world) return -7;
     if (kp.num_m_tiles != t->world * t->tiles_per_shard) return -8;
     TpParams tp = make_tp_params(t);
@@ -872,23 +744,23 @@ static int gemm_entry(const LfGemmArgs* a, const LfTpArgs* t, const LfNf4Args* q
     kp.m_rotate = (t->mode == 1 ? t->rank : (t->rank + 1) % t->world) * t->tiles_per_shard;
     kp.group_m = t->tiles_per_shard < kp.group_m ? t->tiles_per_shard : kp.group_m;
     const int tkey = (t->mode << 8) | (a->nacc << 4) | ((a->b_mn ? 1 : 0) << 1) | (a->epi == LF_EPI_BF16_DROPMIX);
-    if (BN != 256 || a->a_mn) return -9;
+    if (BN != 256) return -9;
     if (q != nullptr) {
       // NF4 weight expanded inside the main loop of the fused compute + collective kernel
       if (a->K2 > 0 && (a->b2_mn != a->b_mn)) return -5;
       switch (tkey) {
         case (1 << 8) | (1 << 4) | 0:
-          return launch_variant<256, 1, false, false, false, LF_EPI_BF16, false, 1, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
+          return launch_variant<256, 1, false, false, LF_EPI_BF16, 1, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
         case (1 << 8) | (1 << 4) | 2:
-          return launch_variant<256, 1, false, true, true, LF_EPI_BF16, false, 1, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
+          return launch_variant<256, 1, true, true, LF_EPI_BF16, 1, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
         case (1 << 8) | (2 << 4) | 3:
-          return launch_variant<256, 2, false, true, true, LF_EPI_BF16_DROPMIX, false, 1, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
+          return launch_variant<256, 2, true, true, LF_EPI_BF16_DROPMIX, 1, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
         case (2 << 8) | (1 << 4) | 0:
-          return launch_variant<256, 1, false, false, false, LF_EPI_BF16, false, 2, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
+          return launch_variant<256, 1, false, false, LF_EPI_BF16, 2, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
         case (2 << 8) | (1 << 4) | 2:
-          return launch_variant<256, 1, false, true, true, LF_EPI_BF16, false, 2, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
+          return launch_variant<256, 1, true, true, LF_EPI_BF16, 2, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
         case (2 << 8) | (2 << 4) | 3:
-          return launch_variant<256, 2, false, true, true, LF_EPI_BF16_DROPMIX, false, 2, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
+          return launch_variant<256, 2, true, true, LF_EPI_BF16_DROPMIX, 2, true>(kp, tA, tB, tA2, tB2, grid, st, tp);
         default:
           fprintf(stderr, "lf_gemm_tp_nf4: no kernel variant for key 0x%x\n", tkey);
           return -5;
@@ -896,17 +768,17 @@ static int gemm_entry(const LfGemmArgs* a, const LfTpArgs* t, const LfNf4Args* q
     }
     switch (tkey) {
       case (1 << 8) | (1 << 4) | 0:
-        return launch_variant<256, 1, false, false, false, LF_EPI_BF16, false, 1>(kp, tA, tB, tA2, tB2, grid, st, tp);
+        return launch_variant<256, 1, false, false, LF_EPI_BF16, 1>(kp, tA, tB, tA2, tB2, grid, st, tp);
       case (1 << 8) | (1 << 4) | 2:
-        return launch_variant<256, 1, false, true, true, LF_EPI_BF16, false, 1>(kp, tA, tB, tA2, tB2, grid, st, tp);
+        return launch_variant<256, 1, true, true, LF_EPI_BF16, 1>(kp, tA, tB, tA2, tB2, grid, st, tp);
       case (1 << 8) | (2 << 4) | 3:
-        return launch_variant<256, 2, false, true, true, LF_EPI_BF16_DROPMIX, false, 1>(kp, tA, tB, tA2, tB2, grid, st, tp);
+        return launch_variant<256, 2, true, true, LF_EPI_BF16_DROPMIX, 1>(kp, tA, tB, tA2, tB2, grid, st, tp);
       case (2 << 8) | (1 << 4) | 0:
-        return launch_variant<256, 1, false, false, false, LF_EPI_BF16, false, 2>(kp, tA, tB, tA2, tB2, grid, st, tp);
+        return launch_variant<256, 1, false, false, LF_EPI_BF16, 2>(kp, tA, tB, tA2, tB2, grid, st, tp);
       case (2 << 8) | (1 << 4) | 2:
-        return launch_variant<256, 1, false, true, true, LF_EPI_BF16, false, 2>(kp, tA, tB, tA2, tB2, grid, st, tp);
+        return launch_variant<256, 1, true, true, LF_EPI_BF16, 2>(kp, tA, tB, tA2, tB2, grid, st, tp);
       case (2 << 8) | (2 << 4) | 3:
-        return launch_variant<256, 2, false, true, true, LF_EPI_BF16_DROPMIX, false, 2>(kp, tA, tB, tA2, tB2, grid, st, tp);
+        return launch_variant<256, 2, true, true, LF_EPI_BF16_DROPMIX, 2>(kp, tA, tB, tA2, tB2, grid, st, tp);
       default:
         fprintf(stderr, "lf_gemm_tp: no kernel variant for key 0x%x\n", tkey);
         return -5;
@@ -919,55 +791,35 @@ static int gemm_entry(const LfGemmArgs* a, const LfTpArgs* t, const LfNf4Args* q
     switch (qkey) {
       case (1 << 4) | 0:
         if (a->epi != LF_EPI_BF16) return -5;
-        return launch_variant<256, 1, false, false, false, LF_EPI_BF16, false, 0, true>(kp, tA, tB, tA2, tB2, grid, st);
+        return launch_variant<256, 1, false, false, LF_EPI_BF16, 0, true>(kp, tA, tB, tA2, tB2, grid, st);
       case (1 << 4) | 2:
         if (a->epi != LF_EPI_BF16) return -5;
-        return launch_variant<256, 1, false, true, true, LF_EPI_BF16, false, 0, true>(kp, tA, tB, tA2, tB2, grid, st);
+        return launch_variant<256, 1, true, true, LF_EPI_BF16, 0, true>(kp, tA, tB, tA2, tB2, grid, st);
       case (2 << 4) | 3:
-        return launch_variant<256, 2, false, true, true, LF_EPI_BF16_DROPMIX, false, 0, true>(kp, tA, tB, tA2, tB2, grid, st);
+        return launch_variant<256, 2, true, true, LF_EPI_BF16_DROPMIX, 0, true>(kp, tA, tB, tA2, tB2, grid, st);
       default:
         fprintf(stderr, "lf_gemm_nf4: no kernel variant for key 0x%x\n", qkey);
         return -5;
     }
   }
 
-  const int key = (BN << 16) | (a->nacc << 12) | ((a->a_mn ? 1 : 0) << 11) |
-                  ((a->b_mn ? 1 : 0) << 10) | ((a->b2_mn ? 1 : 0) << 9) | (a->epi << 4) |
-                  (a->mask_a ? 1 : 0);
-#define LF_KEY(bn, nacc, amn, bmn, b2mn, epi, mask) \
-  (((bn) << 16) | ((nacc) << 12) | ((amn) << 11) | ((bmn) << 10) | ((b2mn) << 9) | ((epi) << 4) | (mask))
-#define LF_CASE(bn, nacc, amn, bmn, b2mn, epi, mask)                                         \
-  case LF_KEY(bn, nacc, amn, bmn, b2mn, epi, mask):                                          \
-    return launch_variant<bn, nacc, (amn) != 0, (bmn) != 0, (b2mn) != 0, epi, (mask) != 0>(  \
-        kp, tA, tB, tA2, tB2, grid, st);
+  const int key = (BN << 16) | (a->nacc << 12) | ((a->b_mn ? 1 : 0) << 10) | ((a->b2_mn ? 1 : 0) << 9) | (a->epi << 4);
+#define LF_CASE(bn, nacc, bmn, b2mn, epi)                                                                     \
+  case ((bn) << 16) | ((nacc) << 12) | ((bmn) << 10) | ((b2mn) << 9) | ((epi) << 4):                          \
+    return launch_variant<bn, nacc, (bmn) != 0, (b2mn) != 0, epi>(kp, tA, tB, tA2, tB2, grid, st);
   switch (key) {
     // forward base+LoRA and plain NT GEMM
-    LF_CASE(256, 1, 0, 0, 0, LF_EPI_BF16, 0)
-    LF_CASE(128, 1, 0, 0, 0, LF_EPI_BF16, 0)
+    LF_CASE(256, 1, 0, 0, LF_EPI_BF16)
+    LF_CASE(128, 1, 0, 0, LF_EPI_BF16)
     // dX without dropout and plain NN GEMM
-    LF_CASE(256, 1, 0, 1, 1, LF_EPI_BF16, 0)
-    LF_CASE(128, 1, 0, 1, 1, LF_EPI_BF16, 0)
+    LF_CASE(256, 1, 1, 1, LF_EPI_BF16)
+    LF_CASE(128, 1, 1, 1, LF_EPI_BF16)
     // dX with the dropout mask regenerated in the epilogue
-    LF_CASE(128, 2, 0, 1, 1, LF_EPI_BF16_DROPMIX, 0)
-    LF_CASE(256, 2, 0, 1, 1, LF_EPI_BF16_DROPMIX, 0)
-#define LF_SKINNY(bn)                                                \
-    /* S' = alpha * dropout(X) A^T */                                  \
-    LF_CASE(bn, 1, 0, 0, 0, LF_EPI_BF16_ADAPTER_SCALE, 0)              \
-    LF_CASE(bn, 1, 0, 0, 0, LF_EPI_BF16_ADAPTER_SCALE, 1)              \
-    /* dS = alpha * dY B */                                            \
-    LF_CASE(bn, 1, 0, 1, 0, LF_EPI_BF16_ADAPTER_SCALE, 0)              \
-    /* dB += dY^T S'   and   dA += dS^T dropout(X) */                  \
-    LF_CASE(bn, 1, 1, 1, 0, LF_EPI_F32_ACCUM, 0)                       \
-    LF_CASE(bn, 1, 1, 1, 0, LF_EPI_F32_ACCUM, 1)
-    LF_SKINNY(64)
-    LF_SKINNY(128)
-    LF_SKINNY(192)
-    LF_SKINNY(256)
-#undef LF_SKINNY
+    LF_CASE(128, 2, 1, 1, LF_EPI_BF16_DROPMIX)
+    LF_CASE(256, 2, 1, 1, LF_EPI_BF16_DROPMIX)
     default:
       fprintf(stderr, "lf_gemm: no kernel variant for key 0x%x\n", key);
       return -5;
   }
 #undef LF_CASE
-#undef LF_KEY
 }

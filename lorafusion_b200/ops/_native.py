@@ -130,6 +130,8 @@ def _declare_cuda(lib: C.CDLL) -> None:
     lib.lf_gemm.restype = C.c_int
     lib.lf_gemm_pair.argtypes = [C.POINTER(LfGemmArgs)]
     lib.lf_gemm_pair.restype = C.c_int
+    lib.lf_lora_skinny.argtypes = [C.POINTER(LfGemmArgs), C.c_int]
+    lib.lf_lora_skinny.restype = C.c_int
     lib.lf_gemm_nf4.argtypes = [C.POINTER(LfGemmArgs), C.POINTER(LfNf4Args)]
     lib.lf_gemm_nf4.restype = C.c_int
     for name, sig in _SIGNATURES.items():

@@ -22,7 +22,7 @@ from typing import Any, Optional, Sequence
 import numpy as np
 import torch
 
-from .lora_kernels import DropoutSpec, SegmentTable, TILE_M
+from .lora_kernels import DropoutSpec, SegmentTable, TILE_M, segment_rows
 from .philox import dropout_threshold
 
 
@@ -125,12 +125,24 @@ def prepare_multi_lora_batch_info(
     p_arr = np.asarray(dropout_p_list, dtype=np.float64)
     alpha_arr = np.asarray(alpha_list, dtype=np.float64)
 
-    # one staging buffer: int32 words [tile_adapter | lookup (3/blk) | thresh (n_ad)]
-    # followed by fp32 words [scale (n_ad) | inv_keep (n_ad) | blk_p | blk_alpha]
+    segments = []
+    start = 0
+    for i in range(n_seg):
+        if padded[i] > 0:
+            segments.append((int(idx_arr[i]), start, start + int(padded[i])))
+        start += int(padded[i])
+    seg_rows = segment_rows(segments)
+
+    # one staging buffer: int32 words [segment rows (4 each) | tile_adapter | lookup (3/blk) | thresh (n_ad)]
+    # followed by fp32 words [scale (n_ad) | inv_keep (n_ad) | blk_p | blk_alpha]; the segment rows
+    # come first because the kernels read them 16 bytes at a time
+    n_row = 4 * len(seg_rows)
     n_int = n_blk + 3 * n_blk + n_ad
     n_flt = 2 * n_ad + 2 * n_blk
-    stage = torch.empty(n_int + n_flt, dtype=torch.int32,
-                        pin_memory=(device.type == "cuda" and torch.cuda.is_available()))
+    staging = torch.empty(n_row + n_int + n_flt, dtype=torch.int32,
+                          pin_memory=(device.type == "cuda" and torch.cuda.is_available()))
+    stage = staging[n_row:]
+    staging.numpy()[:n_row] = np.asarray(seg_rows, dtype=np.int32).reshape(-1)
     words = stage.numpy()
     fwords = words.view(np.float32)
     words[:n_blk] = idx_arr[seg_of_block] if n_blk else 0
@@ -154,14 +166,9 @@ def prepare_multi_lora_batch_info(
     fwords[n_int + 2 * n_ad:n_int + 2 * n_ad + n_blk] = p_arr[seg_of_block] if n_blk else 0
     fwords[n_int + 2 * n_ad + n_blk:] = alpha_arr[seg_of_block] if n_blk else 0
 
-    dev = stage.to(device, non_blocking=True)
+    moved = staging.to(device, non_blocking=True)
+    dev = moved[n_row:]
     fdev = dev.view(torch.float32)
-    segments = []
-    start = 0
-    for i in range(n_seg):
-        if padded[i] > 0:
-            segments.append((int(idx_arr[i]), start, start + int(padded[i])))
-        start += int(padded[i])
     active = [float(p_arr[i]) for i in range(n_seg) if idx_arr[i] >= 0 and padded[i] > 0]
     enable_dropout = any(p > 0 for p in active)
     same = (len(set(active)) <= 1)
@@ -186,7 +193,7 @@ def prepare_multi_lora_batch_info(
         adapter_thresh16=dev[4 * n_blk:n_int],
         adapter_inv_keep=fdev[n_int + n_ad:n_int + 2 * n_ad],
         segments=segments,
-        segment_table=SegmentTable(segments, device, total_rows=start),
+        segment_table=SegmentTable(segments, device, total_rows=start, rows=moved[:n_row].view(-1, 4)),
         seed=seed,
         total_padded_tokens=start,
     )

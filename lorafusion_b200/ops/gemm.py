@@ -18,7 +18,7 @@ from . import _native as nv
 from .tile_config import get_kernel_config
 
 
-def _check2d(t: torch.Tensor, name: str) -> None:
+def check2d(t: torch.Tensor, name: str) -> None:
     if t.dim() != 2 or t.stride(1) != 1:
         raise ValueError(f"{name} must be 2-D with a contiguous last dim, got {tuple(t.shape)} "
                          f"strides {t.stride()}")
@@ -82,18 +82,18 @@ def fill_gemm_args(
         max_ctas = cfg.max_ctas if max_ctas is None else max_ctas
     group_m = 8 if group_m is None else group_m
     max_ctas = 0 if max_ctas is None else max_ctas
-    _check2d(a, "a")
+    check2d(a, "a")
     args = nv.LfGemmArgs()
     args.a, args.a_rows, args.a_cols, args.a_ld = a.data_ptr(), a.shape[0], a.shape[1], a.stride(0)
     if hasattr(b, "packed"):
         # NF4 weight: the packed bytes stand in for the bf16 [rows, cols] matrix
         args.b, args.b_rows, args.b_cols, args.b_ld = b.packed.data_ptr(), b.shape[0], b.shape[1], b.shape[1]
     else:
-        _check2d(b, "b")
+        check2d(b, "b")
         args.b, args.b_rows, args.b_cols, args.b_ld = b.data_ptr(), b.shape[0], b.shape[1], b.stride(0)
     if K2 > 0:
-        _check2d(a2, "a2")
-        _check2d(b2, "b2")
+        check2d(a2, "a2")
+        check2d(b2, "b2")
         args.a2, args.a2_rows, args.a2_cols, args.a2_ld = (
             a2.data_ptr(), a2.shape[0], a2.shape[1], a2.stride(0))
         args.b2, args.b2_rows, args.b2_cols, args.b2_ld = (
@@ -173,6 +173,17 @@ def launch_gemm(pair: Optional[bool] = None, **kwargs) -> None:
     rc = lib.lf_gemm(C.byref(args))
     if rc != 0:
         raise RuntimeError(f"lf_gemm failed with code {rc}")
+
+
+def launch_skinny(split: int, **kwargs) -> None:
+    """Launch one of the rank-wide LoRA products of ``csrc/gemm/lora_skinny.cu`` on the current
+    stream (arguments as for :func:`fill_gemm_args`); ``split`` CTAs share the reduction of a
+    tile.  With ``a_mn`` the work list ``seg_tiles`` holds ``(adapter, start, end, 0)`` rows."""
+    args = fill_gemm_args(**kwargs)
+    nv.note_launch()
+    rc = nv.cuda_lib().lf_lora_skinny(C.byref(args), split)
+    if rc != 0:
+        raise RuntimeError(f"lf_lora_skinny failed with code {rc}")
 
 
 def _pick_bn(n: int) -> int:

@@ -32,13 +32,14 @@ Conventions
 
 from __future__ import annotations
 
-from dataclasses import dataclass, field, replace
+import functools
+from dataclasses import dataclass, field
 from typing import Optional, Sequence
 
 import torch
 
 from . import _native as nv
-from .gemm import launch_gemm
+from .gemm import launch_gemm, launch_skinny
 from .philox import dropout_threshold
 
 RANK_PAD = 64
@@ -82,30 +83,40 @@ class DropoutSpec:
 NO_DROPOUT = DropoutSpec()
 
 
+# How many CTAs share the reduction of one 128-row output tile of a rank-wide product.  Two such
+# CTAs fit on an SM, so a launch has 296 places: the reduction is cut in two, four or eight while
+# all pieces still run at once and each keeps at least two 64-deep blocks to sum.  Measured (us for
+# 1, 2, 4, 8 CTAs a tile, S' with dropout): 100 x 1024 16.6 11.8 8.7 7.7; 8192 x 4096 60.9 35.8 28.5
+# 37.0 (eight no longer fit); 16384 x 4096 63.1 50.2 56.3 69.8.
+_SPLIT_PLACES = 2 * 148
+_SPLIT_MIN_BLOCKS = 2
+_SPLIT_MAX = 8
+
+
+@functools.lru_cache(maxsize=4096)
+def reduction_split(tiles: int, k_blocks: int) -> int:
+    """CTAs per output tile (1, 2, 4 or 8) for ``tiles`` tiles that sum ``k_blocks`` blocks each."""
+    c = 1
+    while c < _SPLIT_MAX and tiles * c * 2 <= _SPLIT_PLACES and k_blocks >= _SPLIT_MIN_BLOCKS * c * 2:
+        c *= 2
+    return c
+
+
 @dataclass
 class SegmentTable:
     """Token segments of one packed microbatch: ``(adapter, start, end)`` with ``start`` and
-    ``end`` multiples of 128 and at most one segment per adapter."""
+    ``end`` multiples of 128 and at most one segment per adapter.  ``rows`` (optional): the
+    :func:`segment_rows` of the segments, already on the device."""
 
     segments: Sequence[tuple[int, int, int]]
     device: torch.device
     total_rows: Optional[int] = None
+    rows: Optional[torch.Tensor] = None
     _cache: dict = field(default_factory=dict)
 
-    def split_plan(self, features: int):
-        """``(work list, owner)`` with long segments cut into token chunks, or ``None`` when the
-        plain work list already fills the GPU.  The work list's fourth column is the CHUNK index
-        (the slice of a partial-result buffer the chunk writes); ``owner[chunk]`` = its adapter."""
-        key = ("split", features)
-        if key not in self._cache:
-            self._cache[key] = _split_plan(self, features)
-        return self._cache[key]
-
-    def tiles_for(self, features: int) -> torch.Tensor:
-        """int32 ``[n_tiles, 4]`` work list ``(feature0, token0, k_blocks, adapter)``."""
-        t = self._cache.get(features)
-        if t is None:
-            rows = []
+    def device_rows(self) -> torch.Tensor:
+        """int32 ``[n, 4]`` work list ``(adapter, start, end, 0)`` of the gradient kernels."""
+        if "checked" not in self._cache:
             seen = set()
             for adapter, start, end in self.segments:
                 if adapter < 0 or end <= start:
@@ -116,47 +127,43 @@ class SegmentTable:
                 last = self.total_rows is not None and end >= self.total_rows
                 if start % TILE_M or (end % TILE_M and not last):
                     raise ValueError("segment bounds must be multiples of 128 tokens")
-                for f0 in range(0, features, TILE_M):
-                    rows.append((f0, start, (end - start + 63) // 64, adapter))
-            t = torch.tensor(rows, dtype=torch.int32).reshape(-1, 4).to(self.device)
-            self._cache[features] = t
-        return t
+            self._cache["checked"] = True
+        if self.rows is None:
+            self.rows = torch.tensor(segment_rows(self.segments), dtype=torch.int32).reshape(-1, 4).to(self.device)
+        return self.rows
+
+    def split_plan(self, features: int):
+        """``(chunks per segment, owner)`` when the tokens of every segment are summed in several
+        chunks, whose partial results are added in token order, or ``None`` when each (segment,
+        128-feature tile) is one chunk.  ``owner[chunk]`` = the adapter of each segment's chunks."""
+        chunks = self.chunks(features)
+        return None if chunks == 1 else (chunks, [r[0] for r in segment_rows(self.segments) for _ in range(chunks)])
+
+    def chunks(self, features: int) -> int:
+        """In how many chunks the tokens of a segment are summed."""
+        c = self._cache.get(features)
+        if c is None:
+            rows = segment_rows(self.segments)
+            tiles = len(rows) * ((features + TILE_M - 1) // TILE_M)
+            c = reduction_split(tiles, (rows[0][2] - rows[0][1] + 63) // 64) if rows else 1
+            self._cache[features] = c
+        return c
 
 
-# A gradient kernel gives every (segment, 128-feature tile) to one CTA, which walks all tokens of
-# the segment.  With few long segments (one adapter, 8K tokens, 4096 features: 32 work items) most
-# SMs idle, so such segments are cut in token chunks that write PARTIAL results, summed afterwards.
-_SPLIT_BELOW_ITEMS = 96      # enough work items already: leave the segments whole
-_SPLIT_TARGET_ITEMS = 148
-_SPLIT_MAX_CHUNKS = 8
-_SPLIT_MIN_TOKENS = 1024
-
-
-def _split_plan(table: SegmentTable, features: int):
-    segs = [(a, s0, e0) for a, s0, e0 in table.segments if a >= 0 and e0 > s0]
-    f_tiles = (features + TILE_M - 1) // TILE_M
-    items = len(segs) * f_tiles
-    if not segs or items >= _SPLIT_BELOW_ITEMS:
-        return None
-    want = min(_SPLIT_MAX_CHUNKS, -(-_SPLIT_TARGET_ITEMS // items))
-    rows, owner = [], []
-    for a, s0, e0 in segs:
-        n_chunks = max(1, min(want, (e0 - s0) // _SPLIT_MIN_TOKENS))
-        step = -(-(e0 - s0) // n_chunks)
-        step = -(-step // TILE_M) * TILE_M
-        for c0 in range(s0, e0, step):
-            c1 = min(e0, c0 + step)
-            v = len(owner)
-            owner.append(a)
-            for f0 in range(0, features, TILE_M):
-                rows.append((f0, c0, (c1 - c0 + 63) // 64, v))
-    if len(owner) == len(segs):
-        return None   # nothing was cut
-    return torch.tensor(rows, dtype=torch.int32).reshape(-1, 4).to(table.device), owner
+def segment_rows(segments) -> list:
+    """``(adapter, start, end, 0)`` of every segment that has an adapter and tokens, the longest
+    first: its tiles start first, and the short ones fill the gaps at the end."""
+    rows = [(a, s, e, 0) for a, s, e in segments if a >= 0 and e > s]
+    rows.sort(key=lambda r: r[1] - r[2])
+    return rows
 
 
 def _flat2d(t: torch.Tensor) -> torch.Tensor:
     return t.reshape(-1, t.shape[-1])
+
+
+def _rows_split(rows: int, k: int) -> int:
+    return reduction_split((rows + TILE_M - 1) // TILE_M, (k + 63) // 64)
 
 
 def lora_down(x: torch.Tensor, a_all: torch.Tensor, *, tile_adapter: Optional[torch.Tensor],
@@ -168,10 +175,10 @@ def lora_down(x: torch.Tensor, a_all: torch.Tensor, *, tile_adapter: Optional[to
     assert K2 == K and R in RANK_PADS
     if out is None:
         out = torch.empty((M, R), dtype=torch.bfloat16, device=x.device)
-    launch_gemm(a=x, b=_flat2d(a_all), out=out, M=M, N=R, K=K, bn=R,
-                epi=nv.EPI_BF16_ADAPTER_SCALE, mask_a=dropout.active,
-                tile_adapter=tile_adapter, b_adapter_rows=R, adapter_scale=adapter_scale,
-                scale=scale, **dropout.kwargs())
+    launch_skinny(_rows_split(M, K), a=x, b=_flat2d(a_all), out=out, M=M, N=R, K=K, bn=R,
+                  epi=nv.EPI_BF16_ADAPTER_SCALE, mask_a=dropout.active,
+                  tile_adapter=tile_adapter, b_adapter_rows=R, adapter_scale=adapter_scale,
+                  scale=scale, **dropout.kwargs())
     return out
 
 
@@ -202,9 +209,9 @@ def lora_ds(dy: torch.Tensor, b_all: torch.Tensor, *, tile_adapter: Optional[tor
     assert N2 == N and R in RANK_PADS
     if out is None:
         out = torch.empty((M, R), dtype=torch.bfloat16, device=dy.device)
-    launch_gemm(a=dy, b=_flat2d(b_all), out=out, M=M, N=R, K=N, b_mn=True, bn=R,
-                epi=nv.EPI_BF16_ADAPTER_SCALE, tile_adapter=tile_adapter, b_adapter_rows=N,
-                adapter_scale=adapter_scale, scale=scale)
+    launch_skinny(_rows_split(M, N), a=dy, b=_flat2d(b_all), out=out, M=M, N=R, K=N, b_mn=True, bn=R,
+                  epi=nv.EPI_BF16_ADAPTER_SCALE, tile_adapter=tile_adapter, b_adapter_rows=N,
+                  adapter_scale=adapter_scale, scale=scale)
     return out
 
 
@@ -213,19 +220,11 @@ def lora_db(dy: torch.Tensor, s: torch.Tensor, segs: SegmentTable, db_all: torch
     M, N = dy.shape
     n, N2, R = db_all.shape
     assert N2 == N and s.shape == (M, R) and db_all.dtype == torch.float32
-    plan = segs.split_plan(N)
-    if plan is not None:
-        tiles, owner = plan
-        tmp = torch.zeros((len(owner), N, R), dtype=torch.float32, device=dy.device)
-        launch_gemm(a=dy, b=s, out=tmp, M=N, N=R, K=M, a_mn=True, b_mn=True, bn=R,
-                    epi=nv.EPI_F32_ACCUM, seg_tiles=tiles, ldo=R, out_adapter_stride=N * R)
-        _fold_chunks(tmp, owner, db_all)
+    rows = segs.device_rows()
+    if rows.shape[0] == 0:
         return
-    tiles = segs.tiles_for(N)
-    if tiles.shape[0] == 0:
-        return
-    launch_gemm(a=dy, b=s, out=db_all, M=N, N=R, K=M, a_mn=True, b_mn=True, bn=R,
-                epi=nv.EPI_F32_ACCUM, seg_tiles=tiles, ldo=R, out_adapter_stride=N * R)
+    launch_skinny(segs.chunks(N), a=dy, b=s, out=db_all, M=N, N=R, K=M, a_mn=True, b_mn=True, bn=R,
+                  epi=nv.EPI_F32_ACCUM, seg_tiles=rows, ldo=R, out_adapter_stride=N * R)
 
 
 def lora_da(x: torch.Tensor, ds: torch.Tensor, segs: SegmentTable, da_all: torch.Tensor, *,
@@ -234,38 +233,12 @@ def lora_da(x: torch.Tensor, ds: torch.Tensor, segs: SegmentTable, da_all: torch
     M, K = x.shape
     n, R, K2 = da_all.shape
     assert K2 == K and ds.shape == (M, R) and da_all.dtype == torch.float32
-    plan = segs.split_plan(K)
-    if plan is not None:
-        tiles, owner = plan
-        drop = dropout
-        if dropout.adapter_thresh16 is not None:   # per-adapter rates follow the chunks
-            idx = torch.tensor(owner, dtype=torch.long, device=x.device)
-            drop = replace(dropout, adapter_thresh16=dropout.adapter_thresh16[idx].contiguous(),
-                           adapter_inv_keep=dropout.adapter_inv_keep[idx].contiguous())
-        tmp = torch.zeros((len(owner), R, K), dtype=torch.float32, device=x.device)
-        launch_gemm(a=x, b=ds, out=tmp, M=K, N=R, K=M, a_mn=True, b_mn=True, bn=R,
-                    epi=nv.EPI_F32_ACCUM, mask_a=drop.active, seg_tiles=tiles, ldo=K,
-                    out_transposed=True, out_adapter_stride=R * K, **drop.kwargs())
-        _fold_chunks(tmp, owner, da_all)
+    rows = segs.device_rows()
+    if rows.shape[0] == 0:
         return
-    tiles = segs.tiles_for(K)
-    if tiles.shape[0] == 0:
-        return
-    launch_gemm(a=x, b=ds, out=da_all, M=K, N=R, K=M, a_mn=True, b_mn=True, bn=R,
-                epi=nv.EPI_F32_ACCUM, mask_a=dropout.active, seg_tiles=tiles, ldo=K,
-                out_transposed=True, out_adapter_stride=R * K, **dropout.kwargs())
-
-
-def _fold_chunks(tmp: torch.Tensor, owner: Sequence[int], out_all: torch.Tensor) -> None:
-    """``out_all[a] += sum of the chunk partials of adapter a``, chunks in token order (a fixed
-    order, so the result does not depend on which CTA finished first)."""
-    start = 0
-    while start < len(owner):
-        end = start
-        while end < len(owner) and owner[end] == owner[start]:
-            end += 1
-        out_all[owner[start]] += tmp[start:end].sum(0)
-        start = end
+    launch_skinny(segs.chunks(K), a=x, b=ds, out=da_all, M=K, N=R, K=M, a_mn=True, b_mn=True, bn=R,
+                  epi=nv.EPI_F32_ACCUM, mask_a=dropout.active, seg_tiles=rows, ldo=K,
+                  out_transposed=True, out_adapter_stride=R * K, **dropout.kwargs())
 
 
 def base_lora_dx(dy: torch.Tensor, w: torch.Tensor, ds: Optional[torch.Tensor],

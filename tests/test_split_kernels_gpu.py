@@ -20,6 +20,57 @@ def _f32mm(a, b):
     return a.float() @ b.float()
 
 
+@pytest.mark.parametrize("split", [1, 2, 4, 8])
+@pytest.mark.parametrize("R,K", [(64, 200), (128, 520), (192, 1032), (256, 4096)])
+def test_rank_wide_products(split, R, K, monkeypatch):
+    """S', dS, dB and dA for every split, down to slices without a single block (K = 200 has four
+    blocks); ragged last tile, three segments of different lengths, one tile without an adapter.
+    Twice the same bits: the partial sums are added in a fixed order."""
+    from lorafusion_b200.ops import lora_kernels as lk
+    from lorafusion_b200.ops.philox import dropout_threshold, keep_mask
+
+    n, M, p = 3, 128 * 5 + 72, [0.1, 0.0, 0.5]
+    segs = [(1, 0, 128), (-1, 128, 256), (2, 256, 640), (0, 640, M)]
+    tile_adapter = torch.tensor([1, -1, 2, 2, 2, 0], dtype=torch.int32, device="cuda")
+    x, s, a, b = _rand(M, K, seed=1), _rand(M, R, scale=0.1, seed=2), _rand(n, R, K, scale=0.05, seed=3), \
+        _rand(n, K, R, scale=0.05, seed=4)
+    alpha = torch.tensor([2.0, 0.5, 1.0], device="cuda")
+    drop = lk.DropoutSpec(seed=(5 << 32) | 77, stream_id=9, row_offset=3, col_offset=16,
+                          adapter_thresh16=torch.tensor([dropout_threshold(v) for v in p], dtype=torch.int32, device="cuda"),
+                          adapter_inv_keep=torch.tensor([1 / (1 - v) for v in p], device="cuda"))
+    monkeypatch.setattr(lk, "reduction_split", lambda *_: split)
+    table = lk.SegmentTable(segs, torch.device("cuda"), total_rows=M)
+    out = []
+    for _ in range(2):
+        da, db = torch.ones(n, R, K, device="cuda"), torch.ones(n, K, R, device="cuda")
+        lk.lora_da(x, s, table, da, dropout=drop)
+        lk.lora_db(x, s, table, db)
+        out.append((lk.lora_down(x, a, tile_adapter=tile_adapter, adapter_scale=alpha, dropout=drop),
+                    lk.lora_ds(x, b, tile_adapter=tile_adapter, adapter_scale=alpha), da, db))
+    assert all(torch.equal(u, v) for u, v in zip(*out))
+    down, ds, da, db = out[0]
+    assert not down[128:256].any() and not ds[128:256].any()
+    for ad, r0, r1 in segs:
+        if ad < 0:
+            continue
+        keep = keep_mask(r1 - r0, K, p[ad], (5 << 32) | 77, 9, row_offset=3 + r0, col_offset=16).cuda()
+        xh = torch.where(keep, x[r0:r1].float() / (1 - p[ad]), torch.zeros((), device="cuda")).to(torch.bfloat16)
+        assert_close_two_rounds(down[r0:r1], alpha[ad] * _f32mm(xh, a[ad].t()), msg=f"S' {ad}")
+        assert_close_two_rounds(ds[r0:r1], alpha[ad] * _f32mm(x[r0:r1], b[ad]), msg=f"dS {ad}")
+        # fp32 sums of at most 384 products of magnitude 0.1 in another order
+        assert_close_two_rounds(db[ad], 1 + _f32mm(x[r0:r1].t(), s[r0:r1]), rtol=1e-4, atol=1e-4, msg=f"dB {ad}")
+        assert_close_two_rounds(da[ad], 1 + _f32mm(s[r0:r1].t(), xh), rtol=1e-4, atol=1e-4, msg=f"dA {ad}")
+
+
+def test_philox_with_row_and_column_parts_taken_out_drops_everything_at_p_near_one():
+    """A threshold of 65536 (p above 1 - 2^-17) does not fit the packed comparison: all is dropped."""
+    from lorafusion_b200.ops import lora_kernels as lk
+
+    x, a = _rand(130, 128), _rand(1, 64, 128)
+    s = lk.lora_down(x, a, tile_adapter=None, adapter_scale=None, dropout=lk.DropoutSpec(p=1 - 2.0 ** -18))
+    assert not s.any()
+
+
 def test_nf4_codes_at_the_midpoints():
     """Codes next to every midpoint, blocks of zeros, and a block count that leaves the last CTA
     nearly empty: the same codes as the CPU quantiser; a NaN weight encodes as the CPU's 0th code."""
