@@ -55,6 +55,18 @@ __device__ __forceinline__ void att_mma_kmn(uint32_t tmem_d, uint32_t sA, uint32
                  (accumulate || k > 0) ? 1u : 0u);
   }
 }
+// Half of D (+)= A * B with A [128 x 128(k)] bf16 in tensor memory (64 columns) and B MN-major:
+// reduction steps [4 * half, 4 * half + 4).
+__device__ __forceinline__ void att_mma_ts_half(uint32_t tmem_d, uint32_t tmem_a, uint32_t sB, int half,
+                                                bool accumulate) {
+  constexpr uint32_t IDESC = make_idesc_bf16(128, 128, 0, 1);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int k = 4 * half + i;
+    umma_bf16_ts(tmem_d, tmem_a + k * 8, make_smem_desc_sw128(sB + k * 2048, ATT_PANEL_BYTES, 1024), IDESC,
+                 (accumulate || k > 0) ? 1u : 0u);
+  }
+}
 // D (+)= A^T * B with A MN-major [128(k) rows x 128(m) cols], B MN-major [128(k) x 128(n)].
 __device__ __forceinline__ void att_mma_mnmn(uint32_t tmem_d, uint32_t sA, uint32_t sB,
                                              bool accumulate) {
