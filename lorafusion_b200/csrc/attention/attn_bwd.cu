@@ -29,6 +29,7 @@ struct AttnBwdParams {
   long long ld_qkv;
   const float* lse;
   const float* delta;
+  int heads_per_cta;           // dQ: query heads of a group that one CTA walks
   long long M_total;
   float scale, scale_log2e;
   int* err;
@@ -40,23 +41,66 @@ constexpr int BWD_SMEM = ATT_TILE_BYTES * 7 + 256 + 1024;
 // quarter warp % 4).  The backward needs no row reductions, so the halves never talk.
 constexpr int BWD_THREADS = 64 + 256;
 
-// ----------------------------------------------------------------------------------
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o,
-                                  const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta,
-                                  long long M, int Hq, long long ld) {
-  const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= M * Hq) return;
-  const long long m = w / Hq;
-  const int h = int(w % Hq);
-  const uint2 a = *reinterpret_cast<const uint2*>(o + m * ld + h * ATT_D + lane * 4);
-  const uint2 b = *reinterpret_cast<const uint2*>(d_o + m * ld + h * ATT_D + lane * 4);
-  const float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y);
-  const float2 b0 = unpack_bf16x2(b.x), b1 = unpack_bf16x2(b.y);
-  float s = a0.x * b0.x + a0.y * b0.y + a1.x * b1.x + a1.y * b1.y;
+// Bound by the reads of O and dO.  A CTA takes eight rows of sixteen heads: each warp reads 4 KB of one
+// row from either matrix, all thirty-two loads in flight, and the sums leave eight rows of a head
+// (32 bytes) at a time through shared memory.  (One head of a row a warp, two loads in flight and single
+// 4-byte stores: 148 us for 16384 rows of 64 heads, 3.6 TB/s.  A warp on sixteen rows of one head, so
+// that it could store them itself, took 194 us, and forming delta inside the dQ kernel cost
+// 220 us there: each head started with the loads' latency.)
+constexpr int DELTA_HEADS = 16;
+
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta,
+                  long long M, int Hq, long long ld) {
+  __shared__ float sums[DELTA_HEADS][8];
+  const int groups = (Hq + DELTA_HEADS - 1) / DELTA_HEADS;
+  const int h0 = int(blockIdx.x % groups) * DELTA_HEADS;
+  const long long m0 = (long long)(blockIdx.x / groups) * 8;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = m0 + warp < M ? min(DELTA_HEADS, Hq - h0) : 0;
+  const long long off = (m0 + warp) * ld + h0 * ATT_D + lane * 4;
+  uint2 a[DELTA_HEADS], b[DELTA_HEADS];
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) delta[(long long)h * M + m] = s;
+  for (int i = 0; i < DELTA_HEADS; ++i) {
+    a[i] = i < n ? *reinterpret_cast<const uint2*>(o + off + i * ATT_D) : make_uint2(0u, 0u);
+    b[i] = i < n ? *reinterpret_cast<const uint2*>(d_o + off + i * ATT_D) : make_uint2(0u, 0u);
+  }
+#pragma unroll
+  for (int i = 0; i < DELTA_HEADS; ++i) {
+    const float2 x0 = unpack_bf16x2(a[i].x), x1 = unpack_bf16x2(a[i].y);
+    const float2 y0 = unpack_bf16x2(b[i].x), y1 = unpack_bf16x2(b[i].y);
+    float t = x0.x * y0.x + x0.y * y0.y + x1.x * y1.x + x1.y * y1.y;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
+    if (lane == i) sums[i][warp] = t;
+  }
+  __syncthreads();
+  const int i = threadIdx.x >> 3, r = threadIdx.x & 7;
+  if (i < DELTA_HEADS && h0 + i < Hq && m0 + r < M) delta[(long long)(h0 + i) * M + m0 + r] = sums[i][r];
+}
+
+// The element-wise arithmetic of a thread's 64 columns, two at a time.
+__device__ __forceinline__ void load_row(uint32_t taddr, float (&v)[64]) {
+  tmem_ld_32x32b_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+  tmem_ld_32x32b_x32(taddr + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+  tmem_ld_wait();
+}
+// P = 2^(S * scale * log2(e) - lse * log2(e))
+__device__ __forceinline__ void exp_rows(float (&v)[64], float scale_log2e, float lse2) {
+  const unsigned long long c2 = f32x2(scale_log2e, scale_log2e), l2 = f32x2(-lse2, -lse2);
+#pragma unroll
+  for (int i = 0; i < 64; i += 2) {
+    unpack_f32x2(fma_f32x2(f32x2(v[i], v[i + 1]), c2, l2), v[i], v[i + 1]);
+    v[i] = fast_exp2(v[i]);
+    v[i + 1] = fast_exp2(v[i + 1]);
+  }
+}
+// dS = P (.) (dP * scale - delta * scale), over P
+__device__ __forceinline__ void ds_rows(float (&v)[64], const float (&dp)[64], float scale, float dlts) {
+  const unsigned long long s2 = f32x2(scale, scale), d2 = f32x2(-dlts, -dlts);
+#pragma unroll
+  for (int i = 0; i < 64; i += 2)
+    unpack_f32x2(mul_f32x2(f32x2(v[i], v[i + 1]), fma_f32x2(f32x2(dp[i], dp[i + 1]), s2, d2)), v[i], v[i + 1]);
 }
 
 // ----------------------------------------------------------------------------------
@@ -100,13 +144,14 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   AbortCtx ctx{p.err, abort_flag};
-  const int4 tile = p.tiles[blockIdx.x];
+  const int4 tile = p.tiles[blockIdx.x / p.Hkv];
   const int row0 = tile.x, rows = tile.y, seq_row0 = tile.z;
   // One CTA per (query tile, KV head): it walks the query heads of the group one after the
   // other, so TMEM, barriers and the K/V ring are set up once (see attn_fwd.cu).
-  const int g = blockIdx.y;
-  const int group = p.Hq / p.Hkv;
-  const int h0 = g * group;
+  const int g = blockIdx.x % p.Hkv;
+  const int first_head = p.heads_per_cta * int(blockIdx.y);
+  const int group = min(p.Hq / p.Hkv - first_head, p.heads_per_cta);  // heads of this CTA
+  const int h0 = g * (p.Hq / p.Hkv) + first_head;
   const int n_kv = (row0 - seq_row0) / ATT_TILE + 1;
   const int total = group * n_kv;  // flat (head, key tile) sequence J = hi * n_kv + j
 
@@ -246,17 +291,11 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
         const bool diag = (j == n_kv - 1);
         // P of this thread's 64 columns from S alone, while the tensor pipe still produces dP
         float pv[64];
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-          uint32_t(&dst)[32] = *reinterpret_cast<uint32_t(*)[32]>(&pv[cc * 32]);
-          tmem_ld_32x32b_x32(tS[sb] + lane_addr + c0 + cc * 32, dst);
-        }
-        tmem_ld_wait();
+        load_row(tS[sb] + lane_addr + c0, pv);
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&s_empty[sb]);
-#pragma unroll
-        for (int i = 0; i < 64; ++i) pv[i] = fast_exp2(pv[i] * p.scale_log2e - lse2);
+        exp_rows(pv, p.scale_log2e, lse2);
         if (diag || rows < ATT_TILE) {   // uniform: only the diagonal tile and a ragged query tile mask anything
 #pragma unroll
           for (int i = 0; i < 64; ++i)
@@ -267,13 +306,10 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
           break;
         }
         tc_fence_after_sync();
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {   // dS in registers (over P); dP's buffer is free right after
-          uint32_t dv[32];
-          tmem_ld_32x32b_x32(tDP + lane_addr + c0 + cc * 32, dv);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) pv[cc * 32 + i] *= fmaf(__uint_as_float(dv[i]), p.scale, -dlts);
+        {   // dS in registers (over P); dP's buffer is free right after
+          float dv[64];
+          load_row(tDP + lane_addr + c0, dv);
+          ds_rows(pv, dv, p.scale, dlts);
         }
         tc_fence_before_sync();
         __syncwarp();
@@ -294,10 +330,8 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
         if (lane == 0) mbar_arrive(ds_full);
       }
       if (!ok) break;
-      if (!__all_sync(0xffffffffu, mbar_wait(dq_done, (hi * n_kv + n_kv - 1) & 1, ctx, ERR_WAIT_MISC))) {
-        ok = false;
-        break;
-      }
+      ok = __all_sync(0xffffffffu, mbar_wait(dq_done, (hi * n_kv + n_kv - 1) & 1, ctx, ERR_WAIT_MISC));
+      if (!ok) break;
       tc_fence_after_sync();
       __nv_bfloat16* orow = p.dqkv + grow * p.ld_qkv + p.q_col0 + h * ATT_D + c0;
 #pragma unroll 1
@@ -314,6 +348,7 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
                          pack_bf16x2(__uint_as_float(o[gq * 8 + 4]), __uint_as_float(o[gq * 8 + 5])),
                          pack_bf16x2(__uint_as_float(o[gq * 8 + 6]), __uint_as_float(o[gq * 8 + 7])));
         }
+        __syncwarp();   // the TMEM load above is .sync.aligned
       }
       tc_fence_before_sync();
       __syncwarp();
@@ -367,9 +402,9 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   AbortCtx ctx{p.err, abort_flag};
-  const int4 tile = p.tiles[blockIdx.x];
+  const int4 tile = p.tiles[p.num_tiles - 1 - blockIdx.x / p.Hkv];   // first key tiles first: they see the most queries
   const int row0 = tile.x, rows = tile.y, seq_row0 = tile.z, seq_rows = tile.w;
-  const int g = blockIdx.y;
+  const int g = blockIdx.x % p.Hkv;
   const int group = p.Hq / p.Hkv;
   const int i_kv = (row0 - seq_row0) / ATT_TILE;
   const int n_q_tiles = (seq_rows + ATT_TILE - 1) / ATT_TILE;
@@ -500,17 +535,11 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
       tc_fence_after_sync();
       // P of this thread's 64 columns in registers first; its store waits for the shared P / dS buffer
       float pv[64];
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        uint32_t(&dst)[32] = *reinterpret_cast<uint32_t(*)[32]>(&pv[cc * 32]);
-        tmem_ld_32x32b_x32(tS + lane_addr + c0 + cc * 32, dst);
-      }
-      tmem_ld_wait();
+      load_row(tS + lane_addr + c0, pv);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(s_empty);   // S has been read: the next iteration's S may be issued
-#pragma unroll
-      for (int i = 0; i < 64; ++i) pv[i] = fast_exp2(pv[i] * p.scale_log2e - lse2);
+      exp_rows(pv, p.scale_log2e, lse2);
       if (need_mask) {   // only the diagonal tile and a ragged last query tile have anything to mask
 #pragma unroll
         for (int i = 0; i < 64; ++i)
@@ -536,13 +565,10 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
       }
       tc_fence_after_sync();
       // dS = P (.) (dP - delta) * scale, in place over P (fp32; the dV product saw the same P rounded to bf16)
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        uint32_t dv[32];
-        tmem_ld_32x32b_x32(tDP + lane_addr + c0 + cc * 32, dv);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) pv[cc * 32 + i] *= fmaf(__uint_as_float(dv[i]), p.scale, -dlts);
+      {
+        float dv[64];
+        load_row(tDP + lane_addr + c0, dv);
+        ds_rows(pv, dv, p.scale, dlts);
       }
       tc_fence_before_sync();
       __syncwarp();
@@ -582,6 +608,7 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
                          pack_bf16x2(__uint_as_float(o[gq * 8 + 4]), __uint_as_float(o[gq * 8 + 5])),
                          pack_bf16x2(__uint_as_float(o[gq * 8 + 6]), __uint_as_float(o[gq * 8 + 7])));
         }
+        __syncwarp();   // the TMEM load above is .sync.aligned
       }
     }
   }
@@ -622,11 +649,9 @@ extern "C" int lf_attn_bwd(const void* qkv, const void* out, const void* d_out, 
       ensure_max_dynamic_smem(dkdv_configured, attn_dkdv_kernel, BWD_SMEM) != cudaSuccess)
     return -10;
   {
-    const long long warps = M * Hq;
-    const int block = 256;
-    const long long grid = (warps * 32 + block - 1) / block;
-    attn_delta_kernel<<<(unsigned)grid, block, 0, st>>>((const __nv_bfloat16*)out,
-                                                         (const __nv_bfloat16*)d_out, delta, M, Hq, ldo);
+    const long long blocks = (M + 7) / 8 * ((Hq + DELTA_HEADS - 1) / DELTA_HEADS);
+    attn_delta_kernel<<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, delta, M, Hq,
+                                                        ldo);
   }
   AttnBwdParams p;
   p.tiles = (const int4*)tiles;
@@ -644,8 +669,17 @@ extern "C" int lf_attn_bwd(const void* qkv, const void* out, const void* d_out, 
   p.scale = scale;
   p.scale_log2e = scale * 1.4426950408889634f;
   p.err = err;
-  attn_dq_kernel<<<dim3(num_tiles, Hkv), BWD_THREADS, BWD_SMEM, st>>>(p, tmQKV, tmDO);  // walks the group's q heads
-  attn_dkdv_kernel<<<dim3(num_tiles, Hkv), BWD_THREADS, BWD_SMEM, st>>>(p, tmQKV, tmDO);
+  // KV heads vary fastest, so that a launch starts with its longest CTAs (the tile list starts with the
+  // longest key ranges): with the tiles fastest the long tiles of the last heads started last.
+  // One CTA walks all query heads of a group, which pays for its set-up once, unless the launch
+  // would leave SMs idle: then the heads of a group go to several CTAs.
+  const int group = Hq / Hkv;
+  int parts = 1;
+  while (parts < group && (long long)num_tiles * Hkv * (parts + 1) <= 148) ++parts;
+  p.heads_per_cta = (group + parts - 1) / parts;
+  attn_dq_kernel<<<dim3(num_tiles * Hkv, (group + p.heads_per_cta - 1) / p.heads_per_cta), BWD_THREADS, BWD_SMEM, st>>>(
+      p, tmQKV, tmDO);
+  attn_dkdv_kernel<<<dim3(num_tiles * Hkv), BWD_THREADS, BWD_SMEM, st>>>(p, tmQKV, tmDO);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

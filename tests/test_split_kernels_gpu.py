@@ -71,6 +71,31 @@ def test_philox_with_row_and_column_parts_taken_out_drops_everything_at_p_near_o
     assert not s.any()
 
 
+@pytest.mark.parametrize("lens,Hq,Hkv", [([1], 1, 1), ([129, 3, 128], 3, 1), ([300, 257], 10, 2), ([700, 31, 513], 8, 1),
+                                         ([128] * 150, 5, 1)])
+def test_attention_head_groups(lens, Hq, Hkv):
+    """Odd groups (the last pair of heads has one), groups split over CTAs (few tiles) and whole
+    (150 tiles), sequences around the tile size; forward, and backward with its row deltas."""
+    from lorafusion_b200.ops import attention as att
+
+    D, M = 128, sum(lens)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    qkv = _rand(M, (Hq + 2 * Hkv) * D, scale=0.7, seed=5).requires_grad_(True)
+    dout = _rand(M, Hq * D, seed=6)
+    out = att.packed_attention(qkv, att.build_attn_tiles(cu, "cuda"), Hq, Hkv)
+    grad, = torch.autograd.grad(out, [qkv], dout)
+    ref_in = qkv.detach().float().requires_grad_(True)
+    parts = ref_in.split([Hq * D, Hkv * D, Hkv * D], dim=1)
+    ref = att.attention_reference(parts[0].reshape(M, Hq, D), parts[1].reshape(M, Hkv, D), parts[2].reshape(M, Hkv, D),
+                                  cu).reshape(M, Hq * D)
+    ref_grad, = torch.autograd.grad(ref, [ref_in], dout.float())
+    # bf16 probabilities and outputs: 2^-8 of values around one
+    assert_close_two_rounds(out, ref, atol=2e-2, msg="attention fwd")
+    assert_close_two_rounds(grad, ref_grad, atol=5e-2, scale_atol_by_rms=True, msg="attention bwd")
+
+
 def test_nf4_codes_at_the_midpoints():
     """Codes next to every midpoint, blocks of zeros, and a block count that leaves the last CTA
     nearly empty: the same codes as the CPU quantiser; a NaN weight encodes as the CPU's 0th code."""
