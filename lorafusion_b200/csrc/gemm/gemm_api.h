@@ -40,6 +40,8 @@ typedef struct LfGemmArgs {
   const float* adapter_inv_keep;     // per-adapter 1 / (1 - p) or null
   int32_t* err;                 // device error word
   void* stream;
+  void* scratch;                // lf_gemm_pair: scratch_bytes of device memory (256-byte aligned) or null,
+  int64_t scratch_bytes;        // see lf_gemm_pair_scratch
   int32_t a_mn, b_mn, b2_mn;
   int32_t M, N, K, K2;
   int32_t bn, nacc, epi, mask_a;
@@ -53,6 +55,9 @@ typedef struct LfGemmArgs {
   int32_t row_offset, col_offset;
   int32_t group_m, max_ctas;
 } LfGemmArgs;
+
+// Scratch a product of the CTA-pair kernels wants (0 = none).
+long long lf_gemm_pair_scratch(int M, int N, int K, int max_ctas);
 
 // Returns 0 on success, negative on argument/launch errors.
 int lf_gemm(const LfGemmArgs* args);

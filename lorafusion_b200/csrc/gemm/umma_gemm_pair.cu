@@ -63,8 +63,35 @@ struct Params {
   int row_offset, col_offset;
   int zero_row;  // a row coordinate outside A2: TMA reads zeros there
   int m_rotate;  // pair rows the tile order is rotated by (tensor-parallel variants start / end with the own shard)
+  // Last wave cut along the reduction (see pick_split): tiles from `whole_tiles` on are computed in
+  // `split` slices, whose fp32 partial tiles meet in `partial`; `arrivals` (zeroed by the launcher)
+  // counts the slices that have stored theirs.
+  int whole_tiles, split;
+  float4* partial;
+  int* arrivals;
   int* err;
 };
+
+// One piece of work of a pair: blocks [kb0, kb1) of the main product of a tile.
+struct Unit {
+  int tile, kb0, kb1, slice;
+};
+
+// Unit `u` of pair `pair_id`.  Slices are ordered slice by slice, so that pairs working at the same
+// time read the same part of the reduction and share it in L2.
+__device__ __forceinline__ bool get_unit(const Params& p, int pair_id, int num_pairs, int u, Unit& w) {
+  const int i = pair_id + u * num_pairs;
+  if (i < p.whole_tiles) {
+    w = Unit{i, 0, p.nkb_main, -1};
+    return true;
+  }
+  const int cut = p.num_tiles - p.whole_tiles;
+  const int k = i - p.whole_tiles;
+  if (k >= cut * p.split) return false;
+  const int slice = k / cut;
+  w = Unit{p.whole_tiles + (k - slice * cut), p.nkb_main * slice / p.split, p.nkb_main * (slice + 1) / p.split, slice};
+  return true;
+}
 
 struct Tile {
   int pm, n_tile;   // pair-row index (256 rows) and column tile
@@ -148,8 +175,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
   const int pair_id = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
   AbortCtx ctx{p.err, abort_flag, TP != 0 ? kPeerWaitNs + kLocalWaitNs : kLocalWaitNs};
-  // main-loop block before which the next tile's slab is slipped in (slab-first variant)
-  const int ks = SLAB_FIRST ? p.nkb_main / 2 : p.nkb_main;
+  // main-loop block of a unit before which the next unit's slab is slipped in (slab-first variant)
+  auto slab_point = [&](const Unit& w) { return SLAB_FIRST ? w.kb0 + (w.kb1 - w.kb0) / 2 : w.kb1; };
+  // the slice that carries the slab: the first one where the slab opens the accumulator, else the last
+  auto has_slab = [&](const Unit& w) { return SLAB_FIRST ? w.kb0 == 0 : w.kb1 == p.nkb_main; };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -248,23 +277,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
         return true;
       };
       bool ok = true;
-      if (SLAB_FIRST && pair_id < p.num_tiles) {
-        const Tile t = decode(p, pair_id);
-        ok = rows_ready(t) && load_slabs(t);
+      Unit w, wn;
+      bool more = get_unit(p, pair_id, num_pairs, 0, w);
+      if (SLAB_FIRST && more) {
+        const Tile t = decode(p, w.tile);
+        ok = rows_ready(t) && (!has_slab(w) || load_slabs(t));
       }
-      for (int tile = pair_id; ok && tile < p.num_tiles; tile += num_pairs) {
-        const Tile t = decode(p, tile);
+      for (int u = 0; ok && more; ++u, w = wn) {
+        const Tile t = decode(p, w.tile);
+        const int ks = slab_point(w);
+        more = get_unit(p, pair_id, num_pairs, u + 1, wn);
         if (!SLAB_FIRST) ok = rows_ready(t);
-        ok = ok && load_main(t, 0, ks);
+        ok = ok && load_main(t, w.kb0, ks);
         if (SLAB_FIRST) {
-          if (ok && tile + num_pairs < p.num_tiles) {
-            const Tile tn = decode(p, tile + num_pairs);
-            ok = rows_ready(tn) && load_slabs(tn);
+          if (ok && more) {
+            const Tile tn = decode(p, wn.tile);
+            ok = rows_ready(tn) && (!has_slab(wn) || load_slabs(tn));
           }
         } else {
-          ok = ok && load_slabs(t);
+          ok = ok && (!has_slab(w) || load_slabs(t));
         }
-        ok = ok && load_main(t, ks, p.nkb_main);
+        ok = ok && load_main(t, ks, w.kb1);
       }
     }
   } else if (warp == 1) {
@@ -300,17 +333,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
           if (!issue_block(d, SLAB_FIRST && i == 0)) return false;
         return true;
       };
-      auto issue_main = [&](uint32_t d, int kb0, int kb1, bool opens) -> bool {
+      // blocks [kb0, kb1); with `opens` block `kb_open` overwrites the accumulator
+      auto issue_main = [&](uint32_t d, int kb0, int kb1, int kb_open, bool opens) -> bool {
         for (int kb = kb0; kb < kb1; ++kb)
-          if (!issue_block(d, opens && kb == 0)) return false;
+          if (!issue_block(d, opens && kb == kb_open)) return false;
         return true;
       };
-      int tile_iter = 0;
       bool ok = true;
-      if (SLAB_FIRST && pair_id < p.num_tiles) {
-        const Tile t = decode(p, pair_id);
+      Unit w, wn;
+      bool more = get_unit(p, pair_id, num_pairs, 0, w);
+      if (SLAB_FIRST && more) {
+        const Tile t = decode(p, w.tile);
         ok = mbar_wait(&tempty[0], 1, ctx, ERR_WAIT_TMEM_EMPTY);   // fresh barrier: passes at once
-        if (ok) {
+        if (ok && has_slab(w)) {
           tc_fence_after_sync();
           ok = issue_slabs(t, tmem_base);
         }
@@ -319,29 +354,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
           tc_commit_pair(mapa_shared(&sfull[0], 1));
         }
       }
-      for (int tile = pair_id; ok && tile < p.num_tiles; tile += num_pairs, ++tile_iter) {
-        const Tile t = decode(p, tile);
-        const int buf = tile_iter % NBUF;
-        const uint32_t bph = (tile_iter / NBUF) & 1;
+      for (int u = 0; ok && more; ++u, w = wn) {
+        const Tile t = decode(p, w.tile);
+        const int ks = slab_point(w);
+        const int buf = u % NBUF;
+        const uint32_t bph = (u / NBUF) & 1;
         const uint32_t acc = tmem_base + uint32_t(buf * BN);
+        more = get_unit(p, pair_id, num_pairs, u + 1, wn);
         bool opens = true;   // does the main product start from a fresh accumulator?
         if (SLAB_FIRST) {
           int ad[2];
-          opens = slab_passes(t, ad) * p.nkb2 == 0;
+          opens = !has_slab(w) || slab_passes(t, ad) * p.nkb2 == 0;
           ok = mbar_wait(&masked[buf], bph, ctx, ERR_WAIT_READY);
         } else {
           ok = mbar_wait(&tempty[buf], bph ^ 1, ctx, ERR_WAIT_TMEM_EMPTY);
         }
         if (!ok) break;
         tc_fence_after_sync();
-        ok = issue_main(acc, 0, ks, opens);
+        ok = issue_main(acc, w.kb0, ks, w.kb0, opens);
         if (SLAB_FIRST) {
-          if (ok && tile + num_pairs < p.num_tiles) {
-            const Tile tn = decode(p, tile + num_pairs);
-            const int nbuf = (tile_iter + 1) % NBUF;
-            const uint32_t nph = ((tile_iter + 1) / NBUF) & 1;
+          if (ok && more) {
+            const Tile tn = decode(p, wn.tile);
+            const int nbuf = (u + 1) % NBUF;
+            const uint32_t nph = ((u + 1) / NBUF) & 1;
             ok = mbar_wait(&tempty[nbuf], nph ^ 1, ctx, ERR_WAIT_TMEM_EMPTY);
-            if (ok) {
+            if (ok && has_slab(wn)) {
               tc_fence_after_sync();
               ok = issue_slabs(tn, tmem_base + uint32_t(nbuf * BN));
             }
@@ -351,10 +388,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
             }
           }
         } else {
-          ok = ok && issue_slabs(t, acc);
+          ok = ok && (!has_slab(w) || issue_slabs(t, acc));
         }
-        // with ks == 0 (a single main block) the main product opens here instead
-        ok = ok && issue_main(acc, ks, p.nkb_main, opens && ks == 0);
+        // with a single main block (ks == kb0) the main product opens here instead
+        ok = ok && issue_main(acc, ks, w.kb1, w.kb0, opens);
         if (!ok) break;
         tc_commit_pair(mapa_shared(&tfull[buf], 0));
         tc_commit_pair(mapa_shared(&tfull[buf], 1));
@@ -373,7 +410,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
     // Slab-first variant: multiply the slab product of tile `t` (in buffer `iter % 2`) by its
     // dropout mask, in place.  A CTA whose rows have no adapter (or an adapter without dropout)
     // only reports in.
-    auto mask_slab = [&](const Tile& t, int iter) -> bool {
+    auto mask_slab = [&](const Unit& w, int iter) -> bool {
+      const Tile t = decode(p, w.tile);
       const int buf = iter % NBUF;
       // warp-uniform: the tcgen05.ld/st below are .sync.aligned, and the warp reports in as one
       bool got = __all_sync(0xffffffffu, mbar_wait(&sfull[buf], uint32_t(iter / NBUF) & 1, ctx, ERR_WAIT_TMEM_FULL));
@@ -388,9 +426,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
         thresh = p.adapter_thresh16[my_adapter];
         inv_keep = p.adapter_inv_keep[my_adapter];
       }
-      if (p.nkb2 > 0 && my_adapter >= 0 && thresh != 0) {
+      if (p.nkb2 > 0 && has_slab(w) && my_adapter >= 0 && thresh != 0) {
         const int row = (2 * t.pm + int(cta)) * BM + q * 32 + lane;
         const uint32_t acc = tmem_base + uint32_t(buf * BN) + lane_addr;
+        const uint32_t thresh_hi = thresh << 16;
+        const PhiloxRow prow = philox_row(uint32_t(row + p.row_offset), p.stream_id, p.seed_lo, p.seed_hi);
         uint32_t r[32];
         tmem_ld_32x32b_x32(acc + c_begin * 32, r);
 #pragma unroll 1
@@ -400,15 +440,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
 #pragma unroll
           for (int j = 0; j < 32; ++j) w[j] = r[j];
           if (c + 1 < c_end) tmem_ld_32x32b_x32(acc + (c + 1) * 32, r);
-          const int col0 = t.n_tile * BN + c * 32;
+          const uint32_t col8 = uint32_t((t.n_tile * BN + c * 32 + p.col_offset) >> 3);
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
-            const uint32_t keep = dropout_keep8(uint32_t(row + p.row_offset),
-                                                uint32_t((col0 + p.col_offset) >> 3) + g, p.stream_id,
-                                                p.seed_lo, p.seed_hi, thresh);
+            const Philox4 o = philox_rest(prow, philox_col(col8 + g, p.stream_id, p.seed_lo), p.seed_lo, p.seed_hi);
+            const uint32_t rnd[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-              w[g * 8 + j] = ((keep >> j) & 1u) ? __float_as_uint(inv_keep * __uint_as_float(w[g * 8 + j])) : 0u;
+            for (int j = 0; j < 4; ++j) {
+              uint32_t& lo = w[g * 8 + 2 * j];
+              uint32_t& hi = w[g * 8 + 2 * j + 1];
+              lo = (rnd[j] & 0xffffu) >= thresh ? __float_as_uint(inv_keep * __uint_as_float(lo)) : 0u;
+              // a threshold past 16 bits drops every element
+              hi = rnd[j] >= thresh_hi && thresh <= 0xffffu ? __float_as_uint(inv_keep * __uint_as_float(hi)) : 0u;
+            }
           }
           tmem_st_32x32b_x32(acc + c * 32, w);
         }
@@ -420,19 +464,49 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
       return true;
     };
 
-    int tile_iter = 0;
+    // one 32-column chunk of a finished row: bias, rounding, store
+    auto store_chunk = [&](const Tile& t, int c, float (&v)[32]) {
+      const int row = (2 * t.pm + int(cta)) * BM + q * 32 + lane;
+      const int col0 = t.n_tile * BN + c * 32;
+      if (EPI == LF_EPI_BF16 && p.bias != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
+      }
+      if (row < p.M) {
+        // reduce-scatter: the partial tile stays in THIS GPU's stage [M, N]; the owner pulls it
+        __nv_bfloat16* out = (TP == 2) ? tp.rs_peer_stage[tp.rank] + (long long)row * p.N
+                                       : p.out + (long long)row * p.ldo;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          const int col = col0 + g * 8;
+          if (col + 8 <= p.N) {
+            st_global_v4(out + col, pack_bf16x2(v[g * 8 + 0], v[g * 8 + 1]),
+                         pack_bf16x2(v[g * 8 + 2], v[g * 8 + 3]), pack_bf16x2(v[g * 8 + 4], v[g * 8 + 5]),
+                         pack_bf16x2(v[g * 8 + 6], v[g * 8 + 7]));
+          } else {
+            for (int j = 0; j < 8; ++j)
+              if (col + j < p.N) out[col + j] = __float2bfloat16(v[g * 8 + j]);
+          }
+        }
+      }
+    };
+
     bool ok = true;
-    if (SLAB_FIRST && pair_id < p.num_tiles) ok = mask_slab(decode(p, pair_id), 0);
-    for (int tile = pair_id; ok && tile < p.num_tiles; tile += num_pairs, ++tile_iter) {
-      const Tile t = decode(p, tile);
-      if (SLAB_FIRST && tile + num_pairs < p.num_tiles) {
-        if (!mask_slab(decode(p, tile + num_pairs), tile_iter + 1)) {
+    Unit w, wn;
+    bool more = get_unit(p, pair_id, num_pairs, 0, w);
+    if (SLAB_FIRST && more) ok = mask_slab(w, 0);
+    for (int u = 0; ok && more; ++u, w = wn) {
+      const Tile t = decode(p, w.tile);
+      more = get_unit(p, pair_id, num_pairs, u + 1, wn);
+      if (SLAB_FIRST && more) {
+        if (!mask_slab(wn, u + 1)) {
           ok = false;
           break;
         }
       }
-      const int buf = tile_iter % NBUF;
-      const uint32_t bph = (tile_iter / NBUF) & 1;
+      const int buf = u % NBUF;
+      const uint32_t bph = (u / NBUF) & 1;
       bool got = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], bph, ctx, ERR_WAIT_TMEM_FULL));
       // the reduce-scatter epilogue ends in a named barrier of its 256 threads: one answer for all
       if (TP == 2) got = named_bar_and<1, 32 * PAIR_EPI_WARPS>(got);
@@ -441,45 +515,66 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
         break;
       }
       tc_fence_after_sync();
-      const int row = (2 * t.pm + int(cta)) * BM + q * 32 + lane;
       const uint32_t acc = tmem_base + uint32_t(buf * BN) + lane_addr;
+      // A slice's partial tile: one region per (tile, slice, CTA, warp), 16 bytes of consecutive lanes
+      // side by side.
+      constexpr int REGION = CHUNKS_PER_HALF * 8 * 32;
+      const int slot = (w.tile - p.whole_tiles) * p.split;   // of slice 0; only used with slices
+      const int wreg = int(cta) * PAIR_EPI_WARPS + (warp - 2);
+      auto region = [&](int slice) { return p.partial + ((long long)(slot + slice) * 2 * PAIR_EPI_WARPS + wreg) * REGION + lane; };
       // the TMEM load of chunk c + 1 is in flight while chunk c is converted and stored
       uint32_t r[32];
       tmem_ld_32x32b_x32(acc + c_begin * 32, r);
 #pragma unroll 1
       for (int c = c_begin; c < c_end; ++c) {
         tmem_ld_wait();
-        const int col0 = t.n_tile * BN + c * 32;
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
         if (c + 1 < c_end) tmem_ld_32x32b_x32(acc + (c + 1) * 32, r);
-        if (EPI == LF_EPI_BF16 && p.bias != nullptr) {
+        if (TP != 0 || w.slice < 0) {
+          store_chunk(t, c, v);
+        } else {
+          float4* dst = region(w.slice) + (c - c_begin) * 8 * 32;
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
+          for (int g = 0; g < 8; ++g) dst[g * 32] = make_float4(v[g * 4], v[g * 4 + 1], v[g * 4 + 2], v[g * 4 + 3]);
         }
-        if (row < p.M) {
-          // reduce-scatter: the partial tile stays in THIS GPU's stage [M, N]; the owner pulls it
-          __nv_bfloat16* out = (TP == 2) ? tp.rs_peer_stage[tp.rank] + (long long)row * p.N
-                                         : p.out + (long long)row * p.ldo;
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            const int col = col0 + g * 8;
-            if (col + 8 <= p.N) {
-              st_global_v4(out + col, pack_bf16x2(v[g * 8 + 0], v[g * 8 + 1]),
-                           pack_bf16x2(v[g * 8 + 2], v[g * 8 + 3]), pack_bf16x2(v[g * 8 + 4], v[g * 8 + 5]),
-                           pack_bf16x2(v[g * 8 + 6], v[g * 8 + 7]));
-            } else {
-              for (int j = 0; j < 8; ++j)
-                if (col + j < p.N) out[col + j] = __float2bfloat16(v[g * 8 + j]);
-            }
-          }
-        }
+        __syncwarp();   // the TMEM load above is .sync.aligned
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(&tempty[buf], 0));
+      if (TP == 0 && w.slice >= 0) {
+        // The warp that stores the last slice of its part of the tile adds all of them, in slice
+        // order: nobody waits, and the sum does not depend on who was last.
+        int before = 0;
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) before = atomicAdd(p.arrivals + (w.tile - p.whole_tiles) * 2 * PAIR_EPI_WARPS + wreg, 1);
+        before = __shfl_sync(0xffffffffu, before, 0);
+        if (before == p.split - 1) {
+          __threadfence();
+#pragma unroll 1
+          for (int c = c_begin; c < c_end; ++c) {
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = 0.f;
+#pragma unroll 2
+            for (int i = 0; i < p.split; ++i) {
+              const float4* src = region(i) + (c - c_begin) * 8 * 32;
+#pragma unroll
+              for (int g = 0; g < 8; ++g) {
+                const float4 f = __ldcg(src + g * 32);
+                v[g * 4] += f.x;
+                v[g * 4 + 1] += f.y;
+                v[g * 4 + 2] += f.z;
+                v[g * 4 + 3] += f.w;
+              }
+            }
+            store_chunk(t, c, v);
+          }
+        }
+      }
       if (TP == 2) {
         // all 256 epilogue threads of this CTA have stored their part of the 128 x 256 partial
         __threadfence_system();
@@ -630,6 +725,57 @@ static int launch(const Params& p, const CUtensorMap& tA, const CUtensorMap& tB,
 }  // namespace pair
 }  // namespace lf
 
+// How the last wave of `tiles` tiles over `pairs` CTA pairs is cut: the number of slices along the
+// reduction (1 = not at all).  Tiles of the last wave that leave pairs idle are computed in s slices,
+// s * tail units over the pairs, which takes ceil(s * tail / pairs) / s of a tile's time instead of
+// all of it.  Against that stand, in 64-deep blocks of the main loop (0.33 us each): 30 for clearing
+// the counters and for the last arrival's round trips, and 0.27 for each partial tile, 256 KB
+// stored and read back; slices are at least 8 blocks long.  Measured, us: dX of 300 x 4096 <- 14336
+// (32 tiles of 224 blocks) 78 -> 55; dX of 2048 x 4096 <- 128256 (128 tiles) 1770 -> 1460; with a
+// cost of 8 + 4 s blocks also products that lost were cut: 1000 x 8192 x 8192 107 -> 117.
+static int pick_split(int tiles, int pairs, int nkb) {
+  const int tail = tiles % pairs;
+  if (tail == 0) return 1;
+  int best = 1;
+  double best_gain = 8.0;   // blocks; less is not worth a second look
+  for (int s = 2; s <= 8 && nkb / s >= 8; ++s) {
+    const int waves = (tail * s + pairs - 1) / pairs;
+    const double gain = nkb * (1.0 - double(waves) / s) - (30.0 + 0.27 * tail * s);
+    if (gain > best_gain) {
+      best_gain = gain;
+      best = s;
+    }
+  }
+  return best;
+}
+
+static int pair_count(int max_ctas) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int pairs = sms / 2;
+  if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
+  return pairs < 1 ? 1 : pairs;
+}
+
+static int tile_count(int M, int N) {
+  using namespace lf::pair;
+  return ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
+}
+
+constexpr long long kPartialBytes = 256ll * 256 * 4;   // one fp32 tile
+static long long arrival_bytes(int tail) { return ((long long)tail * 2 * lf::pair::PAIR_EPI_WARPS * 4 + 255) / 256 * 256; }
+
+// Bytes of scratch lf_gemm_pair wants for a product of this size (0 = none): arrival counters, then
+// the partial tiles of the last wave.  Without that much it computes whole tiles only.
+extern "C" long long lf_gemm_pair_scratch(int M, int N, int K, int max_ctas) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const int tiles = tile_count(M, N), pairs = pair_count(max_ctas);
+  const int s = pick_split(tiles, pairs, (K + lf::pair::BK - 1) / lf::pair::BK);
+  const int tail = tiles % pairs;
+  return s > 1 ? arrival_bytes(tail) + (long long)tail * s * kPartialBytes : 0;
+}
+
 // Same argument struct as lf_gemm.  Supported: a / a2 K-major; b and b2 both K-major or both
 // MN-major; bn = 256; epilogues LF_EPI_BF16 (nacc 1) and LF_EPI_BF16_DROPMIX (callers pass nacc 2,
 // the layout of the single-CTA kernel; here the slab is masked in place in one accumulator); dense
@@ -643,6 +789,7 @@ static int pair_entry(const LfGemmArgs* a, const LfTpArgs* t) {
   const bool dropmix = a->epi == LF_EPI_BF16_DROPMIX && a->nacc == 2;
   if (!dropmix && !(a->epi == LF_EPI_BF16 && a->nacc == 1)) return -5;
   if (a->scale != 1.0f) return -5;
+  if (!gemm_out_aligned(a)) return -6;
 
   CUtensorMap tA, tB, tA2, tB2;
   int rc = make_tmap_2d_b16(&tA, a->a, a->a_rows, a->a_cols, a->a_ld, BM, 64, true);
@@ -698,15 +845,26 @@ static int pair_entry(const LfGemmArgs* a, const LfTpArgs* t) {
     p.m_rotate = (mode == 1 ? t->rank : (t->rank + 1) % t->world) * pairs_per_shard;
     if (pairs_per_shard < p.group_m) p.group_m = pairs_per_shard;
   }
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int pairs = sms / 2;
-  if (a->max_ctas > 0 && a->max_ctas / 2 < pairs) pairs = a->max_ctas / 2;
-  if (p.num_tiles < pairs) pairs = p.num_tiles;
-  if (pairs < 1) pairs = 1;
-  cudaStream_t st = (cudaStream_t)a->stream;
   if (dropmix && !a->b_mn) return -5;
+  cudaStream_t st = (cudaStream_t)a->stream;
+  int pairs = pair_count(a->max_ctas);
+  p.whole_tiles = p.num_tiles;
+  p.split = 1;
+  p.partial = nullptr;
+  p.arrivals = nullptr;
+  if (mode == 0 && a->scratch != nullptr) {
+    const int s = pick_split(p.num_tiles, pairs, p.nkb_main);
+    const int tail = p.num_tiles % pairs;
+    if (s > 1 && a->scratch_bytes >= arrival_bytes(tail) + (long long)tail * s * kPartialBytes) {
+      p.whole_tiles = p.num_tiles - tail;
+      p.split = s;
+      p.arrivals = (int*)a->scratch;
+      p.partial = (float4*)((char*)a->scratch + arrival_bytes(tail));
+      if (cudaMemsetAsync(a->scratch, 0, arrival_bytes(tail), st) != cudaSuccess) return -12;
+    }
+  }
+  const int units = p.whole_tiles + (p.num_tiles - p.whole_tiles) * p.split;
+  if (units < pairs) pairs = units;
 #define LF_PAIR_DISPATCH(TPV)                                                                                  \
   do {                                                                                                         \
     if (dropmix) return launch<true, LF_EPI_BF16_DROPMIX, TPV>(p, tA, tB, tA2, tB2, pairs, st, tp);         \

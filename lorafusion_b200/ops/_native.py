@@ -83,6 +83,8 @@ class LfGemmArgs(C.Structure):
         ("adapter_inv_keep", C.c_void_p),
         ("err", C.c_void_p),
         ("stream", C.c_void_p),
+        ("scratch", C.c_void_p),
+        ("scratch_bytes", C.c_int64),
         ("a_mn", C.c_int32), ("b_mn", C.c_int32), ("b2_mn", C.c_int32),
         ("M", C.c_int32), ("N", C.c_int32), ("K", C.c_int32), ("K2", C.c_int32),
         ("bn", C.c_int32), ("nacc", C.c_int32), ("epi", C.c_int32), ("mask_a", C.c_int32),
@@ -132,6 +134,8 @@ def _declare_cuda(lib: C.CDLL) -> None:
     lib.lf_gemm_pair.restype = C.c_int
     lib.lf_lora_skinny.argtypes = [C.POINTER(LfGemmArgs), C.c_int]
     lib.lf_lora_skinny.restype = C.c_int
+    lib.lf_gemm_pair_scratch.argtypes = [C.c_int] * 4
+    lib.lf_gemm_pair_scratch.restype = C.c_longlong
     lib.lf_gemm_nf4.argtypes = [C.POINTER(LfGemmArgs), C.POINTER(LfNf4Args)]
     lib.lf_gemm_nf4.restype = C.c_int
     for name, sig in _SIGNATURES.items():

@@ -9,6 +9,7 @@ a transpose copy.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 from typing import Optional
 
@@ -145,6 +146,38 @@ def set_pair_kernels(enabled: bool) -> None:
     _PAIR = bool(enabled)
 
 
+@functools.lru_cache(maxsize=4096)
+def _pair_is_faster(M: int, N: int, K: int, max_ctas: int, device: int) -> bool:
+    """Which kernel takes a product of fewer than ``_PAIR_MIN_ROWS`` rows with 256-wide tiles.  Both
+    walk the reduction in 64-deep blocks, the single-CTA one in 0.44 us a block (it loads a whole
+    B tile per SM), a pair in 0.37 us, but over half as many, twice as high tiles at a time and with
+    3 us more around them; a last wave cut along the reduction is the pairs' alone."""
+    if _pair_scratch_bytes(M, N, K, max_ctas, device):
+        return True
+    sms = 148 if max_ctas <= 0 else min(148, max_ctas)
+    n_tiles, blocks = -(-N // 256), -(-K // 64)
+    single = -(-(-(-M // 128) * n_tiles) // sms) * blocks * 0.44
+    pairs = -(-(-(-M // 256) * n_tiles) // max(1, sms // 2)) * blocks * 0.37
+    return pairs + 3.0 < single
+
+
+def use_pair(M: int, N: int, K: int, max_ctas: int, device: torch.device) -> bool:
+    """Whether a product goes to the CTA-pair kernels (given 256-wide tiles)."""
+    return _PAIR and (M >= _PAIR_MIN_ROWS or _pair_is_faster(M, N, K, max_ctas, device.index or 0))
+
+
+@functools.lru_cache(maxsize=4096)
+def _pair_scratch_bytes(M: int, N: int, K: int, max_ctas: int, device: int) -> int:
+    return int(nv.cuda_lib().lf_gemm_pair_scratch(M, N, K, max_ctas))
+
+
+def pair_scratch(M: int, N: int, K: int, max_ctas: int, device: torch.device) -> Optional[torch.Tensor]:
+    """Scratch of one CTA-pair product (the last wave of its tiles may be cut along the
+    reduction), for this launch on the current stream alone; ``None`` when it needs none."""
+    n = _pair_scratch_bytes(M, N, K, max_ctas, device.index or 0)
+    return torch.empty(n, dtype=torch.uint8, device=device) if n else None
+
+
 def launch_gemm(pair: Optional[bool] = None, **kwargs) -> None:
     """Fill :class:`LfGemmArgs` (see :func:`fill_gemm_args`) and launch on the current stream.
     ``pair`` overrides the module default for trying the CTA-pair kernel first.  When ``b`` is
@@ -162,9 +195,12 @@ def launch_gemm(pair: Optional[bool] = None, **kwargs) -> None:
         if rc != 0:
             raise RuntimeError(f"lf_gemm_nf4 failed with code {rc}")
         return
-    use_pair = _PAIR if pair is None else pair
-    if use_pair and args.bn == 256 and args.M >= _PAIR_MIN_ROWS and not args.a_mn and not args.mask_a \
-            and not args.seg_tiles:
+    if args.bn == 256 and not args.a_mn and not args.mask_a and not args.seg_tiles and (
+            use_pair(args.M, args.N, args.K, args.max_ctas, kwargs["a"].device) if pair is None
+            else pair and args.M >= _PAIR_MIN_ROWS):
+        scratch = pair_scratch(args.M, args.N, args.K, args.max_ctas, kwargs["a"].device)
+        if scratch is not None:
+            args.scratch, args.scratch_bytes = scratch.data_ptr(), scratch.numel()
         rc = lib.lf_gemm_pair(C.byref(args))
         if rc == 0:
             return

@@ -71,6 +71,42 @@ def test_philox_with_row_and_column_parts_taken_out_drops_everything_at_p_near_o
     assert not s.any()
 
 
+@pytest.mark.parametrize("M,N,K,ctas", [(600, 1104, 16392, 8), (1000, 2816, 6000, 20), (513, 256, 5000, 0)])
+@pytest.mark.parametrize("p", [None, 0.0, 0.1])
+def test_pair_products_with_the_last_wave_cut(M, N, K, ctas, p):
+    """Forward (``p`` None, with bias) and dX products of the CTA-pair kernels whose last wave is cut
+    along the reduction: same results as fp32 math, twice the same bits."""
+    from lorafusion_b200.ops import _native as nv
+    from lorafusion_b200.ops.gemm import _pair_scratch_bytes, launch_gemm
+    from lorafusion_b200.ops.philox import dropout_threshold, keep_mask
+
+    assert _pair_scratch_bytes(M, N, K, ctas, 0) > 0, "the case is meant to be cut"
+    R = 64
+    x, s = _rand(M, K, seed=1), _rand(M, R, scale=0.2, seed=2)
+    w = _rand(N, K, scale=0.03, seed=3) if p is None else _rand(K, N, scale=0.03, seed=3)
+    b2 = _rand(N, R, scale=0.2, seed=4) if p is None else _rand(R, N, scale=0.2, seed=4)
+    bias = _rand(N, seed=5) if p is None else None
+    kw = dict(a=x, b=w, M=M, N=N, K=K, bn=256, a2=s, b2=b2, K2=R, max_ctas=ctas, pair=True)
+    if p is None:
+        kw.update(bias=bias, b2_adapter_rows=N)
+        ref = _f32mm(x, w.t()) + _f32mm(s, b2.t()) + bias.float()
+    else:
+        kw.update(b_mn=True, b2_mn=True, b2_adapter_rows=R)
+        slab = _f32mm(s, b2)
+        if p > 0:
+            kw.update(nacc=2, epi=nv.EPI_BF16_DROPMIX, thresh16=dropout_threshold(p), inv_keep=1 / (1 - p), seed=7,
+                      stream_id=2)
+            slab = torch.where(keep_mask(M, N, p, 7, 2).cuda(), slab / (1 - p), torch.zeros((), device="cuda"))
+        ref = _f32mm(x, w) + slab
+    outs = []
+    for _ in range(2):
+        out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+        launch_gemm(out=out, **kw)
+        outs.append(out)
+    assert torch.equal(*outs)
+    assert_close_two_rounds(outs[0], ref, msg=f"pair product {M} x {N} x {K}")
+
+
 @pytest.mark.parametrize("lens,Hq,Hkv", [([1], 1, 1), ([129, 3, 128], 3, 1), ([300, 257], 10, 2), ([700, 31, 513], 8, 1),
                                          ([128] * 150, 5, 1)])
 def test_attention_head_groups(lens, Hq, Hkv):
