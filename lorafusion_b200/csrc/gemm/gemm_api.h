@@ -116,6 +116,49 @@ int lf_gemm_tp_nf4(const LfGemmArgs* args, const LfTpArgs* tp, const LfNf4Args* 
 // The rank-wide LoRA products (see lora_skinny.cu); `split` CTAs share the reduction of a tile.
 int lf_lora_skinny(const LfGemmArgs* args, int split);
 
+// One adapter of lf_lora_pack / lf_lora_unpack: A [r, K] (row pitch a_ld), B [N, r] (row pitch b_ld),
+// bf16; r = 0 with null pointers for a missing adapter.
+#define LF_LORA_PIECES 16
+typedef struct LfLoraPiece {
+  const void* a;
+  const void* b;
+  int64_t a_ld, b_ld, r;
+} LfLoraPiece;
+
+// A whole LoRA linear layer (see lora_linear.cu).  All matrices row-major, contiguous but for the
+// row pitches given; stacks [n_adapters, R, K] and [n_adapters, N, R].  tile_adapter and seg_rows may
+// both be null: then every token belongs to adapter 0 (num_segs = 1).
+typedef struct LfLoraLinearArgs {
+  const void* x;
+  const void* w;
+  const void* bias;
+  const void* a_all;
+  const void* b_all;
+  void* s;
+  void* y;
+  const void* dy;
+  void* ds;
+  void* da;
+  void* db;
+  void* dx;
+  const int32_t* tile_adapter;
+  const int32_t* seg_rows;
+  const float* adapter_scale;
+  const uint32_t* adapter_thresh16;
+  const float* adapter_inv_keep;
+  int32_t* err;
+  void* stream;
+  void* scratch;          // of the Y (forward) or dX (backward) product, see lf_gemm_pair_scratch
+  int64_t scratch_bytes;
+  int64_t x_ld, w_ld, dy_ld;
+  int32_t M, K, N, R, n_adapters, num_segs, have_s, dropout;
+  int32_t split_s, split_ds, split_db, split_da;
+  int32_t pair;           // try the CTA-pair kernels first for the big product of this call
+  int32_t fwd_group_m, fwd_max_ctas, dx_group_m, dx_max_ctas, dropmix_bn;
+  float scale, inv_keep;
+  uint32_t thresh16, seed_lo, seed_hi, stream_id;
+} LfLoraLinearArgs;
+
 #ifdef __cplusplus
 }
 #endif

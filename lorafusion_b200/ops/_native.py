@@ -100,6 +100,23 @@ class LfGemmArgs(C.Structure):
     ]
 
 
+class LfLoraPiece(C.Structure):
+    _fields_ = [("a", C.c_void_p), ("b", C.c_void_p), ("a_ld", C.c_int64), ("b_ld", C.c_int64), ("r", C.c_int64)]
+
+
+class LfLoraLinearArgs(C.Structure):
+    _fields_ = (
+        [(f, C.c_void_p) for f in ("x", "w", "bias", "a_all", "b_all", "s", "y", "dy", "ds", "da", "db", "dx",
+                                   "tile_adapter", "seg_rows", "adapter_scale", "adapter_thresh16",
+                                   "adapter_inv_keep", "err", "stream", "scratch")]
+        + [(f, C.c_int64) for f in ("scratch_bytes", "x_ld", "w_ld", "dy_ld")]
+        + [(f, C.c_int32) for f in ("M", "K", "N", "R", "n_adapters", "num_segs", "have_s", "dropout",
+                                    "split_s", "split_ds", "split_db", "split_da", "pair",
+                                    "fwd_group_m", "fwd_max_ctas", "dx_group_m", "dx_max_ctas", "dropmix_bn")]
+        + [("scale", C.c_float), ("inv_keep", C.c_float)]
+        + [(f, C.c_uint32) for f in ("thresh16", "seed_lo", "seed_hi", "stream_id")])
+
+
 EPI_BF16 = 0
 EPI_BF16_DROPMIX = 1
 EPI_F32_ACCUM = 2
@@ -109,6 +126,8 @@ EPI_BF16_ADAPTER_SCALE = 3
 _VP, _LL, _I, _F = C.c_void_p, C.c_longlong, C.c_int, C.c_float
 
 _SIGNATURES = {
+    "lf_lora_pack": [_VP, _I, _VP, _VP, _I, _I, _I, _VP],
+    "lf_lora_unpack": [_VP, _I, _VP, _VP, _I, _I, _I, _VP],
     "lf_rmsnorm_fwd": [_VP, _VP, _VP, _VP, _VP, _VP, _LL, _I, _F, _VP],
     "lf_rmsnorm_bwd": [_VP, _VP, _VP, _VP, _VP, _VP, _LL, _I, _VP],
     "lf_rope_inplace": [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _VP],
@@ -132,6 +151,10 @@ def _declare_cuda(lib: C.CDLL) -> None:
     lib.lf_gemm.restype = C.c_int
     lib.lf_gemm_pair.argtypes = [C.POINTER(LfGemmArgs)]
     lib.lf_gemm_pair.restype = C.c_int
+    lib.lf_lora_linear_fwd.argtypes = [C.POINTER(LfLoraLinearArgs)]
+    lib.lf_lora_linear_fwd.restype = C.c_int
+    lib.lf_lora_linear_bwd.argtypes = [C.POINTER(LfLoraLinearArgs)]
+    lib.lf_lora_linear_bwd.restype = C.c_int
     lib.lf_lora_skinny.argtypes = [C.POINTER(LfGemmArgs), C.c_int]
     lib.lf_lora_skinny.restype = C.c_int
     lib.lf_gemm_pair_scratch.argtypes = [C.c_int] * 4
@@ -206,4 +229,4 @@ def check_device_errors(device=None, *, reset: bool = True) -> None:
 
 
 def current_stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())

@@ -30,7 +30,7 @@ from typing import Optional, Sequence, Union
 import torch
 
 from . import lora_kernels as lk
-from .batch_info import MultiLoRABatchInfo, prepare_multi_lora_batch_info, single_adapter_batch_info
+from .batch_info import MultiLoRABatchInfo, prepare_multi_lora_batch_info
 from .nf4 import NF4Weight, dequantize_nf4
 from .reference import torch_ref_linear_lora, torch_ref_linear_multi_lora
 
@@ -157,10 +157,14 @@ def lora_linear_forward(x: torch.Tensor, w: Weight, stack: Optional[LoRAStack],
         return _unfused_forward(x, wd, stack, info, stream_id, bias, training)
     if stack is None or info is None:
         return lk.base_lora_fwd(x, wd, None, None, tile_adapter=None, bias=bias), None
-    if s is None or isinstance(s, list):
-        drop = info.dropout_spec(stream_id, training)
+    if isinstance(s, list):
+        s = None
+    drop = info.dropout_spec(stream_id, training)
+    if not isinstance(wd, NF4Weight):
+        return lk.linear_fwd(x, wd, stack.a, stack.b, info, drop, bias=bias, s=s)
+    if s is None:
         s = lk.lora_down(x, stack.a, tile_adapter=info.tile_adapter, adapter_scale=info.adapter_scale,
-                         dropout=drop)
+                         scale=getattr(info, "scale", 1.0), dropout=drop)
     y = lk.base_lora_fwd(x, wd, s, stack.b, tile_adapter=info.tile_adapter, bias=bias)
     return y, s
 
@@ -175,61 +179,79 @@ def lora_linear_backward(dy: torch.Tensor, x: torch.Tensor, s: Optional[torch.Te
     if stack is None or info is None or s is None:
         return lk.base_lora_dx(dy, wd, None, None, tile_adapter=None) if need_dx else None
     drop = info.dropout_spec(stream_id, training)
-    ds = lk.lora_ds(dy, stack.b, tile_adapter=info.tile_adapter, adapter_scale=info.adapter_scale)
+    if not isinstance(wd, NF4Weight):
+        return lk.linear_bwd(dy, x, s, wd if need_dx else None, stack.a, stack.b, info, drop, stack.da, stack.db, need_dx)
+    ds = lk.lora_ds(dy, stack.b, tile_adapter=info.tile_adapter, adapter_scale=info.adapter_scale,
+                    scale=getattr(info, "scale", 1.0))
+    segs = info.segment_table if info.tile_adapter is not None else \
+        lk.SegmentTable(info.segments, dy.device, total_rows=dy.shape[0])
     if stack.db is not None:
-        lk.lora_db(dy, s, info.segment_table, stack.db)
+        lk.lora_db(dy, s, segs, stack.db)
     if stack.da is not None:
-        lk.lora_da(x, ds, info.segment_table, stack.da, dropout=drop)
+        lk.lora_da(x, ds, segs, stack.da, dropout=drop)
     if not need_dx:
         return None
     return lk.base_lora_dx(dy, wd, ds, stack.a, tile_adapter=info.tile_adapter, dropout=drop)
 
 
 class _FusedLoRAFunction(torch.autograd.Function):
-    """Autograd node over the functional forward/backward.  ``a_stack`` / ``b_stack`` are the
-    padded stacks ``[n, R, K]`` / ``[n, N, R]``; their gradients are returned in their dtype."""
+    """Autograd node over the functional forward/backward.  ``ab`` = the adapters' ``A [r, K]``, then
+    their ``B [N, r]`` (``None`` for a missing adapter): one kernel lays them out as padded stacks,
+    one takes the gradient stacks apart, so that no tensor operation runs per adapter."""
 
     @staticmethod
-    def forward(ctx, x2d, w, bias, a_stack, b_stack, info, stream_id, training):
-        stack = LoRAStack(a_stack.detach(), b_stack.detach())
+    def forward(ctx, x2d, w, bias, info, stream_id, training, *ab):
+        n = len(ab) // 2
+        K, N = x2d.shape[1], w.shape[0]
+        entries = [_adapter_entry(a, b, K, N, x2d.device) for a, b in zip(ab[:n], ab[n:])]
+        R = rank_pad(max(max(e[2] for e in entries), 1))
+        stack = LoRAStack(*lk.pack_stacks(entries, K, N, R, x2d.device))
         y, s = lora_linear_forward(x2d, w, stack, info, stream_id=stream_id, bias=bias,
                                    training=training)
-        ctx.save_for_backward(x2d, s, a_stack, b_stack)
+        ctx.save_for_backward(x2d, s, stack.a, stack.b)
         ctx.w, ctx.info, ctx.stream_id, ctx.training = w, info, stream_id, training
+        ctx.meta = [None if t is None else (t.dtype, e[2]) for t, e in zip(ab, entries * 2)]
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x2d, s, a_stack, b_stack = ctx.saved_tensors
+        x2d, s, a_all, b_all = ctx.saved_tensors
         dy = dy.contiguous()
-        need_a, need_b = ctx.needs_input_grad[3], ctx.needs_input_grad[4]
-        stack = LoRAStack(
-            a_stack.detach(), b_stack.detach(),
-            torch.zeros(a_stack.shape, dtype=torch.float32, device=dy.device) if need_a else None,
-            torch.zeros(b_stack.shape, dtype=torch.float32, device=dy.device) if need_b else None)
+        n, R, K = a_all.shape
+        N = b_all.shape[1]
+        need = ctx.needs_input_grad[6:]
+        na = n * R * K if any(need[:n]) else 0
+        nb = n * R * N if any(need[n:]) else 0
+        flat = torch.zeros(na + nb, dtype=torch.float32, device=dy.device) if na + nb else None
+        stack = LoRAStack(a_all, b_all, flat[:na].view(n, R, K) if na else None,
+                          flat[na:].view(n, N, R) if nb else None)
         dx = lora_linear_backward(dy, x2d, s, ctx.w, stack, ctx.info, stream_id=ctx.stream_id,
                                   need_dx=ctx.needs_input_grad[0], training=ctx.training)
-        da = stack.da.to(a_stack.dtype) if need_a else None
-        db = stack.db.to(b_stack.dtype) if need_b else None
+        grads = [None] * (2 * n)
+        for i, want in enumerate(need):
+            if want:
+                r = ctx.meta[i][1]
+                grads[i] = torch.empty((r, K) if i < n else (N, r), dtype=torch.bfloat16, device=dy.device)
+        if na + nb:
+            ranks = [0 if m is None else m[1] for m in ctx.meta[:n]]
+            lk.unpack_grads(list(zip(grads[:n], grads[n:], ranks)), stack.da, stack.db, K, N, R)
+            grads = [g if g is None or m[0] == g.dtype else g.to(m[0]) for g, m in zip(grads, ctx.meta)]
         dbias = dy.float().sum(0).to(dy.dtype) if ctx.needs_input_grad[2] else None
-        return dx, None, dbias, da, db, None, None, None
+        return (dx, None, dbias, None, None, None, *grads)
 
 
-def _pad_stack(a_list: Sequence[Optional[torch.Tensor]], b_list: Sequence[Optional[torch.Tensor]],
-               K: int, N: int, device, dtype=torch.bfloat16):
-    """Differentiable stacking of per-adapter ``A [r, K]`` / ``B [N, r]`` into padded stacks."""
-    ranks = [a.shape[0] for a in a_list if a is not None]
-    R = rank_pad(max(ranks) if ranks else 1)
-    a_rows, b_rows = [], []
-    for a, b in zip(a_list, b_list):
-        if a is None:
-            a_rows.append(torch.zeros(R, K, dtype=dtype, device=device))
-            b_rows.append(torch.zeros(N, R, dtype=dtype, device=device))
-        else:
-            r = a.shape[0]
-            a_rows.append(torch.nn.functional.pad(a.to(dtype), (0, 0, 0, R - r)))
-            b_rows.append(torch.nn.functional.pad(b.to(dtype), (0, R - r)))
-    return torch.stack(a_rows), torch.stack(b_rows)
+def _adapter_entry(a: Optional[torch.Tensor], b: Optional[torch.Tensor], K: int, N: int, device) -> tuple:
+    """``(A, B, rank)`` of one adapter as the packing kernel reads them: bf16 on ``device`` with a
+    contiguous last dimension."""
+    if a is None:
+        return None, None, 0
+    r = a.shape[0]
+    if tuple(a.shape) != (r, K) or tuple(b.shape) != (N, r):
+        raise ValueError(f"adapter shapes A {tuple(a.shape)}, B {tuple(b.shape)} do not fit a [{N}, {K}] layer")
+    if a.device != device or b.device != device:
+        raise ValueError(f"adapter on {a.device} / {b.device}, input on {device}")
+    a, b = (t if t.dtype == torch.bfloat16 else t.to(torch.bfloat16) for t in (a, b))
+    return a if a.stride(1) == 1 else a.contiguous(), b if b.stride(1) == 1 else b.contiguous(), r
 
 
 def fused_linear_lora(x: torch.Tensor, linear_w: Weight, lora_a: torch.Tensor,
@@ -245,13 +267,9 @@ def fused_linear_lora(x: torch.Tensor, linear_w: Weight, lora_a: torch.Tensor,
                                      stream_id, linear_bias)
     shape = x.shape
     x2d = x.reshape(-1, shape[-1]).contiguous()
-    N = lora_b.shape[0]
-    a_stack, b_stack = _pad_stack([lora_a], [lora_b], shape[-1], N, x.device)
-    info = single_adapter_batch_info(x2d.shape[0], lora_a.shape[0], alpha, dropout_p,
-                                     device=x.device, seed=seed)
-    y = _FusedLoRAFunction.apply(x2d, linear_w, linear_bias, a_stack, b_stack, info, stream_id,
-                                 dropout_p > 0.0)
-    return y.reshape(*shape[:-1], N)
+    info = lk.OneAdapter(x2d.shape[0], float(alpha), float(dropout_p), seed)
+    y = _FusedLoRAFunction.apply(x2d, linear_w, linear_bias, info, stream_id, dropout_p > 0.0, lora_a, lora_b)
+    return y.reshape(*shape[:-1], lora_b.shape[0])
 
 
 def fused_linear_multi_lora(
@@ -305,8 +323,9 @@ def fused_linear_multi_lora(
             seed=info.seed, stream_id=stream_id, linear_bias=linear_bias)
     shape = padded_x.shape
     x2d = padded_x.reshape(-1, shape[-1]).contiguous()
-    N = linear_w.shape[0]
-    a_stack, b_stack = _pad_stack(lora_a_list, lora_b_list, shape[-1], N, padded_x.device)
-    y = _FusedLoRAFunction.apply(x2d, linear_w, linear_bias, a_stack, b_stack, info, stream_id,
-                                 enable_dropout)
-    return y.reshape(*shape[:-1], N)
+    n = min(len(lora_a_list), len(lora_b_list))
+    if n == 0:
+        raise ValueError("at least one adapter entry is required")
+    y = _FusedLoRAFunction.apply(x2d, linear_w, linear_bias, info, stream_id, enable_dropout,
+                                 *lora_a_list[:n], *lora_b_list[:n])
+    return y.reshape(*shape[:-1], linear_w.shape[0])

@@ -32,6 +32,7 @@ Conventions
 
 from __future__ import annotations
 
+import ctypes as C
 import functools
 from dataclasses import dataclass, field
 from typing import Optional, Sequence
@@ -39,8 +40,9 @@ from typing import Optional, Sequence
 import torch
 
 from . import _native as nv
-from .gemm import launch_gemm, launch_skinny
+from .gemm import check2d, launch_gemm, launch_skinny, pair_scratch, use_pair
 from .philox import dropout_threshold
+from .tile_config import get_kernel_config
 
 RANK_PAD = 64
 RANK_PADS = (64, 128, 192, 256)  # stacked-rank widths the skinny kernels are built for
@@ -239,6 +241,167 @@ def lora_da(x: torch.Tensor, ds: torch.Tensor, segs: SegmentTable, da_all: torch
     launch_skinny(segs.chunks(K), a=x, b=ds, out=da_all, M=K, N=R, K=M, a_mn=True, b_mn=True, bn=R,
                   epi=nv.EPI_F32_ACCUM, mask_a=dropout.active, seg_tiles=rows, ldo=K,
                   out_transposed=True, out_adapter_stride=R * K, **dropout.kwargs())
+
+
+@dataclass
+class OneAdapter:
+    """Every token belongs to adapter 0: what the kernels need to know of a batch in that case,
+    without any table on the device (:class:`~.batch_info.MultiLoRABatchInfo` is the general one)."""
+
+    tokens: int
+    scale: float
+    p: float
+    seed: int
+    tile_adapter = None
+    adapter_scale = None
+
+    @property
+    def segments(self) -> list:
+        return [(0, 0, self.tokens)]
+
+    @property
+    def alpha_by_adapter(self) -> dict:
+        return {0: self.scale}
+
+    @property
+    def dropout_by_adapter(self) -> dict:
+        return {0: self.p}
+
+    def dropout_spec(self, stream_id: int, training: bool = True) -> DropoutSpec:
+        return DropoutSpec(seed=self.seed, stream_id=stream_id, p=self.p) if training and self.p > 0 else NO_DROPOUT
+
+
+def _linear_args(x: torch.Tensor, w: Optional[torch.Tensor], a_all: torch.Tensor, b_all: torch.Tensor, info,
+                 drop: DropoutSpec, **fields) -> nv.LfLoraLinearArgs:
+    """Describe one LoRA linear layer (``lf_lora_linear_fwd`` / ``_bwd``) for the current stream."""
+    M, K = x.shape
+    n, R, K2 = a_all.shape
+    n2, N, R2 = b_all.shape
+    if K2 != K or (n2, R2) != (n, R) or R not in RANK_PADS or (w is not None and tuple(w.shape) != (N, K)):
+        raise ValueError(f"shapes do not match: x {tuple(x.shape)}, w {None if w is None else tuple(w.shape)}, "
+                         f"A {tuple(a_all.shape)}, B {tuple(b_all.shape)}")
+    check2d(x, "x")
+    if w is not None:   # (a backward that wants no dX does not read it)
+        check2d(w, "w")
+        fields.update(w=w.data_ptr(), w_ld=w.stride(0))
+    if "y" in fields:
+        cfg = get_kernel_config("fwd", M, K, N)
+        fields.update(fwd_group_m=cfg.group_m, fwd_max_ctas=cfg.max_ctas)
+    else:
+        cfg = get_kernel_config("dx_dropout" if drop.active else "dx", M, N, K)
+        fields.update(dx_group_m=cfg.group_m, dx_max_ctas=cfg.max_ctas)
+    args = nv.LfLoraLinearArgs(
+        x=x.data_ptr(), a_all=a_all.data_ptr(), b_all=b_all.data_ptr(), x_ld=x.stride(0),
+        err=nv.err_word(x.device).data_ptr(), stream=nv.current_stream_ptr(),
+        M=M, K=K, N=N, R=R, n_adapters=n,
+        dropmix_bn=DROPMIX_BN, scale=getattr(info, "scale", 1.0), **fields)
+    if info.tile_adapter is not None:
+        args.tile_adapter = info.tile_adapter.data_ptr()
+        args.adapter_scale = info.adapter_scale.data_ptr()
+    if drop.active:
+        args.dropout = 1
+        args.thresh16 = dropout_threshold(drop.p)
+        args.inv_keep = 1.0 / (1.0 - drop.p) if drop.p > 0 else 1.0
+        if drop.adapter_thresh16 is not None:
+            args.adapter_thresh16 = drop.adapter_thresh16.data_ptr()
+            args.adapter_inv_keep = drop.adapter_inv_keep.data_ptr()
+        args.seed_lo, args.seed_hi = drop.seed & 0xFFFFFFFF, (drop.seed >> 32) & 0xFFFFFFFF
+        args.stream_id = drop.stream_id & 0xFFFFFFFF
+    return args
+
+
+def _pair_setup(args: nv.LfLoraLinearArgs, M: int, N: int, K: int, max_ctas: int, device) -> Optional[torch.Tensor]:
+    """Route the layer's big product (256-wide tiles) and give it the scratch it wants."""
+    if N < 256 or not use_pair(M, N, K, max_ctas, device):
+        return None
+    args.pair = 1
+    scratch = pair_scratch(M, N, K, max_ctas, device)
+    if scratch is not None:
+        args.scratch, args.scratch_bytes = scratch.data_ptr(), scratch.numel()
+    return scratch
+
+
+def linear_fwd(x: torch.Tensor, w: torch.Tensor, a_all: torch.Tensor, b_all: torch.Tensor, info, drop: DropoutSpec,
+               bias: Optional[torch.Tensor] = None, s: Optional[torch.Tensor] = None):
+    """``lora_down`` (unless ``s`` is given) and ``base_lora_fwd`` in one call: ``(y, s)``."""
+    M, K = x.shape
+    N, R = b_all.shape[1:]
+    have_s = s is not None
+    if not have_s:
+        s = torch.empty((M, R), dtype=torch.bfloat16, device=x.device)
+    y = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
+    args = _linear_args(x, w, a_all, b_all, info, drop, s=s.data_ptr(), y=y.data_ptr(), have_s=int(have_s),
+                        bias=None if bias is None else bias.data_ptr(), split_s=_rows_split(M, K))
+    scratch = _pair_setup(args, M, N, K, args.fwd_max_ctas, x.device)
+    nv.note_launch(1 if have_s else 2)
+    rc = nv.cuda_lib().lf_lora_linear_fwd(C.byref(args))
+    if rc != 0:
+        raise RuntimeError(f"lf_lora_linear_fwd failed with code {rc}")
+    del scratch   # back to the allocator, in stream order, once the launch is queued
+    return y, s
+
+
+def linear_bwd(dy: torch.Tensor, x: torch.Tensor, s: torch.Tensor, w: Optional[torch.Tensor], a_all: torch.Tensor,
+               b_all: torch.Tensor, info, drop: DropoutSpec, da: Optional[torch.Tensor], db: Optional[torch.Tensor],
+               need_dx: bool) -> Optional[torch.Tensor]:
+    """``lora_ds``, ``lora_db`` into ``db``, ``lora_da`` into ``da`` and ``base_lora_dx`` in one call."""
+    M, N = dy.shape
+    K, R = x.shape[1], s.shape[1]
+    check2d(dy, "dy")
+    ds = torch.empty((M, R), dtype=torch.bfloat16, device=dy.device)
+    dx = torch.empty((M, K), dtype=torch.bfloat16, device=dy.device) if need_dx else None
+    if info.tile_adapter is None:
+        seg_rows, num_segs = None, 1
+        split_da, split_db = (reduction_split((f + TILE_M - 1) // TILE_M, (M + 63) // 64) for f in (K, N))
+    else:
+        rows = info.segment_table.device_rows()
+        seg_rows, num_segs = rows.data_ptr(), rows.shape[0]
+        split_da, split_db = info.segment_table.chunks(K), info.segment_table.chunks(N)
+    args = _linear_args(x, w, a_all, b_all, info, drop, dy=dy.data_ptr(), dy_ld=dy.stride(0), s=s.data_ptr(),
+                        ds=ds.data_ptr(), da=None if da is None else da.data_ptr(),
+                        db=None if db is None else db.data_ptr(), dx=None if dx is None else dx.data_ptr(),
+                        seg_rows=seg_rows, num_segs=num_segs, split_ds=_rows_split(M, N), split_db=split_db,
+                        split_da=split_da)
+    scratch = _pair_setup(args, M, K, N, args.dx_max_ctas, dy.device) if need_dx else None
+    nv.note_launch(1 + (da is not None) + (db is not None) + need_dx)
+    rc = nv.cuda_lib().lf_lora_linear_bwd(C.byref(args))
+    if rc != 0:
+        raise RuntimeError(f"lf_lora_linear_bwd failed with code {rc}")
+    del scratch
+    return dx
+
+
+def _pieces(entries: Sequence[tuple]):
+    """C array of ``(a, b, r)`` adapter entries (tensors or ``None``)."""
+    arr = (nv.LfLoraPiece * len(entries))()
+    for e, (a, b, r) in zip(arr, entries):
+        if a is not None:
+            e.a, e.a_ld = a.data_ptr(), a.stride(0)
+        if b is not None:
+            e.b, e.b_ld = b.data_ptr(), b.stride(0)
+        e.r = r
+    return arr
+
+
+def pack_stacks(entries: Sequence[tuple], K: int, N: int, R: int, device):
+    """``(A, B, r)`` per adapter (bf16 ``[r, K]`` / ``[N, r]`` with a contiguous last dimension, or
+    ``(None, None, 0)``) -> zero-padded stacks ``[n, R, K]``, ``[n, N, R]``."""
+    n = len(entries)
+    flat = torch.empty(n * R * (K + N), dtype=torch.bfloat16, device=device)
+    a_all, b_all = flat[:n * R * K].view(n, R, K), flat[n * R * K:].view(n, N, R)
+    nv.call("lf_lora_pack", C.addressof(arr := _pieces(entries)), n, a_all.data_ptr(), b_all.data_ptr(), R, K, N,
+            nv.current_stream_ptr())
+    del arr
+    return a_all, b_all
+
+
+def unpack_grads(entries: Sequence[tuple], da: Optional[torch.Tensor], db: Optional[torch.Tensor], K: int, N: int,
+                 R: int) -> None:
+    """fp32 gradient stacks -> the bf16 tensors of ``entries`` (contiguous ``[r, K]`` / ``[N, r]``)."""
+    nv.call("lf_lora_unpack", C.addressof(arr := _pieces(entries)), len(entries),
+            None if da is None else da.data_ptr(), None if db is None else db.data_ptr(), R, K, N,
+            nv.current_stream_ptr())
+    del arr
 
 
 def base_lora_dx(dy: torch.Tensor, w: torch.Tensor, ds: Optional[torch.Tensor],

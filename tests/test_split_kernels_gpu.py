@@ -152,3 +152,39 @@ def test_nf4_codes_at_the_midpoints():
     assert torch.allclose(nf4.dequantize_nf4(q_gpu).float(), ref.float(), rtol=1e-2, atol=1e-6)
     w[0, 5] = float("nan")
     assert int(nf4.quantize_nf4(w.cuda()).packed[0, 2]) & 15 == 0
+
+
+@pytest.mark.parametrize("n", [1, 17])
+def test_adapters_are_packed_and_gradients_unpacked(n):
+    """Rank 4 to 40, a missing adapter, an unaligned and a strided and an fp32 source; more adapters than
+    one launch takes."""
+    from lorafusion_b200.ops import lora_kernels as lk
+    from lorafusion_b200.ops.lora import _adapter_entry
+
+    K, N, R = 200, 72, 64
+    dev = torch.device("cuda", torch.cuda.current_device())
+    ab = []
+    for i in range(n):
+        r = (4, 40, 9)[i % 3]
+        a, b = _rand(r, K, seed=i), _rand(N, r, seed=100 + i)
+        if i % 4 == 1:
+            a = _rand(r, K + 1, seed=i)[:, 1:]
+        if i % 4 == 2:
+            a, b = a.float(), _rand(r, N, seed=100 + i).t()
+        ab.append((None, None) if i == 3 else (a, b))
+    entries = [_adapter_entry(a, b, K, N, dev) for a, b in ab]
+    a_all, b_all = lk.pack_stacks(entries, K, N, R, dev)
+    da, db = torch.randn(n, R, K, device=dev), torch.randn(n, N, R, device=dev)
+    grads = [(None, None, 0) if a is None else (torch.empty(a.shape, dtype=torch.bfloat16, device=dev),
+                                                None if i == 0 else torch.empty(b.shape, dtype=torch.bfloat16, device=dev),
+                                                a.shape[0]) for i, (a, b) in enumerate(ab)]
+    lk.unpack_grads(grads, da, db, K, N, R)
+    for i, (a, b) in enumerate(ab):
+        ra, rb = torch.zeros(R, K, device=dev), torch.zeros(N, R, device=dev)
+        if a is not None:
+            r = a.shape[0]
+            ra[:r], rb[:, :r] = a.float(), b.float()
+            assert torch.equal(grads[i][0], da[i, :r].to(torch.bfloat16))
+            assert grads[i][1] is None or torch.equal(grads[i][1], db[i, :, :r].to(torch.bfloat16))
+        assert torch.equal(a_all[i].float(), ra.to(torch.bfloat16).float())
+        assert torch.equal(b_all[i].float(), rb.to(torch.bfloat16).float())
