@@ -1,7 +1,8 @@
 """Kernel-level building blocks of the fused (multi-)LoRA linear layer.
 
-Every function here is one launch of the tcgen05 GEMM template with a different operand
-layout / epilogue; together they replace the reference's Triton kernels K1-K11 and its
+The functions of the table are one launch each, of the tcgen05 GEMM kernels or of the rank-wide
+kernel (``csrc/gemm/lora_skinny.cu``); ``linear_fwd`` / ``linear_bwd`` issue a whole layer's launches
+in one native call.  Together they replace the reference's Triton kernels K1-K11 and its
 cuBLAS calls for the skinny products (``lorafusion/ops/lora_v1.py:87-166``,
 ``lorafusion/ops/multi_lora.py:456-600``):
 

@@ -188,3 +188,36 @@ def test_adapters_are_packed_and_gradients_unpacked(n):
             assert grads[i][1] is None or torch.equal(grads[i][1], db[i, :, :r].to(torch.bfloat16))
         assert torch.equal(a_all[i].float(), ra.to(torch.bfloat16).float())
         assert torch.equal(b_all[i].float(), rb.to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("M", [1, 100, 640])
+@pytest.mark.parametrize("p", [0.0, 0.1])
+def test_one_call_layer_equals_its_building_blocks(M, p):
+    """``linear_fwd`` / ``linear_bwd`` against the separate launches, and a single adapter without tables
+    against the same batch with them: the same bits, bias and precomputed S' included; no dX wanted."""
+    from lorafusion_b200.ops import lora_kernels as lk
+    from lorafusion_b200.ops.batch_info import single_adapter_batch_info
+
+    K, N, R = 264, 520, 64
+    x, dy, w, bias = _rand(M, K, seed=1), _rand(M, N, seed=2), _rand(N, K, scale=0.05, seed=3), _rand(N, seed=4)
+    a, b = _rand(1, R, K, scale=0.05, seed=5), _rand(1, N, R, scale=0.05, seed=6)
+    one = lk.OneAdapter(M, 2.0, p, 11)
+    table = single_adapter_batch_info(M, 16, 2.0, p, device="cuda", seed=11)
+    drop = one.dropout_spec(5)
+    assert drop == table.dropout_spec(5) or p == 0
+    s = lk.lora_down(x, a, tile_adapter=None, adapter_scale=None, scale=2.0, dropout=drop)
+    y = lk.base_lora_fwd(x, w, s, b, tile_adapter=None, bias=bias)
+    ds = lk.lora_ds(dy, b, tile_adapter=None, adapter_scale=None, scale=2.0)
+    dx = lk.base_lora_dx(dy, w, ds, a, tile_adapter=None, dropout=drop)
+    da, db = torch.zeros(1, R, K, device="cuda"), torch.zeros(1, N, R, device="cuda")
+    segs = lk.SegmentTable([(0, 0, M)], torch.device("cuda"), total_rows=M)
+    lk.lora_db(dy, s, segs, db)
+    lk.lora_da(x, ds, segs, da, dropout=drop)
+    for info in (one, table):
+        got_y, got_s = lk.linear_fwd(x, w, a, b, info, drop, bias=bias)
+        assert torch.equal(got_y, y) and torch.equal(got_s, s)
+        assert torch.equal(lk.linear_fwd(x, w, a, b, info, drop, bias=bias, s=s)[0], y)
+        got_da, got_db = torch.zeros_like(da), torch.zeros_like(db)
+        assert torch.equal(lk.linear_bwd(dy, x, s, w, a, b, info, drop, got_da, got_db, True), dx)
+        assert torch.equal(got_da, da) and torch.equal(got_db, db)
+        assert lk.linear_bwd(dy, x, s, None, a, b, info, drop, None, None, False) is None
