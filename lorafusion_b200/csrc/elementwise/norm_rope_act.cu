@@ -259,29 +259,50 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
   }
 }
 
-// dgu[M, 2I] from dout[M, I] and the saved gu.
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dout,
-                                  const __nv_bfloat16* __restrict__ gu,
-                                  __nv_bfloat16* __restrict__ dgu, long long M, int I) {
+// dgu[M, 2I] from dout[M, I] and the saved gu.  One CTA per piece of a row, the pieces of a row side by
+// side: one small division a CTA and all loads of two vectors in flight a thread, 421 -> 330 us for
+// 16384 x 14336 (a flat index over all vectors takes two 64-bit divisions each).  The forward kernel,
+// which has a third fewer loads to wait for, is the faster one with the flat index: 243 against 286.
+constexpr int SWIGLU_THREADS = 256;
+constexpr int SWIGLU_VECS = 2;
+
+__global__ void __launch_bounds__(SWIGLU_THREADS)
+swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ gu,
+                  __nv_bfloat16* __restrict__ dgu, int I, int pieces) {
   const int vec = I / 8;
-  const long long total = M * vec;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long row = idx / vec;
-    const int c = int(idx % vec) * 8;
-    float g[8], u[8], d[8], dg[8], du[8];
-    load8(gu + row * 2 * I + c, g);
-    load8(gu + row * 2 * I + I + c, u);
-    load8(dout + row * I + c, d);
+  const long long m = blockIdx.x / pieces;
+  const __nv_bfloat16* row = gu + m * 2 * I;
+  const __nv_bfloat16* drow = dout + m * I;
+  __nv_bfloat16* orow = dgu + m * 2 * I;
+  const int c0 = blockIdx.x % pieces * (SWIGLU_THREADS * SWIGLU_VECS) + threadIdx.x;
+  uint4 gv[SWIGLU_VECS], uv[SWIGLU_VECS], dv[SWIGLU_VECS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float sig = 1.f / (1.f + __expf(-g[j]));
-      const float silu = g[j] * sig;
-      du[j] = d[j] * silu;
-      dg[j] = d[j] * u[j] * (sig + silu * (1.f - sig));
+  for (int k = 0; k < SWIGLU_VECS; ++k) {
+    const int c = c0 + k * SWIGLU_THREADS;
+    if (c < vec) {
+      gv[k] = *reinterpret_cast<const uint4*>(row + c * 8);
+      uv[k] = *reinterpret_cast<const uint4*>(row + I + c * 8);
+      dv[k] = *reinterpret_cast<const uint4*>(drow + c * 8);
     }
-    store8(dgu + row * 2 * I + c, dg);
-    store8(dgu + row * 2 * I + I + c, du);
+  }
+#pragma unroll
+  for (int k = 0; k < SWIGLU_VECS; ++k) {
+    const int c = c0 + k * SWIGLU_THREADS;
+    if (c < vec) {
+      float g[8], u[8], d[8], dg[8], du[8];
+      unpack8(gv[k], g);
+      unpack8(uv[k], u);
+      unpack8(dv[k], d);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float sig = 1.f / (1.f + __expf(-g[j]));
+        const float silu = g[j] * sig;
+        du[j] = d[j] * silu;
+        dg[j] = d[j] * u[j] * (sig + silu * (1.f - sig));
+      }
+      store8(orow + c * 8, dg);
+      store8(orow + I + c * 8, du);
+    }
   }
 }
 
@@ -321,6 +342,11 @@ static inline int grid_for(long long total, int threads) {
   long long b = (total + threads - 1) / threads;
   const long long cap = 148LL * 16;
   return int(b < 1 ? 1 : (b > cap ? cap : b));
+}
+
+static inline int swiglu_pieces(int I) {
+  const int per = SWIGLU_THREADS * SWIGLU_VECS;
+  return (I / 8 + per - 1) / per;
 }
 
 }  // namespace lf
@@ -380,7 +406,7 @@ int lf_rope_inplace(void* qkv, const int* pos, const float* cos_t, const float* 
 
 int lf_swiglu_fwd(const void* gu, void* out, long long M, int I, void* stream) {
   if (I % 8 != 0) return -1;
-  if (M == 0) return 0;
+  if (M == 0 || I == 0) return 0;
   swiglu_fwd_kernel<<<grid_for(M * (I / 8), 256), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, M, I);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -388,9 +414,9 @@ int lf_swiglu_fwd(const void* gu, void* out, long long M, int I, void* stream) {
 
 int lf_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long M, int I, void* stream) {
   if (I % 8 != 0) return -1;
-  if (M == 0) return 0;
-  swiglu_bwd_kernel<<<grid_for(M * (I / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)dout, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, M, I);
+  if (M == 0 || I == 0) return 0;
+  swiglu_bwd_kernel<<<(unsigned)(M * swiglu_pieces(I)), SWIGLU_THREADS, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)dout, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, I, swiglu_pieces(I));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
