@@ -16,9 +16,12 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "../common/ptx.cuh"
+
 namespace lf {
 
 constexpr int CE_THREADS = 512;
+constexpr int CE_VECS = 4;   // 16-byte vectors in flight a thread
 
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
@@ -31,7 +34,21 @@ __device__ __forceinline__ float warp_sum2(float v) {
   return v;
 }
 
-// One CTA per token.  Pass 1: online max / sum-exp.  Pass 2: write the gradient in place.
+// e^x of two packed bf16 logits relative to a maximum.
+__device__ __forceinline__ unsigned long long exp_pair(uint32_t w, unsigned long long neg_m2, unsigned long long log2e2) {
+  const float2 f = unpack_bf16x2(w);
+  float a, b;
+  unpack_f32x2(mul_f32x2(add_f32x2(f32x2(f.x, f.y), neg_m2), log2e2), a, b);
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(a));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(b));
+  return f32x2(a, b);
+}
+
+// One CTA per token.  Pass 1: online max / sum-exp.  Pass 2: write the gradient in place.  Two
+// exponentials a logit keep the special-function units busy for 117 us of 2048 rows of 128256, next
+// to 158 us of memory traffic, so the rest of the arithmetic is done two logits at a time, the label's
+// column apart, and four vectors of a thread are in flight: 265 -> 233 us (either alone gave nothing,
+// nor did keeping part of the row in shared memory instead of reading it twice).
 // labels < 0 are ignored (loss 0, gradient 0).  grad_scale multiplies the gradient
 // (1 / number of valid tokens for a mean loss).
 __global__ void __launch_bounds__(CE_THREADS)
@@ -53,26 +70,33 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
     return;
   }
 
+  const unsigned long long log2e2 = f32x2(1.4426950408889634f, 1.4426950408889634f);
   float m = -INFINITY, s = 0.f;
-  for (int c = threadIdx.x; c < nvec; c += CE_THREADS) {
-    uint4 raw = reinterpret_cast<const uint4*>(lr)[c];
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-    float f[8];
+  for (int c0 = threadIdx.x; c0 < nvec; c0 += CE_VECS * CE_THREADS) {
+    uint4 raw[CE_VECS];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float2 t = __bfloat1622float2(h[j]);
-      f[2 * j] = t.x;
-      f[2 * j + 1] = t.y;
+    for (int k = 0; k < CE_VECS; ++k)
+      if (c0 + k * CE_THREADS < nvec) raw[k] = reinterpret_cast<const uint4*>(lr)[c0 + k * CE_THREADS];
+#pragma unroll
+    for (int k = 0; k < CE_VECS; ++k) {
+      if (c0 + k * CE_THREADS >= nvec) continue;
+      const uint32_t w[4] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w};
+      // the maximum of bf16 values is one of them: taken on packed pairs
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(w);
+      const __nv_bfloat162 m2 = __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3]));
+      const float lm = fmaxf(__low2float(m2), __high2float(m2));
+      if (lm > m) {
+        s *= __expf(m - lm);
+        m = lm;
+      }
+      const unsigned long long neg_m2 = f32x2(-m, -m);
+      unsigned long long sum = 0ull;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sum = add_f32x2(sum, exp_pair(w[j], neg_m2, log2e2));
+      float s0, s1;
+      unpack_f32x2(sum, s0, s1);
+      s += s0 + s1;
     }
-    float lm = f[0];
-#pragma unroll
-    for (int j = 1; j < 8; ++j) lm = fmaxf(lm, f[j]);
-    if (lm > m) {
-      s *= __expf(m - lm);
-      m = lm;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) s += __expf(f[j] - m);
   }
   for (int c = nvec * 8 + threadIdx.x; c < V; c += CE_THREADS) {
     const float f = __bfloat162float(lr[c]);
@@ -97,29 +121,37 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
   for (int i = 0; i < CE_THREADS / 32; ++i)
     bs += (red_m[i] == -INFINITY) ? 0.f : red_s[i] * __expf(red_m[i] - bm);
   const float lse = bm + __logf(bs);
-  const float inv_sum = 1.f / bs;
+  const float inv_sum = 1.f / bs, scale = inv_sum * grad_scale;
   const float label_logit = __bfloat162float(lr[label]);
   __syncthreads();  // everyone has read lr[label] before it is overwritten
   if (threadIdx.x == 0) loss_out[row] = lse - label_logit;
 
-  for (int c = threadIdx.x; c < nvec; c += CE_THREADS) {
-    uint4 raw = reinterpret_cast<const uint4*>(lr)[c];
-    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
+  const unsigned long long neg_bm2 = f32x2(-bm, -bm), scale2 = f32x2(scale, scale);
+  for (int c0 = threadIdx.x; c0 < nvec; c0 += CE_VECS * CE_THREADS) {
+    uint4 raw[CE_VECS];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float2 t = __bfloat1622float2(h[j]);
-      const int col = c * 8 + 2 * j;
-      float g0 = __expf(t.x - bm) * inv_sum - (col == label ? 1.f : 0.f);
-      float g1 = __expf(t.y - bm) * inv_sum - (col + 1 == label ? 1.f : 0.f);
-      h[j] = __floats2bfloat162_rn(g0 * grad_scale, g1 * grad_scale);
+    for (int k = 0; k < CE_VECS; ++k)
+      if (c0 + k * CE_THREADS < nvec) raw[k] = reinterpret_cast<const uint4*>(lr)[c0 + k * CE_THREADS];
+#pragma unroll
+    for (int k = 0; k < CE_VECS; ++k) {
+      if (c0 + k * CE_THREADS >= nvec) continue;
+      uint32_t w[4] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float g0, g1;
+        unpack_f32x2(mul_f32x2(exp_pair(w[j], neg_bm2, log2e2), scale2), g0, g1);
+        w[j] = pack_bf16x2(g0, g1);
+      }
+      reinterpret_cast<uint4*>(lr)[c0 + k * CE_THREADS] = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    reinterpret_cast<uint4*>(lr)[c] = raw;
   }
   for (int c = nvec * 8 + threadIdx.x; c < V; c += CE_THREADS) {
     const float f = __bfloat162float(lr[c]);
-    const float g = __expf(f - bm) * inv_sum - (c == label ? 1.f : 0.f);
-    lr[c] = __float2bfloat16(g * grad_scale);
+    lr[c] = __float2bfloat16(__expf(f - bm) * scale);
   }
+  __syncthreads();
+  // the label's column, which the loops above treated like any other
+  if (threadIdx.x == 0) lr[label] = __float2bfloat16((__expf(label_logit - bm) * inv_sum - 1.f) * grad_scale);
 }
 
 // ---------------------------------------------------------------------------------
@@ -166,10 +198,11 @@ struct AdamWorkItem {
 };
 
 //
-// An item is shared by kAdamShares neighbouring CTAs.  With one CTA an item every thread walked 32
-// pieces, each a chain of two loads and a store, and all CTAs that ran together touched memory at
-// a stride of one item, 128 KB, which a few memory channels serve: 267 us for the 86 MB of a two-layer
-// 8B adapter.
+// Bound by latency unless every load of a thread is issued before its first use: an item is shared by
+// kAdamShares neighbouring CTAs, and a thread loads gradient, weight and moments of its two pieces
+// first (padding is not read at all).  The 86 MB of a two-layer 8B adapter take 34 us (2.5 TB/s); one
+// CTA an item, whose threads walked 32 pieces one after the other, took 267 us, and sixteen CTAs an
+// item with two pieces one after the other 152 us.
 constexpr unsigned kAdamShares = 16;
 
 __global__ void __launch_bounds__(256)
@@ -188,30 +221,44 @@ adam_chunks_kernel(const AdamChunk* __restrict__ chunks, const AdamWorkItem* __r
     float4* g4p = reinterpret_cast<float4*>(grad + c.offset);
     const unsigned ld = unsigned(c.ld), col0 = unsigned(c.col0), cols = unsigned(c.cols);
     const unsigned end4 = (item.first + item.count) >> 2;
-    for (unsigned i4 = (item.first >> 2) + first; i4 < end4; i4 += 256u * kAdamShares) {
-      const float4 g = g4p[i4];
-      g4p[i4] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (cols == 0) continue;  // padding: cleared only
-      const unsigned e = i4 << 2;
-      const unsigned row = e / ld;
-      const unsigned col = e - row * ld;
-      if (col < col0 || col >= col0 + cols) continue;
-      const long long se = c.state + (long long)row * cols + (col - col0);
-      float4 w4 = *reinterpret_cast<const float4*>(master + se);
-      float4 m4 = *reinterpret_cast<const float4*>(m + se);
-      float4 v4 = *reinterpret_cast<const float4*>(v + se);
-      adam_one(g.x * h.grad_scale, w4.x, m4.x, v4.x, h, inv_c1, inv_sqrt_c2);
-      adam_one(g.y * h.grad_scale, w4.y, m4.y, v4.y, h, inv_c1, inv_sqrt_c2);
-      adam_one(g.z * h.grad_scale, w4.z, m4.z, v4.z, h, inv_c1, inv_sqrt_c2);
-      adam_one(g.w * h.grad_scale, w4.w, m4.w, v4.w, h, inv_c1, inv_sqrt_c2);
-      *reinterpret_cast<float4*>(master + se) = w4;
-      *reinterpret_cast<float4*>(m + se) = m4;
-      *reinterpret_cast<float4*>(v + se) = v4;
-      __nv_bfloat162 lo = __floats2bfloat162_rn(w4.x, w4.y), hi = __floats2bfloat162_rn(w4.z, w4.w);
-      uint2 packed;
-      packed.x = *reinterpret_cast<uint32_t*>(&lo);
-      packed.y = *reinterpret_cast<uint32_t*>(&hi);
-      *reinterpret_cast<uint2*>(work + c.offset + e) = packed;
+    constexpr int U = 2;   // pieces in flight: 32768-element items are done in one go
+    for (unsigned i0 = (item.first >> 2) + first; i0 < end4; i0 += U * 256u * kAdamShares) {
+      float4 g[U], w4[U], m4[U], v4[U];
+      long long se[U];
+      bool live[U];
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        const unsigned i4 = i0 + k * 256u * kAdamShares;
+        live[k] = false;
+        if (i4 < end4) {
+          const unsigned e = i4 << 2;
+          const unsigned row = e / ld;
+          const unsigned col = e - row * ld;
+          live[k] = cols != 0 && col >= col0 && col < col0 + cols;   // padding is cleared only
+          se[k] = c.state + (long long)row * cols + (col - col0);
+          if (live[k]) {
+            g[k] = g4p[i4];
+            w4[k] = *reinterpret_cast<const float4*>(master + se[k]);
+            m4[k] = *reinterpret_cast<const float4*>(m + se[k]);
+            v4[k] = *reinterpret_cast<const float4*>(v + se[k]);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        const unsigned i4 = i0 + k * 256u * kAdamShares;
+        if (i4 < end4) g4p[i4] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!live[k]) continue;
+        adam_one(g[k].x * h.grad_scale, w4[k].x, m4[k].x, v4[k].x, h, inv_c1, inv_sqrt_c2);
+        adam_one(g[k].y * h.grad_scale, w4[k].y, m4[k].y, v4[k].y, h, inv_c1, inv_sqrt_c2);
+        adam_one(g[k].z * h.grad_scale, w4[k].z, m4[k].z, v4[k].z, h, inv_c1, inv_sqrt_c2);
+        adam_one(g[k].w * h.grad_scale, w4[k].w, m4[k].w, v4[k].w, h, inv_c1, inv_sqrt_c2);
+        *reinterpret_cast<float4*>(master + se[k]) = w4[k];
+        *reinterpret_cast<float4*>(m + se[k]) = m4[k];
+        *reinterpret_cast<float4*>(v + se[k]) = v4[k];
+        *reinterpret_cast<uint2*>(work + c.offset + (i4 << 2)) =
+            make_uint2(pack_bf16x2(w4[k].x, w4[k].y), pack_bf16x2(w4[k].z, w4[k].w));
+      }
     }
     return;
   }
