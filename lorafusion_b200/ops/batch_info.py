@@ -133,19 +133,18 @@ def prepare_multi_lora_batch_info(
         start += int(padded[i])
     seg_rows = segment_rows(segments)
 
-    # one staging buffer: int32 words [segment rows (4 each) | tile_adapter | lookup (3/blk) | thresh (n_ad)]
-    # followed by fp32 words [scale (n_ad) | inv_keep (n_ad) | blk_p | blk_alpha]; the segment rows
-    # come first because the kernels read them 16 bytes at a time
-    n_row = 4 * len(seg_rows)
-    n_int = n_blk + 3 * n_blk + n_ad
+    # one staging buffer: int32 words [tile_adapter | lookup (3/blk) | thresh (n_ad) | segment rows (4 each, at
+    # a multiple of four: the kernels read them 16 bytes at a time)] followed by fp32 words
+    # [scale (n_ad) | inv_keep (n_ad) | blk_p | blk_alpha]
+    seg_at = (4 * n_blk + n_ad + 3) // 4 * 4
+    n_int = seg_at + 4 * len(seg_rows)
     n_flt = 2 * n_ad + 2 * n_blk
-    staging = torch.empty(n_row + n_int + n_flt, dtype=torch.int32,
-                          pin_memory=(device.type == "cuda" and torch.cuda.is_available()))
-    stage = staging[n_row:]
-    staging.numpy()[:n_row] = np.asarray(seg_rows, dtype=np.int32).reshape(-1)
+    stage = torch.empty(n_int + n_flt, dtype=torch.int32,
+                        pin_memory=(device.type == "cuda" and torch.cuda.is_available()))
     words = stage.numpy()
     fwords = words.view(np.float32)
     words[:n_blk] = idx_arr[seg_of_block] if n_blk else 0
+    words[4 * n_blk + n_ad:n_int] = [0] * (seg_at - 4 * n_blk - n_ad) + [v for r in seg_rows for v in r]
     lookup = words[n_blk:4 * n_blk].reshape(n_blk, 3)
     lookup[:, 0] = ranks[seg_of_block]
     lookup[:, 1] = valid
@@ -160,14 +159,13 @@ def prepare_multi_lora_batch_info(
         thresh[a] = dropout_threshold(float(p_arr[i]))
         scale[a] = alpha_arr[i]
         inv_keep[a] = 1.0 / (1.0 - p_arr[i]) if p_arr[i] > 0 else 1.0
-    words[4 * n_blk:n_int] = thresh
+    words[4 * n_blk:4 * n_blk + n_ad] = thresh
     fwords[n_int:n_int + n_ad] = scale
     fwords[n_int + n_ad:n_int + 2 * n_ad] = inv_keep
     fwords[n_int + 2 * n_ad:n_int + 2 * n_ad + n_blk] = p_arr[seg_of_block] if n_blk else 0
     fwords[n_int + 2 * n_ad + n_blk:] = alpha_arr[seg_of_block] if n_blk else 0
 
-    moved = staging.to(device, non_blocking=True)
-    dev = moved[n_row:]
+    dev = stage.to(device, non_blocking=True)
     fdev = dev.view(torch.float32)
     active = [float(p_arr[i]) for i in range(n_seg) if idx_arr[i] >= 0 and padded[i] > 0]
     enable_dropout = any(p > 0 for p in active)
@@ -190,10 +188,10 @@ def prepare_multi_lora_batch_info(
         allow_empty_micro_batch_info=allow_empty_micro_batch_info,
         tile_adapter=dev[:n_blk],
         adapter_scale=fdev[n_int:n_int + n_ad],
-        adapter_thresh16=dev[4 * n_blk:n_int],
+        adapter_thresh16=dev[4 * n_blk:4 * n_blk + n_ad],
         adapter_inv_keep=fdev[n_int + n_ad:n_int + 2 * n_ad],
         segments=segments,
-        segment_table=SegmentTable(segments, device, total_rows=start, rows=moved[:n_row].view(-1, 4)),
+        segment_table=SegmentTable(segments, device, total_rows=start, staged=(dev, seg_at, n_int)),
         seed=seed,
         total_padded_tokens=start,
     )

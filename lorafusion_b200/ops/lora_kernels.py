@@ -108,18 +108,19 @@ def reduction_split(tiles: int, k_blocks: int) -> int:
 @dataclass
 class SegmentTable:
     """Token segments of one packed microbatch: ``(adapter, start, end)`` with ``start`` and
-    ``end`` multiples of 128 and at most one segment per adapter.  ``rows`` (optional): the
-    :func:`segment_rows` of the segments, already on the device."""
+    ``end`` multiples of 128 and at most one segment per adapter.  ``staged`` (optional):
+    ``(int32 device tensor, first, end)`` where the :func:`segment_rows` of the segments already lie."""
 
     segments: Sequence[tuple[int, int, int]]
     device: torch.device
     total_rows: Optional[int] = None
-    rows: Optional[torch.Tensor] = None
+    staged: Optional[tuple] = None
     _cache: dict = field(default_factory=dict)
 
     def device_rows(self) -> torch.Tensor:
         """int32 ``[n, 4]`` work list ``(adapter, start, end, 0)`` of the gradient kernels."""
-        if "checked" not in self._cache:
+        t = self._cache.get("rows")
+        if t is None:
             seen = set()
             for adapter, start, end in self.segments:
                 if adapter < 0 or end <= start:
@@ -130,10 +131,13 @@ class SegmentTable:
                 last = self.total_rows is not None and end >= self.total_rows
                 if start % TILE_M or (end % TILE_M and not last):
                     raise ValueError("segment bounds must be multiples of 128 tokens")
-            self._cache["checked"] = True
-        if self.rows is None:
-            self.rows = torch.tensor(segment_rows(self.segments), dtype=torch.int32).reshape(-1, 4).to(self.device)
-        return self.rows
+            if self.staged is not None:
+                src, first, end = self.staged
+                t = src[first:end].view(-1, 4)
+            else:
+                t = torch.tensor(segment_rows(self.segments), dtype=torch.int32).reshape(-1, 4).to(self.device)
+            self._cache["rows"] = t
+        return t
 
     def split_plan(self, features: int):
         """``(chunks per segment, owner)`` when the tokens of every segment are summed in several
