@@ -191,10 +191,10 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 // by position id.  `sign` = +1 forward, -1 backward (the transpose of a rotation).
 // ---------------------------------------------------------------------------------
 // One CTA per token; threadIdx.x = 16-byte vector of a half head, threadIdx.y = head.  A thread keeps
-// its piece of the cos / sin row for all the heads it rotates, and has the loads of two heads in
-// flight.  (A flat index over all vectors spent its time in two 64-bit divisions and a cos / sin
-// load per vector: 92 us for 16384 tokens of 40 heads, 3.6 TB/s.)
-constexpr int ROPE_THREADS = 128;
+// its piece of the cos / sin row for all the heads it rotates (two at a time), and the first heads are on
+// their way before the position that selects the row is known.  (A flat index over all vectors spent
+// its time in two 64-bit divisions and a cos / sin load per vector: 92 us for 16384 tokens of 40 heads.)
+constexpr int ROPE_THREADS = 256;
 
 __global__ void __launch_bounds__(ROPE_THREADS)
 rope_inplace_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ pos, const float* __restrict__ cos_t,
@@ -202,8 +202,20 @@ rope_inplace_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ pos
   const int half = D / 2;
   const long long row = blockIdx.x;
   const int by = blockDim.y;
-  for (int vi = threadIdx.x; vi < half / 8; vi += blockDim.x) {   // (once, up to head size 2048)
+  for (int vi = threadIdx.x; vi < half / 8; vi += blockDim.x) {   // (once, up to head size 4096)
     __nv_bfloat16* base = qkv + row * row_stride + vi * 8;
+    uint4 lo[2], hi[2];
+    auto load = [&](int h0) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int head = h0 + k * by;
+        if (head < n_rot_heads) {
+          lo[k] = *reinterpret_cast<const uint4*>(base + head * D);
+          hi[k] = *reinterpret_cast<const uint4*>(base + head * D + half);
+        }
+      }
+    };
+    load(threadIdx.y);
     const long long table = (long long)pos[row] * half + vi * 8;
     float c[8], s[8];
 #pragma unroll
@@ -212,29 +224,23 @@ rope_inplace_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ pos
       s[j] = sign * sin_t[table + j];
     }
     for (int h0 = threadIdx.y; h0 < n_rot_heads; h0 += 2 * by) {
-      float lo[2][8], hi[2][8];
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const int head = h0 + k * by;
         if (head < n_rot_heads) {
-          load8(base + head * D, lo[k]);
-          load8(base + head * D + half, hi[k]);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int head = h0 + k * by;
-        if (head < n_rot_heads) {
-          float olo[8], ohi[8];
+          float l[8], h[8], olo[8], ohi[8];
+          unpack8(lo[k], l);
+          unpack8(hi[k], h);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            olo[j] = lo[k][j] * c[j] - hi[k][j] * s[j];
-            ohi[j] = hi[k][j] * c[j] + lo[k][j] * s[j];
+            olo[j] = l[j] * c[j] - h[j] * s[j];
+            ohi[j] = h[j] * c[j] + l[j] * s[j];
           }
           store8(base + head * D, olo);
           store8(base + head * D + half, ohi);
         }
       }
+      load(h0 + 2 * by);
     }
   }
 }
