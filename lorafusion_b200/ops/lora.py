@@ -201,6 +201,7 @@ class _FusedLoRAFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x2d, w, bias, info, stream_id, training, *ab):
+        lk.check2d(x2d, "x")
         n = len(ab) // 2
         K, N = x2d.shape[1], w.shape[0]
         entries = [_adapter_entry(a, b, K, N, x2d.device) for a, b in zip(ab[:n], ab[n:])]
@@ -210,7 +211,8 @@ class _FusedLoRAFunction(torch.autograd.Function):
                                    training=training)
         ctx.save_for_backward(x2d, s, stack.a, stack.b)
         ctx.w, ctx.info, ctx.stream_id, ctx.training = w, info, stream_id, training
-        ctx.meta = [None if t is None else (t.dtype, e[2]) for t, e in zip(ab, entries * 2)]
+        # (a B without its A takes no part and gets no gradient)
+        ctx.meta = [None if e[0] is None else (t.dtype, e[2]) for t, e in zip(ab, entries * 2)]
         return y
 
     @staticmethod
@@ -229,7 +231,7 @@ class _FusedLoRAFunction(torch.autograd.Function):
                                   need_dx=ctx.needs_input_grad[0], training=ctx.training)
         grads = [None] * (2 * n)
         for i, want in enumerate(need):
-            if want:
+            if want and ctx.meta[i] is not None:
                 r = ctx.meta[i][1]
                 grads[i] = torch.empty((r, K) if i < n else (N, r), dtype=torch.bfloat16, device=dy.device)
         if na + nb:

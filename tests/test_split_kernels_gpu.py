@@ -221,3 +221,24 @@ def test_one_call_layer_equals_its_building_blocks(M, p):
         assert torch.equal(lk.linear_bwd(dy, x, s, w, a, b, info, drop, got_da, got_db, True), dx)
         assert torch.equal(got_da, da) and torch.equal(got_db, db)
         assert lk.linear_bwd(dy, x, s, None, a, b, info, drop, None, None, False) is None
+
+
+def test_fused_multi_lora_gradients_of_a_partly_missing_adapter():
+    """``A`` missing while ``B`` is given: that adapter contributes nothing and its ``B`` gets no gradient; the
+    other one's gradients are those of a layer that holds it alone.  Wrong shapes and types are refused."""
+    from lorafusion_b200.ops import fused_linear_lora, fused_linear_multi_lora
+
+    x, w = _rand(256, 128, seed=1).requires_grad_(True), _rand(264, 128, scale=0.05, seed=2)
+    a, b, b2 = (_rand(*s, scale=0.1, seed=i).requires_grad_(True) for i, s in enumerate([(8, 128), (264, 8), (264, 4)], 3))
+    y = fused_linear_multi_lora(x, w, lora_a_list=[a, None], lora_b_list=[b, b2], seq_len_list=[256], lora_idx_list=[0],
+                                alpha_list=[2.0])
+    dy = _rand(256, 264, seed=9)
+    dx, da, db, none = torch.autograd.grad(y, [x, a, b, b2], dy, allow_unused=True)
+    alone = fused_linear_lora(x, w, a, b, 2.0)
+    assert none is None and torch.equal(y, alone)
+    for got, want in zip((dx, da, db), torch.autograd.grad(alone, [x, a, b], dy)):
+        assert torch.equal(got, want)
+    with pytest.raises(ValueError):
+        fused_linear_lora(x.float(), w, a, b, 2.0)
+    with pytest.raises(ValueError):
+        fused_linear_lora(x, w, a[:, :64], b, 2.0)
