@@ -195,14 +195,14 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
         for (int j = 0; j < n_kv; ++j) {
           const int J = hi * n_kv + j;
           const int s = J % 3;
-          if (!mbar_wait(&k_empty[s], ((J / 3) & 1) ^ 1, ctx, ERR_WAIT_EMPTY)) {
+          if (!mbar_wait<false>(&k_empty[s], ((J / 3) & 1) ^ 1, ctx, ERR_WAIT_EMPTY)) {
             ok = false;
             break;
           }
           mbar_expect_tx(&k_full[s], ATT_TILE_BYTES);
           att_load_tile(sK3 + s * ATT_TILE_BYTES, &tmQKV, &k_full[s], p.k_col0 + g * ATT_D, seq_row0 + j * ATT_TILE);
           if (j == 0) {
-            if (hi > 0 && !mbar_wait(q_empty, (hi - 1) & 1, ctx, ERR_WAIT_EMPTY)) {
+            if (hi > 0 && !mbar_wait<false>(q_empty, (hi - 1) & 1, ctx, ERR_WAIT_EMPTY)) {
               ok = false;
               break;
             }
@@ -210,7 +210,7 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
             att_load_tile(sQ, &tmQKV, q_full, p.q_col0 + (h0 + hi) * ATT_D, row0);
             att_load_tile(sDO, &tmDO, q_full, (h0 + hi) * ATT_D, row0);
           }
-          if (!mbar_wait(v_empty, (J & 1) ^ 1, ctx, ERR_WAIT_EMPTY)) {
+          if (!mbar_wait<false>(v_empty, (J & 1) ^ 1, ctx, ERR_WAIT_EMPTY)) {
             ok = false;
             break;
           }
@@ -227,9 +227,9 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
         const int hi1 = J1 / n_kv, j1 = J1 - hi1 * n_kv;
         const int b1 = J1 & 1;
         const uint32_t ph = (J1 >> 1) & 1;
-        if ((j1 == 0 && !mbar_wait(q_full, hi1 & 1, ctx, ERR_WAIT_FULL)) ||
-            !mbar_wait(&k_full[J1 % 3], (J1 / 3) & 1, ctx, ERR_WAIT_FULL) ||
-            !mbar_wait(&s_empty[b1], ph ^ 1, ctx, ERR_WAIT_TMEM_EMPTY))
+        if ((j1 == 0 && !mbar_wait<false>(q_full, hi1 & 1, ctx, ERR_WAIT_FULL)) ||
+            !mbar_wait<false>(&k_full[J1 % 3], (J1 / 3) & 1, ctx, ERR_WAIT_FULL) ||
+            !mbar_wait<false>(&s_empty[b1], ph ^ 1, ctx, ERR_WAIT_TMEM_EMPTY))
           return false;
         tc_fence_after_sync();
         att_mma_kk(tS[b1], smem_u32(sQ), smem_u32(sK3 + (J1 % 3) * ATT_TILE_BYTES), false);
@@ -238,8 +238,8 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
       };
       auto issue_dp = [&](int J1) -> bool {  // dP of tile J1 (dO of its head was awaited by issue_s(J1))
         const int hi1 = J1 / n_kv, j1 = J1 - hi1 * n_kv;
-        if (!mbar_wait(v_full, J1 & 1, ctx, ERR_WAIT_FULL) ||
-            !mbar_wait(dp_empty, (J1 & 1) ^ 1, ctx, ERR_WAIT_TMEM_EMPTY))
+        if (!mbar_wait<false>(v_full, J1 & 1, ctx, ERR_WAIT_FULL) ||
+            !mbar_wait<false>(dp_empty, (J1 & 1) ^ 1, ctx, ERR_WAIT_TMEM_EMPTY))
           return false;
         tc_fence_after_sync();
         att_mma_kk(tDP, smem_u32(sDO), smem_u32(sV), false);
@@ -257,8 +257,8 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
           ok = false;
           break;
         }
-        if (!mbar_wait(ds_full, J & 1, ctx, ERR_WAIT_READY) ||
-            (j == 0 && hi > 0 && !mbar_wait(dq_empty, (hi - 1) & 1, ctx, ERR_WAIT_TMEM_EMPTY))) {
+        if (!mbar_wait<false>(ds_full, J & 1, ctx, ERR_WAIT_READY) ||
+            (j == 0 && hi > 0 && !mbar_wait<false>(dq_empty, (hi - 1) & 1, ctx, ERR_WAIT_TMEM_EMPTY))) {
           ok = false;
           break;
         }
@@ -283,7 +283,7 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
       for (int j = 0; j < n_kv; ++j) {
         const int J = hi * n_kv + j;
         const int sb = J & 1;
-        if (!__all_sync(0xffffffffu, mbar_wait(&s_full[sb], (J >> 1) & 1, ctx, ERR_WAIT_TMEM_FULL))) {
+        if (!__all_sync(0xffffffffu, mbar_wait<false>(&s_full[sb], (J >> 1) & 1, ctx, ERR_WAIT_TMEM_FULL))) {
           ok = false;
           break;
         }
@@ -301,7 +301,7 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
           for (int i = 0; i < 64; ++i)
             if (!row_valid || (diag && c0 + i > r)) pv[i] = 0.f;
         }
-        if (!__all_sync(0xffffffffu, mbar_wait(dp_full, J & 1, ctx, ERR_WAIT_TMEM_FULL))) {
+        if (!__all_sync(0xffffffffu, mbar_wait<false>(dp_full, J & 1, ctx, ERR_WAIT_TMEM_FULL))) {
           ok = false;
           break;
         }
@@ -316,7 +316,7 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
         if (lane == 0) mbar_arrive(dp_empty);
         // sDS is still being read by the previous tile's dQ product (for j == 0 the previous
         // head's final store has already waited for it)
-        if (j > 0 && !__all_sync(0xffffffffu, mbar_wait(dq_done, (J - 1) & 1, ctx, ERR_WAIT_MISC))) {
+        if (j > 0 && !__all_sync(0xffffffffu, mbar_wait<false>(dq_done, (J - 1) & 1, ctx, ERR_WAIT_MISC))) {
           ok = false;
           break;
         }
@@ -330,7 +330,7 @@ attn_dq_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQKV,
         if (lane == 0) mbar_arrive(ds_full);
       }
       if (!ok) break;
-      ok = __all_sync(0xffffffffu, mbar_wait(dq_done, (hi * n_kv + n_kv - 1) & 1, ctx, ERR_WAIT_MISC));
+      ok = __all_sync(0xffffffffu, mbar_wait<false>(dq_done, (hi * n_kv + n_kv - 1) & 1, ctx, ERR_WAIT_MISC));
       if (!ok) break;
       tc_fence_after_sync();
       __nv_bfloat16* orow = p.dqkv + grow * p.ld_qkv + p.q_col0 + h * ATT_D + c0;
@@ -447,7 +447,7 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
         const int s = it & 1;
         const int h = g * group + it / per_head;
         const int qrow0 = seq_row0 + (i_kv + it % per_head) * ATT_TILE;
-        if (!mbar_wait(&qd_empty[s], ((it >> 1) & 1) ^ 1, ctx, ERR_WAIT_EMPTY)) break;
+        if (!mbar_wait<false>(&qd_empty[s], ((it >> 1) & 1) ^ 1, ctx, ERR_WAIT_EMPTY)) break;
         mbar_expect_tx(&qd_full[s], 2 * ATT_TILE_BYTES);
         uint8_t* sQ = sQD + s * 2 * ATT_TILE_BYTES;
         att_load_tile(sQ, &tmQKV, &qd_full[s], p.q_col0 + h * ATT_D, qrow0);
@@ -459,8 +459,8 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
       // Issue order per iteration: [P ready] dV(it), S(it + 1), dP(it + 1), [dS ready] dK(it).
       auto issue_s = [&](int i1) -> bool {   // S = Q K^T of iteration i1 (its Q / dO stage must have landed)
         const int s1 = i1 & 1;
-        if (!mbar_wait(&qd_full[s1], (i1 >> 1) & 1, ctx, ERR_WAIT_FULL) ||
-            !mbar_wait(s_empty, (i1 & 1) ^ 1, ctx, ERR_WAIT_TMEM_EMPTY))
+        if (!mbar_wait<false>(&qd_full[s1], (i1 >> 1) & 1, ctx, ERR_WAIT_FULL) ||
+            !mbar_wait<false>(s_empty, (i1 & 1) ^ 1, ctx, ERR_WAIT_TMEM_EMPTY))
           return false;
         tc_fence_after_sync();
         att_mma_kk(tS, smem_u32(sQD + s1 * 2 * ATT_TILE_BYTES), smem_u32(sK), false);
@@ -468,19 +468,19 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
         return true;
       };
       auto issue_dp = [&](int i1) -> bool {  // dP = dO V^T of iteration i1 (stage awaited by issue_s(i1))
-        if (!mbar_wait(dp_empty, (i1 & 1) ^ 1, ctx, ERR_WAIT_TMEM_EMPTY)) return false;
+        if (!mbar_wait<false>(dp_empty, (i1 & 1) ^ 1, ctx, ERR_WAIT_TMEM_EMPTY)) return false;
         tc_fence_after_sync();
         att_mma_kk(tDP, smem_u32(sQD + (i1 & 1) * 2 * ATT_TILE_BYTES + ATT_TILE_BYTES), smem_u32(sV), false);
         tc_commit(dp_full);
         return true;
       };
-      bool ok = mbar_wait(kv_full, 0, ctx, ERR_WAIT_FULL);
+      bool ok = mbar_wait<false>(kv_full, 0, ctx, ERR_WAIT_FULL);
       ok = ok && n_it > 0 && issue_s(0) && issue_dp(0);
       for (int it = 0; ok && it < n_it; ++it) {
         const int s = it & 1;
         const uint32_t sQ = smem_u32(sQD + s * 2 * ATT_TILE_BYTES);
         const uint32_t sDO = sQ + ATT_TILE_BYTES;
-        if (!mbar_wait(p_full, it & 1, ctx, ERR_WAIT_READY)) {
+        if (!mbar_wait<false>(p_full, it & 1, ctx, ERR_WAIT_READY)) {
           ok = false;
           break;
         }
@@ -491,7 +491,7 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
           ok = false;
           break;
         }
-        if (!mbar_wait(ds_full, it & 1, ctx, ERR_WAIT_READY)) {
+        if (!mbar_wait<false>(ds_full, it & 1, ctx, ERR_WAIT_READY)) {
           ok = false;
           break;
         }
@@ -528,7 +528,7 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
       const bool need_mask = diag || q_valid < ATT_TILE;   // uniform over the CTA
       const float lse2 = lse2_next, dlts = dlts_next;       // dlts = delta * softmax scale
       if (it + 1 < n_it) row_stats(it + 1, lse2_next, dlts_next);
-      if (!__all_sync(0xffffffffu, mbar_wait(s_full, it & 1, ctx, ERR_WAIT_TMEM_FULL))) {
+      if (!__all_sync(0xffffffffu, mbar_wait<false>(s_full, it & 1, ctx, ERR_WAIT_TMEM_FULL))) {
         ok = false;
         break;
       }
@@ -546,7 +546,7 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
           if (!row_valid || (diag && c0 + i > r)) pv[i] = 0.f;
       }
       // sPD still holds dS of the previous iteration until its dK product has read it
-      if (it > 0 && !__all_sync(0xffffffffu, mbar_wait(dk_done, (it - 1) & 1, ctx, ERR_WAIT_MISC))) {
+      if (it > 0 && !__all_sync(0xffffffffu, mbar_wait<false>(dk_done, (it - 1) & 1, ctx, ERR_WAIT_MISC))) {
         ok = false;
         break;
       }
@@ -559,7 +559,7 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
       // dS of this thread's 64 columns in registers while the dV product still reads P from sPD
-      if (!__all_sync(0xffffffffu, mbar_wait(dp_full, it & 1, ctx, ERR_WAIT_TMEM_FULL))) {
+      if (!__all_sync(0xffffffffu, mbar_wait<false>(dp_full, it & 1, ctx, ERR_WAIT_TMEM_FULL))) {
         ok = false;
         break;
       }
@@ -573,7 +573,7 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(dp_empty);
-      if (!__all_sync(0xffffffffu, mbar_wait(dv_done, it & 1, ctx, ERR_WAIT_MISC))) {
+      if (!__all_sync(0xffffffffu, mbar_wait<false>(dv_done, it & 1, ctx, ERR_WAIT_MISC))) {
         ok = false;
         break;
       }
@@ -586,7 +586,7 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_full);
     }
-    if (ok && n_it > 0 && __all_sync(0xffffffffu, mbar_wait(dk_done, (n_it - 1) & 1, ctx, ERR_WAIT_MISC))) {
+    if (ok && n_it > 0 && __all_sync(0xffffffffu, mbar_wait<false>(dk_done, (n_it - 1) & 1, ctx, ERR_WAIT_MISC))) {
       tc_fence_after_sync();
       const long long grow = (long long)row0 + r;  // key row owned by this thread
       __nv_bfloat16* krow = p.dqkv + grow * p.ld_qkv + p.k_col0 + g * ATT_D;

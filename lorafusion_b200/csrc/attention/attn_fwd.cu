@@ -110,7 +110,7 @@ attn_fwd_kernel(const AttnFwdParams p, const __grid_constant__ CUtensorMap tm) {
         for (int j = 0; j < n_kv; ++j) {
           const int J = pr * n_kv + j;
           const int s = J & 1;
-          if (!mbar_wait(&k_empty[s], ((J >> 1) & 1) ^ 1, ctx, ERR_WAIT_EMPTY)) {
+          if (!mbar_wait<false>(&k_empty[s], ((J >> 1) & 1) ^ 1, ctx, ERR_WAIT_EMPTY)) {
             ok = false;
             break;
           }
@@ -120,7 +120,7 @@ attn_fwd_kernel(const AttnFwdParams p, const __grid_constant__ CUtensorMap tm) {
           if (j == 0) {
             for (int i = 0; i < active; ++i) {
               // a head's Q buffer is free once the previous pair's last S product has read it
-              if (pr > 0 && !mbar_wait(&q_empty[i], (pr - 1) & 1, ctx, ERR_WAIT_EMPTY)) {
+              if (pr > 0 && !mbar_wait<false>(&q_empty[i], (pr - 1) & 1, ctx, ERR_WAIT_EMPTY)) {
                 ok = false;
                 break;
               }
@@ -129,7 +129,7 @@ attn_fwd_kernel(const AttnFwdParams p, const __grid_constant__ CUtensorMap tm) {
             }
             if (!ok) break;
           }
-          if (!mbar_wait(&v_empty[s], ((J >> 1) & 1) ^ 1, ctx, ERR_WAIT_EMPTY)) {
+          if (!mbar_wait<false>(&v_empty[s], ((J >> 1) & 1) ^ 1, ctx, ERR_WAIT_EMPTY)) {
             ok = false;
             break;
           }
@@ -142,8 +142,8 @@ attn_fwd_kernel(const AttnFwdParams p, const __grid_constant__ CUtensorMap tm) {
     if (lane == 0) {
       auto issue_s = [&](int i, int J) -> bool {   // S of head i for element J of the sequence
         const int pr = J / n_kv, j = J - pr * n_kv;
-        if ((j == 0 && !mbar_wait(&q_full[i], pr & 1, ctx, ERR_WAIT_FULL)) ||
-            !mbar_wait(&k_full[J & 1], (J >> 1) & 1, ctx, ERR_WAIT_FULL))
+        if ((j == 0 && !mbar_wait<false>(&q_full[i], pr & 1, ctx, ERR_WAIT_FULL)) ||
+            !mbar_wait<false>(&k_full[J & 1], (J >> 1) & 1, ctx, ERR_WAIT_FULL))
           return false;
         tc_fence_after_sync();
         att_mma_kk(tmem_base + 128 * i, smem_u32(sQ + i * ATT_TILE_BYTES), smem_u32(sKV + (J & 1) * 2 * ATT_TILE_BYTES),
@@ -162,14 +162,14 @@ attn_fwd_kernel(const AttnFwdParams p, const __grid_constant__ CUtensorMap tm) {
         const uint32_t sV = smem_u32(sKV + (J & 1) * 2 * ATT_TILE_BYTES + ATT_TILE_BYTES);
         for (int i = 0; i < active; ++i) {
           const uint32_t tP = tmem_base + 128 * i, tO = tmem_base + 256 + 128 * i;
-          if (!mbar_wait(&p_full[2 * i], J & 1, ctx, ERR_WAIT_READY) ||
-              !mbar_wait(&v_full[J & 1], (J >> 1) & 1, ctx, ERR_WAIT_FULL)) {
+          if (!mbar_wait<false>(&p_full[2 * i], J & 1, ctx, ERR_WAIT_READY) ||
+              !mbar_wait<false>(&v_full[J & 1], (J >> 1) & 1, ctx, ERR_WAIT_FULL)) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
           att_mma_ts_half(tO, tP, sV, 0, j > 0);
-          if (!mbar_wait(&p_full[2 * i + 1], J & 1, ctx, ERR_WAIT_READY)) {
+          if (!mbar_wait<false>(&p_full[2 * i + 1], J & 1, ctx, ERR_WAIT_READY)) {
             ok = false;
             break;
           }
@@ -200,7 +200,7 @@ attn_fwd_kernel(const AttnFwdParams p, const __grid_constant__ CUtensorMap tm) {
       float m_ref = -INFINITY, l = 0.f;
       for (int j = 0; j < n_kv; ++j) {
         const int J = pr * n_kv + j;
-        ok = __all_sync(FULL, mbar_wait(&s_full[i], J & 1, ctx, ERR_WAIT_TMEM_FULL));
+        ok = __all_sync(FULL, mbar_wait<false>(&s_full[i], J & 1, ctx, ERR_WAIT_TMEM_FULL));
         if (!ok) break;
         tc_fence_after_sync();
         float s[128];
@@ -278,7 +278,7 @@ attn_fwd_kernel(const AttnFwdParams p, const __grid_constant__ CUtensorMap tm) {
       if (!ok) break;
       // ---- this head is complete: normalise and store.  The next P V into this O waits for a P that
       // these same warps write afterwards.
-      ok = __all_sync(FULL, mbar_wait(&o_full[i], pr & 1, ctx, ERR_WAIT_MISC));
+      ok = __all_sync(FULL, mbar_wait<false>(&o_full[i], pr & 1, ctx, ERR_WAIT_MISC));
       if (!ok) break;
       tc_fence_after_sync();
       const float inv_l = 1.f / l;

@@ -90,31 +90,48 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 // How long a waiting thread may sleep in the barrier before it comes back to poll: the abort flag and the
-// time limit are looked at every 256 polls, 5 ms.
+// time limit are looked at every 256 polls, 5 ms.  Under the large products, at the power cap, ten warps
+// of every CTA wait for most of a main loop, and sleeping instead of polling at the default rate is worth
+// 1 to 5 % (a layer of 8192 x 4096 x 4096: 582 -> 555 us).  In the attention kernels the waits are short
+// and on the critical path, and the same hint cost 2 to 4 % (8192 tokens: 2109 -> 2152 us): they poll.
 constexpr uint32_t kSuspendHintNs = 20000;
 
+template <bool SLEEP = true>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendHintNs)
-      : "memory");
+  if (SLEEP) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendHintNs)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+  }
   return ok != 0;
 }
 
 // Bounded wait on an mbarrier phase.  Returns false after an abort (own timeout or
 // another role's); the caller must leave its loop and go to teardown.
+template <bool SLEEP = true>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const AbortCtx& ctx,
                                           int code) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_try_wait<SLEEP>(bar, parity)) return true;
   const unsigned long long t0 = globaltimer_ns();
   for (uint32_t it = 1;; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<SLEEP>(bar, parity)) return true;
     if ((it & 0xff) == 0) {
       if (aborted(ctx)) return false;
       if (globaltimer_ns() - t0 > ctx.local_wait_ns) {
