@@ -126,7 +126,9 @@ typedef struct LfLoraPiece {
 } LfLoraPiece;
 
 // A whole LoRA linear layer (see lora_linear.cu).  All matrices row-major, contiguous but for the
-// row pitches given; stacks [n_adapters, R, K] and [n_adapters, N, R].  tile_adapter and seg_rows may
+// row pitches given; stacks [n_adapters, R, K] and [n_adapters, N, R] (a_all, b_all with one row pitch
+// throughout).  What a call does not read may be null: x without da in the backward, s without db, w and
+// a_all without dx, a_all in the forward with have_s.  tile_adapter and seg_rows may
 // both be null: then every token belongs to adapter 0 (num_segs = 1).
 typedef struct LfLoraLinearArgs {
   const void* x;
@@ -150,11 +152,12 @@ typedef struct LfLoraLinearArgs {
   void* stream;
   void* scratch;          // of the Y (forward) or dX (backward) product, see lf_gemm_pair_scratch
   int64_t scratch_bytes;
-  int64_t x_ld, w_ld, dy_ld;
+  int64_t x_ld, w_ld, dy_ld, a_ld, b_ld, s_ld;
   int32_t M, K, N, R, n_adapters, num_segs, have_s, dropout;
   int32_t split_s, split_ds, split_db, split_da;
   int32_t pair;           // try the CTA-pair kernels first for the big product of this call
   int32_t fwd_group_m, fwd_max_ctas, dx_group_m, dx_max_ctas, dropmix_bn;
+  int32_t row_offset, col_offset;  // of the dropout mask
   float scale, inv_keep;
   uint32_t thresh16, seed_lo, seed_hi, stream_id;
 } LfLoraLinearArgs;

@@ -149,6 +149,8 @@ static void set_dropout(LfGemmArgs& g, const LfLoraLinearArgs* l) {
   g.seed_lo = l->seed_lo;
   g.seed_hi = l->seed_hi;
   g.stream_id = l->stream_id;
+  g.row_offset = l->row_offset;
+  g.col_offset = l->col_offset;
 }
 static int big_gemm(LfGemmArgs& g, const LfLoraLinearArgs* l) {
   g.scratch = l->scratch;
@@ -167,12 +169,12 @@ int lf_lora_linear_fwd(const LfLoraLinearArgs* l) {
   if (!l->have_s) {
     LfGemmArgs g = base_args(l);
     set_operand(g.a, g.a_rows, g.a_cols, g.a_ld, l->x, M, K, l->x_ld);
-    set_operand(g.b, g.b_rows, g.b_cols, g.b_ld, l->a_all, n * R, K, K);
+    set_operand(g.b, g.b_rows, g.b_cols, g.b_ld, l->a_all, n * R, K, l->a_ld);
     g.tile_adapter = l->tile_adapter;
     g.adapter_scale = l->adapter_scale;
     g.scale = l->scale;
     g.out = l->s;
-    g.ldo = R;
+    g.ldo = l->s_ld;
     g.M = int(M);
     g.N = g.bn = g.b_adapter_rows = int(R);
     g.K = int(K);
@@ -185,8 +187,8 @@ int lf_lora_linear_fwd(const LfLoraLinearArgs* l) {
   LfGemmArgs g = base_args(l);
   set_operand(g.a, g.a_rows, g.a_cols, g.a_ld, l->x, M, K, l->x_ld);
   set_operand(g.b, g.b_rows, g.b_cols, g.b_ld, l->w, N, K, l->w_ld);
-  set_operand(g.a2, g.a2_rows, g.a2_cols, g.a2_ld, l->s, M, R, R);
-  set_operand(g.b2, g.b2_rows, g.b2_cols, g.b2_ld, l->b_all, n * N, R, R);
+  set_operand(g.a2, g.a2_rows, g.a2_cols, g.a2_ld, l->s, M, R, l->s_ld);
+  set_operand(g.b2, g.b2_rows, g.b2_cols, g.b2_ld, l->b_all, n * N, R, l->b_ld);
   g.tile_adapter = l->tile_adapter;
   g.out = l->y;
   g.ldo = N;
@@ -211,7 +213,7 @@ int lf_lora_linear_bwd(const LfLoraLinearArgs* l) {
   {
     LfGemmArgs g = base_args(l);
     set_operand(g.a, g.a_rows, g.a_cols, g.a_ld, l->dy, M, N, l->dy_ld);
-    set_operand(g.b, g.b_rows, g.b_cols, g.b_ld, l->b_all, n * N, R, R);
+    set_operand(g.b, g.b_rows, g.b_cols, g.b_ld, l->b_all, n * N, R, l->b_ld);
     g.tile_adapter = l->tile_adapter;
     g.adapter_scale = l->adapter_scale;
     g.scale = l->scale;
@@ -227,7 +229,7 @@ int lf_lora_linear_bwd(const LfLoraLinearArgs* l) {
   if (l->db != nullptr && l->num_segs > 0) {
     LfGemmArgs g = base_args(l);
     set_operand(g.a, g.a_rows, g.a_cols, g.a_ld, l->dy, M, N, l->dy_ld);
-    set_operand(g.b, g.b_rows, g.b_cols, g.b_ld, l->s, M, R, R);
+    set_operand(g.b, g.b_rows, g.b_cols, g.b_ld, l->s, M, R, l->s_ld);
     g.seg_tiles = l->seg_rows;
     g.num_seg_tiles = l->num_segs;
     g.out = l->db;
@@ -264,7 +266,7 @@ int lf_lora_linear_bwd(const LfLoraLinearArgs* l) {
   set_operand(g.a, g.a_rows, g.a_cols, g.a_ld, l->dy, M, N, l->dy_ld);
   set_operand(g.b, g.b_rows, g.b_cols, g.b_ld, l->w, N, K, l->w_ld);
   set_operand(g.a2, g.a2_rows, g.a2_cols, g.a2_ld, l->ds, M, R, R);
-  set_operand(g.b2, g.b2_rows, g.b2_cols, g.b2_ld, l->a_all, n * R, K, K);
+  set_operand(g.b2, g.b2_rows, g.b2_cols, g.b2_ld, l->a_all, n * R, K, l->a_ld);
   g.tile_adapter = l->tile_adapter;
   g.out = l->dx;
   g.ldo = K;

@@ -109,10 +109,11 @@ class LfLoraLinearArgs(C.Structure):
         [(f, C.c_void_p) for f in ("x", "w", "bias", "a_all", "b_all", "s", "y", "dy", "ds", "da", "db", "dx",
                                    "tile_adapter", "seg_rows", "adapter_scale", "adapter_thresh16",
                                    "adapter_inv_keep", "err", "stream", "scratch")]
-        + [(f, C.c_int64) for f in ("scratch_bytes", "x_ld", "w_ld", "dy_ld")]
+        + [(f, C.c_int64) for f in ("scratch_bytes", "x_ld", "w_ld", "dy_ld", "a_ld", "b_ld", "s_ld")]
         + [(f, C.c_int32) for f in ("M", "K", "N", "R", "n_adapters", "num_segs", "have_s", "dropout",
                                     "split_s", "split_ds", "split_db", "split_da", "pair",
-                                    "fwd_group_m", "fwd_max_ctas", "dx_group_m", "dx_max_ctas", "dropmix_bn")]
+                                    "fwd_group_m", "fwd_max_ctas", "dx_group_m", "dx_max_ctas", "dropmix_bn",
+                                    "row_offset", "col_offset")]
         + [("scale", C.c_float), ("inv_keep", C.c_float)]
         + [(f, C.c_uint32) for f in ("thresh16", "seed_lo", "seed_hi", "stream_id")])
 

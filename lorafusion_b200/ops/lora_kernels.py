@@ -276,19 +276,39 @@ class OneAdapter:
         return DropoutSpec(seed=self.seed, stream_id=stream_id, p=self.p) if training and self.p > 0 else NO_DROPOUT
 
 
-def _linear_args(x: torch.Tensor, w: Optional[torch.Tensor], a_all: torch.Tensor, b_all: torch.Tensor, info,
-                 drop: DropoutSpec, **fields) -> nv.LfLoraLinearArgs:
-    """Describe one LoRA linear layer (``lf_lora_linear_fwd`` / ``_bwd``) for the current stream."""
-    M, K = x.shape
-    n, R, K2 = a_all.shape
-    n2, N, R2 = b_all.shape
-    if K2 != K or (n2, R2) != (n, R) or R not in RANK_PADS or (w is not None and tuple(w.shape) != (N, K)):
-        raise ValueError(f"shapes do not match: x {tuple(x.shape)}, w {None if w is None else tuple(w.shape)}, "
-                         f"A {tuple(a_all.shape)}, B {tuple(b_all.shape)}")
-    check2d(x, "x")
-    if w is not None:   # (a backward that wants no dX does not read it)
-        check2d(w, "w")
-        fields.update(w=w.data_ptr(), w_ld=w.stride(0))
+def _matrix(t: torch.Tensor, name: str, shape: tuple) -> tuple[int, int]:
+    """Address and row pitch of a bf16 matrix of the given shape."""
+    if t.shape != shape:
+        raise ValueError(f"{name} must have the shape {shape}, got {tuple(t.shape)}")
+    check2d(t, name)
+    return t.data_ptr(), t.stride(0)
+
+
+def _stack(t: torch.Tensor, name: str, shape: tuple) -> torch.Tensor:
+    """``[n, *shape]`` adapters as the bf16 matrix ``[n * shape[0], shape[1]]`` that the kernels read (a copy
+    where they do not lie one behind the other)."""
+    if t.dim() != 3 or t.shape[1:] != shape:
+        raise ValueError(f"{name} must have the shape [n, {shape[0]}, {shape[1]}], got {tuple(t.shape)}")
+    flat = _flat2d(t)
+    check2d(flat, name)
+    return flat
+
+
+def _grad_stack(t: Optional[torch.Tensor], name: str, shape: tuple) -> Optional[int]:
+    """Address of the fp32 gradient accumulators ``[n, *shape]`` of all adapters."""
+    if t is None:
+        return None
+    if t.dim() != 3 or t.shape[1:] != shape or t.dtype != torch.float32 or not t.is_contiguous():
+        raise ValueError(f"{name} must be contiguous fp32 [n, {shape[0]}, {shape[1]}], got {t.dtype} {tuple(t.shape)} "
+                         f"strides {t.stride()}")
+    return t.data_ptr()
+
+
+def _linear_args(M: int, K: int, N: int, R: int, n: int, info, drop: DropoutSpec, device, **fields) -> nv.LfLoraLinearArgs:
+    """Describe one LoRA linear layer (``lf_lora_linear_fwd`` / ``_bwd``) for the current stream.  The operands come as
+    addresses: the callers have checked them, since the kernels read and write what the sizes say."""
+    if R not in RANK_PADS and not fields.get("have_s"):
+        raise ValueError(f"adapter stacks must be {RANK_PADS} wide, got {R}")
     if "y" in fields:
         cfg = get_kernel_config("fwd", M, K, N)
         fields.update(fwd_group_m=cfg.group_m, fwd_max_ctas=cfg.max_ctas)
@@ -296,9 +316,7 @@ def _linear_args(x: torch.Tensor, w: Optional[torch.Tensor], a_all: torch.Tensor
         cfg = get_kernel_config("dx_dropout" if drop.active else "dx", M, N, K)
         fields.update(dx_group_m=cfg.group_m, dx_max_ctas=cfg.max_ctas)
     args = nv.LfLoraLinearArgs(
-        x=x.data_ptr(), a_all=a_all.data_ptr(), b_all=b_all.data_ptr(), x_ld=x.stride(0),
-        err=nv.err_word(x.device).data_ptr(), stream=nv.current_stream_ptr(),
-        M=M, K=K, N=N, R=R, n_adapters=n,
+        err=nv.err_word(device).data_ptr(), stream=nv.current_stream_ptr(), M=M, K=K, N=N, R=R, n_adapters=n,
         dropmix_bn=DROPMIX_BN, scale=getattr(info, "scale", 1.0), **fields)
     if info.tile_adapter is not None:
         args.tile_adapter = info.tile_adapter.data_ptr()
@@ -312,6 +330,7 @@ def _linear_args(x: torch.Tensor, w: Optional[torch.Tensor], a_all: torch.Tensor
             args.adapter_inv_keep = drop.adapter_inv_keep.data_ptr()
         args.seed_lo, args.seed_hi = drop.seed & 0xFFFFFFFF, (drop.seed >> 32) & 0xFFFFFFFF
         args.stream_id = drop.stream_id & 0xFFFFFFFF
+        args.row_offset, args.col_offset = drop.row_offset, drop.col_offset
     return args
 
 
@@ -326,17 +345,25 @@ def _pair_setup(args: nv.LfLoraLinearArgs, M: int, N: int, K: int, max_ctas: int
     return scratch
 
 
-def linear_fwd(x: torch.Tensor, w: torch.Tensor, a_all: torch.Tensor, b_all: torch.Tensor, info, drop: DropoutSpec,
-               bias: Optional[torch.Tensor] = None, s: Optional[torch.Tensor] = None):
-    """``lora_down`` (unless ``s`` is given) and ``base_lora_fwd`` in one call: ``(y, s)``."""
+def linear_fwd(x: torch.Tensor, w: torch.Tensor, a_all: Optional[torch.Tensor], b_all: torch.Tensor, info,
+               drop: DropoutSpec, bias: Optional[torch.Tensor] = None, s: Optional[torch.Tensor] = None):
+    """``lora_down`` (unless ``s`` is given: then ``a_all`` is not read) and ``base_lora_fwd`` in one call: ``(y, s)``."""
     M, K = x.shape
-    N, R = b_all.shape[1:]
+    n, N, R = b_all.shape
     have_s = s is not None
+    x_ptr, x_ld = _matrix(x, "x", (M, K))
+    w_ptr, w_ld = _matrix(w, "w", (N, K))
+    b2d = _stack(b_all, "B", (N, R))
+    fields = dict(x=x_ptr, x_ld=x_ld, w=w_ptr, w_ld=w_ld, b_all=b2d.data_ptr(), b_ld=b2d.stride(0))
     if not have_s:
+        a2d = _stack(a_all, "A", (R, K))
+        n = min(n, a_all.shape[0])
+        fields.update(a_all=a2d.data_ptr(), a_ld=a2d.stride(0))
         s = torch.empty((M, R), dtype=torch.bfloat16, device=x.device)
+    fields["s"], fields["s_ld"] = _matrix(s, "S'", (M, R))
     y = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
-    args = _linear_args(x, w, a_all, b_all, info, drop, s=s.data_ptr(), y=y.data_ptr(), have_s=int(have_s),
-                        bias=None if bias is None else bias.data_ptr(), split_s=_rows_split(M, K))
+    args = _linear_args(M, K, N, R, n, info, drop, x.device, y=y.data_ptr(), have_s=int(have_s),
+                        bias=None if bias is None else bias.data_ptr(), split_s=_rows_split(M, K), **fields)
     scratch = _pair_setup(args, M, N, K, args.fwd_max_ctas, x.device)
     nv.note_launch(1 if have_s else 2)
     rc = nv.cuda_lib().lf_lora_linear_fwd(C.byref(args))
@@ -346,15 +373,32 @@ def linear_fwd(x: torch.Tensor, w: torch.Tensor, a_all: torch.Tensor, b_all: tor
     return y, s
 
 
-def linear_bwd(dy: torch.Tensor, x: torch.Tensor, s: torch.Tensor, w: Optional[torch.Tensor], a_all: torch.Tensor,
-               b_all: torch.Tensor, info, drop: DropoutSpec, da: Optional[torch.Tensor], db: Optional[torch.Tensor],
-               need_dx: bool) -> Optional[torch.Tensor]:
-    """``lora_ds``, ``lora_db`` into ``db``, ``lora_da`` into ``da`` and ``base_lora_dx`` in one call."""
-    M, N = dy.shape
-    K, R = x.shape[1], s.shape[1]
-    check2d(dy, "dy")
+def linear_bwd(dy: torch.Tensor, x: Optional[torch.Tensor], s: Optional[torch.Tensor], w: Optional[torch.Tensor],
+               a_all: Optional[torch.Tensor], b_all: torch.Tensor, info, drop: DropoutSpec, da: Optional[torch.Tensor],
+               db: Optional[torch.Tensor], need_dx: bool) -> Optional[torch.Tensor]:
+    """``lora_ds``, ``lora_db`` into ``db``, ``lora_da`` into ``da`` and ``base_lora_dx`` in one call.  ``x`` is read for
+    ``da``, ``s`` for ``db``, ``w`` and ``a_all`` for dX."""
+    n, N, R = b_all.shape
+    M = dy.shape[0]
+    K = w.shape[1] if need_dx else (0 if da is None else x.shape[1])
+    dy_ptr, dy_ld = _matrix(dy, "dy", (M, N))
+    b2d = _stack(b_all, "B", (N, R))
+    fields = dict(dy=dy_ptr, dy_ld=dy_ld, b_all=b2d.data_ptr(), b_ld=b2d.stride(0),
+                  da=_grad_stack(da, "dA", (R, K)), db=_grad_stack(db, "dB", (N, R)))
+    if da is not None:
+        fields["x"], fields["x_ld"] = _matrix(x, "x", (M, K))
+        n = min(n, da.shape[0])
+    if db is not None:
+        fields["s"], fields["s_ld"] = _matrix(s, "S'", (M, R))
+        n = min(n, db.shape[0])
     ds = torch.empty((M, R), dtype=torch.bfloat16, device=dy.device)
-    dx = torch.empty((M, K), dtype=torch.bfloat16, device=dy.device) if need_dx else None
+    dx = None
+    if need_dx:
+        fields["w"], fields["w_ld"] = _matrix(w, "w", (N, K))
+        a2d = _stack(a_all, "A", (R, K))
+        n = min(n, a_all.shape[0])
+        dx = torch.empty((M, K), dtype=torch.bfloat16, device=dy.device)
+        fields.update(a_all=a2d.data_ptr(), a_ld=a2d.stride(0), dx=dx.data_ptr())
     if info.tile_adapter is None:
         seg_rows, num_segs = None, 1
         split_da, split_db = (reduction_split((f + TILE_M - 1) // TILE_M, (M + 63) // 64) for f in (K, N))
@@ -362,11 +406,8 @@ def linear_bwd(dy: torch.Tensor, x: torch.Tensor, s: torch.Tensor, w: Optional[t
         rows = info.segment_table.device_rows()
         seg_rows, num_segs = rows.data_ptr(), rows.shape[0]
         split_da, split_db = info.segment_table.chunks(K), info.segment_table.chunks(N)
-    args = _linear_args(x, w, a_all, b_all, info, drop, dy=dy.data_ptr(), dy_ld=dy.stride(0), s=s.data_ptr(),
-                        ds=ds.data_ptr(), da=None if da is None else da.data_ptr(),
-                        db=None if db is None else db.data_ptr(), dx=None if dx is None else dx.data_ptr(),
-                        seg_rows=seg_rows, num_segs=num_segs, split_ds=_rows_split(M, N), split_db=split_db,
-                        split_da=split_da)
+    args = _linear_args(M, K, N, R, n, info, drop, dy.device, ds=ds.data_ptr(), seg_rows=seg_rows, num_segs=num_segs,
+                        split_ds=_rows_split(M, N), split_db=split_db, split_da=split_da, **fields)
     scratch = _pair_setup(args, M, K, N, args.dx_max_ctas, dy.device) if need_dx else None
     nv.note_launch(1 + (da is not None) + (db is not None) + need_dx)
     rc = nv.cuda_lib().lf_lora_linear_bwd(C.byref(args))

@@ -223,6 +223,44 @@ def test_one_call_layer_equals_its_building_blocks(M, p):
         assert lk.linear_bwd(dy, x, s, None, a, b, info, drop, None, None, False) is None
 
 
+@pytest.mark.parametrize("K,N", [(264, 520), (5000, 256), (256, 5000)])
+@pytest.mark.parametrize("ps", [(0.0, 0.0, 0.0), (0.1, 0.1, 0.1), (0.1, 0.0, 0.5)])
+def test_one_call_layer_of_several_adapters_equals_its_building_blocks(K, N, ps):
+    """Three adapters and a tile without one, stacks cut out of longer and wider ones, a pitched ``S'``, a mask of a
+    shard (row and column offset); with 5000 features the last wave of the forward's or of dX's big product is cut:
+    the same bits as the separate launches."""
+    from dataclasses import replace
+
+    from lorafusion_b200.ops import lora_kernels as lk
+    from lorafusion_b200.ops.batch_info import prepare_multi_lora_batch_info
+    from lorafusion_b200.ops.gemm import _pair_scratch_bytes
+
+    R, n, M = 64, 3, 640
+    info = prepare_multi_lora_batch_info([100, 128, 128, 200], [1, -1, 0, 2], [16, 0, 16, 16],
+                                         [ps[1], 0.0, ps[0], ps[2]], [2.0, 0.0, 0.5, 1.0], device="cuda", seed=(3 << 32) | 5)
+    assert info.total_padded_tokens == M
+    assert (_pair_scratch_bytes(M, N, K, 0, 0) > 0) == (K == 5000) and (_pair_scratch_bytes(M, K, N, 0, 0) > 0) == (N == 5000)
+    drop = replace(info.dropout_spec(5), row_offset=256, col_offset=512)
+    x, dy, w = _rand(M, K, seed=1), _rand(M, N, seed=2), _rand(N, K, scale=0.05, seed=3)
+    a, b = _rand(n, 2 * R, K, scale=0.05, seed=5)[:, R:], _rand(n, N, R + 64, scale=0.05, seed=6)[:, :, 64:]
+    ta, sc, segs = info.tile_adapter, info.adapter_scale, info.segment_table
+    s = lk.lora_down(x, a, tile_adapter=ta, adapter_scale=sc, dropout=drop)
+    y = lk.base_lora_fwd(x, w, s, b, tile_adapter=ta)
+    ds = lk.lora_ds(dy, b, tile_adapter=ta, adapter_scale=sc)
+    dx = lk.base_lora_dx(dy, w, ds, a, tile_adapter=ta, dropout=drop)
+    da, db = torch.zeros(n, R, K, device="cuda"), torch.zeros(n, N, R, device="cuda")
+    lk.lora_db(dy, s, segs, db)
+    lk.lora_da(x, ds, segs, da, dropout=drop)
+    got_y, got_s = lk.linear_fwd(x, w, a, b, info, drop)
+    assert torch.equal(got_y, y) and torch.equal(got_s, s)
+    pitched = torch.full((M, R + 8), float("nan"), dtype=torch.bfloat16, device="cuda")[:, 8:]
+    pitched.copy_(s)
+    assert torch.equal(lk.linear_fwd(x, w, None, b, info, drop, s=pitched)[0], y)
+    got_da, got_db = torch.zeros_like(da), torch.zeros_like(db)
+    assert torch.equal(lk.linear_bwd(dy, x, pitched, w, a, b, info, drop, got_da, got_db, True), dx)
+    assert torch.equal(got_da, da) and torch.equal(got_db, db)
+
+
 def test_fused_multi_lora_gradients_of_a_partly_missing_adapter():
     """``A`` missing while ``B`` is given: that adapter contributes nothing and its ``B`` gets no gradient; the
     other one's gradients are those of a layer that holds it alone.  Wrong shapes and types are refused."""
