@@ -49,7 +49,9 @@ __device__ __forceinline__ unsigned long long exp_pair(uint32_t w, unsigned long
 // to 158 us of memory traffic, so the rest of the arithmetic is done two logits at a time, the label's
 // column apart, and four vectors of a thread are in flight: 265 -> 233 us (either alone gave nothing,
 // nor did keeping part of the row in shared memory instead of reading it twice).
-// labels < 0 are ignored (loss 0, gradient 0).  grad_scale multiplies the gradient
+// labels < 0 are ignored (loss 0, gradient 0).  A label of V or more, which the embedding would clamp, has
+// no column: the gradient is that of the log-sum-exp alone, the loss takes the last column's logit, and
+// nothing outside the row's V columns is touched.  grad_scale multiplies the gradient
 // (1 / number of valid tokens for a mean loss).
 __global__ void __launch_bounds__(CE_THREADS)
 cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__ labels,
@@ -122,9 +124,13 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
     bs += (red_m[i] == -INFINITY) ? 0.f : red_s[i] * __expf(red_m[i] - bm);
   const float lse = bm + __logf(bs);
   const float inv_sum = 1.f / bs, scale = inv_sum * grad_scale;
-  const float label_logit = __bfloat162float(lr[label]);
-  __syncthreads();  // everyone has read lr[label] before it is overwritten
-  if (threadIdx.x == 0) loss_out[row] = lse - label_logit;
+  const float label_logit = __bfloat162float(lr[min(label, V - 1)]);
+  __syncthreads();  // everyone has read the label's logit before it is overwritten
+  float* label_grad = red_m;   // kept there by thread 0: in a register it would be spilled over the second pass
+  if (threadIdx.x == 0) {
+    loss_out[row] = lse - label_logit;
+    *label_grad = (__expf(label_logit - bm) * inv_sum - 1.f) * grad_scale;
+  }
 
   const unsigned long long neg_bm2 = f32x2(-bm, -bm), scale2 = f32x2(scale, scale);
   for (int c0 = threadIdx.x; c0 < nvec; c0 += CE_VECS * CE_THREADS) {
@@ -151,7 +157,8 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
   }
   __syncthreads();
   // the label's column, which the loops above treated like any other
-  if (threadIdx.x == 0) lr[label] = __float2bfloat16((__expf(label_logit - bm) * inv_sum - 1.f) * grad_scale);
+  // (patching it into its vector on the way cost 7 % at V = 50257: one more comparison a vector)
+  if (threadIdx.x == 0 && label < V) lr[label] = __float2bfloat16(*label_grad);
 }
 
 // ---------------------------------------------------------------------------------

@@ -280,3 +280,34 @@ def test_fused_multi_lora_gradients_of_a_partly_missing_adapter():
         fused_linear_lora(x.float(), w, a, b, 2.0)
     with pytest.raises(ValueError):
         fused_linear_lora(x, w, a[:, :64], b, 2.0)
+
+
+@pytest.mark.parametrize("V", [64, 1000, 50257])
+def test_cross_entropy_stays_inside_its_row(V):
+    """Labels in the first and last column, ignored ones and ones of V or more (up to the next row and past the last):
+    rows with a valid label get exactly what they get alone, columns past V and the memory behind stay as they were,
+    and a row whose label has no column gets softmax * grad_scale."""
+    from lorafusion_b200.ops import elementwise as ew
+
+    ld, scale = V // 8 * 8 + 16, 0.25
+    labels = [0, V, V - 1, V + 7, -1, ld + 3, V // 2, 5 * V]
+    buf = _rand(len(labels) + 2, ld, seed=1)
+    before = buf.clone()
+    lab = torch.tensor(labels, dtype=torch.int32, device="cuda")
+    loss = ew.cross_entropy_inplace(buf[:len(labels), :V], lab, scale)
+    assert torch.equal(buf[:, V:], before[:, V:]) and torch.equal(buf[len(labels):], before[len(labels):])
+    for i, label in enumerate(labels):
+        logits = before[i, :V].float()
+        want = logits.softmax(0)
+        if 0 <= label < V:
+            want[label] -= 1
+        elif label < 0:
+            want.zero_()
+        # bf16 results (2^-9 of the value) of fp32 exponentials
+        assert torch.allclose(buf[i, :V].float(), want * scale, rtol=6e-3, atol=1e-6), label
+        ref = 0.0 if label < 0 else float(logits.logsumexp(0) - logits[min(label, V - 1)])
+        assert abs(float(loss[i]) - ref) < 1e-3
+        alone = before[i:i + 1].clone()
+        if label < V:
+            ew.cross_entropy_inplace(alone[:, :V], lab[i:i + 1], scale)
+            assert torch.equal(alone[0], buf[i]), label
