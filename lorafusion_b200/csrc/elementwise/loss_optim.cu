@@ -20,7 +20,6 @@
 
 namespace lf {
 
-constexpr int CE_THREADS = 512;
 constexpr int CE_VECS = 4;   // 16-byte vectors in flight a thread
 
 __device__ __forceinline__ float warp_max(float v) {
@@ -49,15 +48,20 @@ __device__ __forceinline__ unsigned long long exp_pair(uint32_t w, unsigned long
 // to 158 us of memory traffic, so the rest of the arithmetic is done two logits at a time, the label's
 // column apart, and four vectors of a thread are in flight: 265 -> 233 us (either alone gave nothing,
 // nor did keeping part of the row in shared memory instead of reading it twice).
+// Rows of at most 4096 logits, one batch of vectors of 128 threads, get CTAs of that size: they wait for
+// memory and for one another most of the time, and of the larger CTAs, whose registers leave room for
+// three on an SM instead of four, too few are resident (2048 rows of 64, 1000, 4096: 5.6, 5.8, 8.7 us, and
+// 14.3, 14.3, 17.5 us in CTAs of 512).
 // labels < 0 are ignored (loss 0, gradient 0).  A label of V or more, which the embedding would clamp, has
 // no column: the gradient is that of the log-sum-exp alone, the loss takes the last column's logit, and
 // nothing outside the row's V columns is touched.  grad_scale multiplies the gradient
 // (1 / number of valid tokens for a mean loss).
-__global__ void __launch_bounds__(CE_THREADS)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
 cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__ labels,
                      float* __restrict__ loss_out, int V, long long ld, float grad_scale) {
-  __shared__ float red_m[CE_THREADS / 32];
-  __shared__ float red_s[CE_THREADS / 32];
+  __shared__ float red_m[THREADS / 32];
+  __shared__ float red_s[THREADS / 32];
   const long long row = blockIdx.x;
   __nv_bfloat16* lr = logits + row * ld;
   const int label = labels[row];
@@ -66,22 +70,22 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
 
   if (label < 0) {
     const uint4 z = make_uint4(0, 0, 0, 0);
-    for (int c = threadIdx.x; c < nvec; c += CE_THREADS) reinterpret_cast<uint4*>(lr)[c] = z;
-    for (int c = nvec * 8 + threadIdx.x; c < V; c += CE_THREADS) lr[c] = __float2bfloat16(0.f);
+    for (int c = threadIdx.x; c < nvec; c += THREADS) reinterpret_cast<uint4*>(lr)[c] = z;
+    for (int c = nvec * 8 + threadIdx.x; c < V; c += THREADS) lr[c] = __float2bfloat16(0.f);
     if (threadIdx.x == 0) loss_out[row] = 0.f;
     return;
   }
 
   const unsigned long long log2e2 = f32x2(1.4426950408889634f, 1.4426950408889634f);
   float m = -INFINITY, s = 0.f;
-  for (int c0 = threadIdx.x; c0 < nvec; c0 += CE_VECS * CE_THREADS) {
+  for (int c0 = threadIdx.x; c0 < nvec; c0 += CE_VECS * THREADS) {
     uint4 raw[CE_VECS];
 #pragma unroll
     for (int k = 0; k < CE_VECS; ++k)
-      if (c0 + k * CE_THREADS < nvec) raw[k] = reinterpret_cast<const uint4*>(lr)[c0 + k * CE_THREADS];
+      if (c0 + k * THREADS < nvec) raw[k] = reinterpret_cast<const uint4*>(lr)[c0 + k * THREADS];
 #pragma unroll
     for (int k = 0; k < CE_VECS; ++k) {
-      if (c0 + k * CE_THREADS >= nvec) continue;
+      if (c0 + k * THREADS >= nvec) continue;
       const uint32_t w[4] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w};
       // the maximum of bf16 values is one of them: taken on packed pairs
       const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(w);
@@ -100,7 +104,7 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
       s += s0 + s1;
     }
   }
-  for (int c = nvec * 8 + threadIdx.x; c < V; c += CE_THREADS) {
+  for (int c = nvec * 8 + threadIdx.x; c < V; c += THREADS) {
     const float f = __bfloat162float(lr[c]);
     if (f > m) {
       s *= __expf(m - f);
@@ -118,9 +122,9 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
   }
   __syncthreads();
   float bm = red_m[0];
-  for (int i = 1; i < CE_THREADS / 32; ++i) bm = fmaxf(bm, red_m[i]);
+  for (int i = 1; i < THREADS / 32; ++i) bm = fmaxf(bm, red_m[i]);
   float bs = 0.f;
-  for (int i = 0; i < CE_THREADS / 32; ++i)
+  for (int i = 0; i < THREADS / 32; ++i)
     bs += (red_m[i] == -INFINITY) ? 0.f : red_s[i] * __expf(red_m[i] - bm);
   const float lse = bm + __logf(bs);
   const float inv_sum = 1.f / bs, scale = inv_sum * grad_scale;
@@ -133,14 +137,14 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
   }
 
   const unsigned long long neg_bm2 = f32x2(-bm, -bm), scale2 = f32x2(scale, scale);
-  for (int c0 = threadIdx.x; c0 < nvec; c0 += CE_VECS * CE_THREADS) {
+  for (int c0 = threadIdx.x; c0 < nvec; c0 += CE_VECS * THREADS) {
     uint4 raw[CE_VECS];
 #pragma unroll
     for (int k = 0; k < CE_VECS; ++k)
-      if (c0 + k * CE_THREADS < nvec) raw[k] = reinterpret_cast<const uint4*>(lr)[c0 + k * CE_THREADS];
+      if (c0 + k * THREADS < nvec) raw[k] = reinterpret_cast<const uint4*>(lr)[c0 + k * THREADS];
 #pragma unroll
     for (int k = 0; k < CE_VECS; ++k) {
-      if (c0 + k * CE_THREADS >= nvec) continue;
+      if (c0 + k * THREADS >= nvec) continue;
       uint32_t w[4] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -148,10 +152,10 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
         unpack_f32x2(mul_f32x2(exp_pair(w[j], neg_bm2, log2e2), scale2), g0, g1);
         w[j] = pack_bf16x2(g0, g1);
       }
-      reinterpret_cast<uint4*>(lr)[c0 + k * CE_THREADS] = make_uint4(w[0], w[1], w[2], w[3]);
+      reinterpret_cast<uint4*>(lr)[c0 + k * THREADS] = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
-  for (int c = nvec * 8 + threadIdx.x; c < V; c += CE_THREADS) {
+  for (int c = nvec * 8 + threadIdx.x; c < V; c += THREADS) {
     const float f = __bfloat162float(lr[c]);
     lr[c] = __float2bfloat16(__expf(f - bm) * scale);
   }
@@ -295,8 +299,12 @@ int lf_cross_entropy(void* logits, const int* labels, float* loss, long long M, 
                      long long ld, float grad_scale, void* stream) {
   if (M == 0) return 0;
   if (ld % 8 != 0) return -1;
-  cross_entropy_kernel<<<(unsigned)M, CE_THREADS, 0, (cudaStream_t)stream>>>(
-      (__nv_bfloat16*)logits, labels, loss, V, ld, grad_scale);
+  if (V <= 128 * CE_VECS * 8)
+    cross_entropy_kernel<128><<<(unsigned)M, 128, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)logits, labels, loss, V, ld,
+                                                                             grad_scale);
+  else
+    cross_entropy_kernel<512><<<(unsigned)M, 512, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)logits, labels, loss, V, ld,
+                                                                             grad_scale);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

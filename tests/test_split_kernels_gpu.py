@@ -282,7 +282,7 @@ def test_fused_multi_lora_gradients_of_a_partly_missing_adapter():
         fused_linear_lora(x, w, a[:, :64], b, 2.0)
 
 
-@pytest.mark.parametrize("V", [64, 1000, 50257])
+@pytest.mark.parametrize("V", [1, 64, 1000, 4096, 4097, 50257])
 def test_cross_entropy_stays_inside_its_row(V):
     """Labels in the first and last column, ignored ones and ones of V or more (up to the next row and past the last):
     rows with a valid label get exactly what they get alone, columns past V and the memory behind stay as they were,
