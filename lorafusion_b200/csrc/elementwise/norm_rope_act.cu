@@ -400,8 +400,7 @@ int lf_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rs
 int lf_rope_inplace(void* qkv, const int* pos, const float* cos_t, const float* sin_t, int M,
                     int n_rot_heads, int D, int row_stride, int backward, void* stream) {
   if (D % 16 != 0 || row_stride % 8 != 0) return -1;
-  if (M == 0) return 0;
-  if (n_rot_heads <= 0) return 0;
+  if (M == 0 || n_rot_heads <= 0 || D <= 0) return 0;
   const int bx = D / 16 < ROPE_THREADS ? D / 16 : ROPE_THREADS;
   int by = ROPE_THREADS / bx;
   if (by > n_rot_heads) by = n_rot_heads;
