@@ -190,17 +190,21 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 // QKV activation [M, (Hq + 2 Hkv) * D].  cos/sin come from a table [max_pos, D/2] gathered
 // by position id.  `sign` = +1 forward, -1 backward (the transpose of a rotation).
 // ---------------------------------------------------------------------------------
-// One CTA per token; threadIdx.x = 16-byte vector of a half head, threadIdx.y = head.  A thread keeps
-// its piece of the cos / sin row for all the heads it rotates (two at a time), and the first heads are on
-// their way before the position that selects the row is known.  (A flat index over all vectors spent
-// its time in two 64-bit divisions and a cos / sin load per vector: 92 us for 16384 tokens of 40 heads.)
+// One CTA per token, or as many tokens as fill it where there are few heads; threadIdx.x = 16-byte vector
+// of a half head, threadIdx.y = head, threadIdx.z = token.  A thread keeps its piece of the cos / sin row
+// for all the heads it rotates, two at a time and as many as every other thread (lf_rope_inplace), and
+// the first heads are on their way before the position that selects the row is known.  16384 tokens of 1,
+// 40 and 72 heads of 128: 6.2, 66, 105 us; 6.8, 74, 126 with a flat index over all vectors, two
+// 64-bit divisions and a cos / sin load each; 11, 75, 118 with one token a CTA and 32 heads at a time,
+// where a quarter of the threads rotated two of 40 heads and the others one.
 constexpr int ROPE_THREADS = 256;
 
 __global__ void __launch_bounds__(ROPE_THREADS)
 rope_inplace_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ pos, const float* __restrict__ cos_t,
-                    const float* __restrict__ sin_t, int n_rot_heads, int D, int row_stride, float sign) {
+                    const float* __restrict__ sin_t, int M, int n_rot_heads, int D, int row_stride, float sign) {
   const int half = D / 2;
-  const long long row = blockIdx.x;
+  const long long row = (long long)blockIdx.x * blockDim.z + threadIdx.z;
+  if (row >= M) return;
   const int by = blockDim.y;
   for (int vi = threadIdx.x; vi < half / 8; vi += blockDim.x) {   // (once, up to head size 4096)
     __nv_bfloat16* base = qkv + row * row_stride + vi * 8;
@@ -403,9 +407,16 @@ int lf_rope_inplace(void* qkv, const int* pos, const float* cos_t, const float* 
   if (M == 0 || n_rot_heads <= 0 || D <= 0) return 0;
   const int bx = D / 16 < ROPE_THREADS ? D / 16 : ROPE_THREADS;
   int by = ROPE_THREADS / bx;
-  if (by > n_rot_heads) by = n_rot_heads;
-  rope_inplace_kernel<<<(unsigned)M, dim3(bx, by), 0, (cudaStream_t)stream>>>(
-      (__nv_bfloat16*)qkv, pos, cos_t, sin_t, n_rot_heads, D, row_stride, backward ? -1.f : 1.f);
+  if (by < n_rot_heads) {   // an even number of heads a thread, the same for all but the last
+    const int per = ((n_rot_heads + by - 1) / by + 1) / 2 * 2;
+    by = (n_rot_heads + per - 1) / per;
+  } else {
+    by = n_rot_heads;
+  }
+  int bz = ROPE_THREADS / (bx * by);
+  if (bz > 64) bz = 64;   // the most a block may have in z
+  rope_inplace_kernel<<<((unsigned)M + bz - 1) / bz, dim3(bx, by, bz), 0, (cudaStream_t)stream>>>(
+      (__nv_bfloat16*)qkv, pos, cos_t, sin_t, M, n_rot_heads, D, row_stride, backward ? -1.f : 1.f);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

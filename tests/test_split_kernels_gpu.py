@@ -311,3 +311,23 @@ def test_cross_entropy_stays_inside_its_row(V):
         if label < V:
             ew.cross_entropy_inplace(alone[:, :V], lab[i:i + 1], scale)
             assert torch.equal(alone[0], buf[i]), label
+
+
+@pytest.mark.parametrize("M,heads,D", [(1, 1, 128), (129, 1, 16), (67, 1, 128), (100, 5, 128), (33, 40, 128), (7, 3, 256),
+                                       (65, 2, 64)])
+def test_rope_with_several_tokens_a_block(M, heads, D):
+    """Token counts that leave the last block ragged; the heads behind the rotated ones and the rows behind the batch
+    stay as they were."""
+    from lorafusion_b200.ops import elementwise as ew
+
+    qkv = _rand(M + 70, (heads + 1) * D, seed=3)
+    before = qkv.clone()
+    pos = torch.randint(0, 50, (M,), device="cuda", dtype=torch.int32)
+    ang = torch.rand(50, D // 2, device="cuda") * 6
+    ew.rope_inplace(qkv[:M], pos, ang.cos(), ang.sin(), heads, D)
+    c, s = ang.cos()[pos.long()][:, None], ang.sin()[pos.long()][:, None]
+    lo, hi = before[:M, :heads * D].float().view(M, heads, 2, D // 2).unbind(2)
+    ref = torch.stack([lo * c - hi * s, hi * c + lo * s], dim=2).reshape(M, heads * D)
+    # fp32 arithmetic rounded to bf16 once: half an ulp is 2^-9 of the value, plus cancellation of fp32 products
+    assert torch.allclose(qkv[:M, :heads * D].float(), ref, rtol=4e-3, atol=1e-5)
+    assert torch.equal(qkv[:M, heads * D:], before[:M, heads * D:]) and torch.equal(qkv[M:], before[M:])
