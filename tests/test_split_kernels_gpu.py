@@ -331,3 +331,16 @@ def test_rope_with_several_tokens_a_block(M, heads, D):
     # fp32 arithmetic rounded to bf16 once: half an ulp is 2^-9 of the value, plus cancellation of fp32 products
     assert torch.allclose(qkv[:M, :heads * D].float(), ref, rtol=4e-3, atol=1e-5)
     assert torch.equal(qkv[:M, heads * D:], before[:M, heads * D:]) and torch.equal(qkv[M:], before[M:])
+
+
+@pytest.mark.parametrize("M,I", [(1, 8), (300, 8), (65, 24), (257, 64), (100, 1000), (33, 2056), (3, 4104), (5, 8200)])
+def test_swiglu_backward_of_short_and_long_rows(M, I):
+    """Rows that share a CTA, one row a CTA (2056 to 4096) and rows in pieces; ragged last CTAs and odd vector counts."""
+    from lorafusion_b200.ops import elementwise as ew
+
+    gu, d = _rand(M, 2 * I, seed=1), _rand(M, I, seed=2)
+    leaf = gu.float().requires_grad_(True)
+    g, u = leaf.split(I, dim=1)
+    ref, = torch.autograd.grad(torch.nn.functional.silu(g) * u, [leaf], d.float())
+    # fp32 arithmetic with an approximate exponential (2^-22), rounded to bf16 once
+    assert torch.allclose(ew.swiglu_bwd(d, gu).float(), ref, rtol=5e-3, atol=1e-5)
