@@ -273,19 +273,43 @@ adam_chunks_kernel(const AdamChunk* __restrict__ chunks, const AdamWorkItem* __r
     }
     return;
   }
-  for (long long i = (long long)item.first + first; i < (long long)item.first + item.count; i += 256 * kAdamShares) {
-    const long long e = c.offset + i;
-    const float g = grad[e] * h.grad_scale;
-    grad[e] = 0.f;
-    const long long col = i % c.ld;
-    if (col < c.col0 || col >= c.col0 + c.cols) continue;
-    const long long se = c.state + (i / c.ld) * c.cols + (col - c.col0);
-    float w = master[se], mi = m[se], vi = v[se];
-    adam_one(g, w, mi, vi, h, inv_c1, inv_sqrt_c2);
-    m[se] = mi;
-    v[se] = vi;
-    master[se] = w;
-    work[e] = __float2bfloat16(w);
+  // Anything else: the same, an element at a time (indices inside a region fit the items' 32 bits).  Sixteen
+  // regions of 3000 x 30: 11 us; 26 with the elements of a thread one after the other, and 19 so in one
+  // CTA an item.
+  const unsigned ld = unsigned(c.ld), end = item.first + item.count;
+  constexpr int U = 2;
+  for (unsigned i0 = item.first + first; i0 < end; i0 += U * 256u * kAdamShares) {
+    float g[U], w[U], mi[U], vi[U];
+    long long se[U];
+    bool live[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const unsigned i = i0 + k * 256u * kAdamShares;
+      live[k] = false;
+      if (i < end) {
+        const unsigned row = i / ld;
+        const long long col = (long long)(i - row * ld) - c.col0;
+        live[k] = col >= 0 && col < c.cols;
+        se[k] = c.state + row * c.cols + col;
+        if (live[k]) {
+          g[k] = grad[c.offset + i];
+          w[k] = master[se[k]];
+          mi[k] = m[se[k]];
+          vi[k] = v[se[k]];
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const unsigned i = i0 + k * 256u * kAdamShares;
+      if (i < end) grad[c.offset + i] = 0.f;
+      if (!live[k]) continue;
+      adam_one(g[k] * h.grad_scale, w[k], mi[k], vi[k], h, inv_c1, inv_sqrt_c2);
+      m[se[k]] = mi[k];
+      v[se[k]] = vi[k];
+      master[se[k]] = w[k];
+      work[c.offset + i] = __float2bfloat16(w[k]);
+    }
   }
 }
 

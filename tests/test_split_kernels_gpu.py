@@ -344,3 +344,31 @@ def test_swiglu_backward_of_short_and_long_rows(M, I):
     ref, = torch.autograd.grad(torch.nn.functional.silu(g) * u, [leaf], d.float())
     # fp32 arithmetic with an approximate exponential (2^-22), rounded to bf16 once
     assert torch.allclose(ew.swiglu_bwd(d, gu).float(), ref, rtol=5e-3, atol=1e-5)
+
+
+@pytest.mark.parametrize("rows,ld,col0,cols", [(700, 30, 3, 24), (1, 12289, 0, 12289), (333, 7, 0, 7), (300, 64, 16, 16)])
+def test_adam_regions_of_any_size(rows, ld, col0, cols):
+    """One update of regions with odd sizes (the last one vectorisable), longer than what the CTAs of a work item take in
+    one go: weights, moments, bf16 copy and cleared gradient; memory around the region untouched."""
+    from lorafusion_b200.ops import elementwise as ew
+
+    n, off, st = rows * ld, 12, 8
+    g0 = torch.Generator(device="cuda").manual_seed(7)
+    grad, mas, m, v = (torch.rand(k, generator=g0, device="cuda") + 0.1 for k in [n + 40] + [rows * cols + 20] * 3)
+    work = torch.full((n + 40,), 3.0, dtype=torch.bfloat16, device="cuda")
+    want = [t[st:st + rows * cols].clone() for t in (mas, m, v)]
+    before = [t.clone() for t in (grad, mas, m, v)]
+    table = torch.tensor([[off, rows, ld, col0, cols, st]], dtype=torch.int64, device="cuda")
+    ew.adam_chunks(table, grad, mas, m, v, work, lr=0.01, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=1, grad_scale=0.5)
+    g = 0.5 * before[0][off:off + n].view(rows, ld)[:, col0:col0 + cols].reshape(-1)
+    want[1] = 0.9 * want[1] + 0.1 * g
+    want[2] = 0.95 * want[2] + 0.05 * g * g
+    want[0] = want[0] * (1 - 0.01 * 0.1) - 0.01 * (want[1] / (1 - 0.9)) / ((want[2] / (1 - 0.95)).sqrt() + 1e-8)
+    # fp32 with approximate divisions and roots (2^-22) of values around one
+    for got, ref, old in zip((mas, m, v), want, before[1:]):
+        assert torch.allclose(got[st:st + rows * cols], ref, rtol=1e-5, atol=1e-6)
+        assert torch.equal(got[:st], old[:st]) and torch.equal(got[st + rows * cols:], old[st + rows * cols:])
+    copy = torch.full((rows, ld), 3.0, dtype=torch.bfloat16, device="cuda")
+    copy[:, col0:col0 + cols] = mas[st:st + rows * cols].to(torch.bfloat16).view(rows, cols)
+    assert torch.equal(work[off:off + n], copy.view(-1)) and (work[:off] == 3).all() and (work[off + n:] == 3).all()
+    assert not grad[off:off + n].any() and torch.equal(grad[off + n:], before[0][off + n:])
