@@ -372,3 +372,17 @@ def test_adam_regions_of_any_size(rows, ld, col0, cols):
     copy[:, col0:col0 + cols] = mas[st:st + rows * cols].to(torch.bfloat16).view(rows, cols)
     assert torch.equal(work[off:off + n], copy.view(-1)) and (work[:off] == 3).all() and (work[off + n:] == 3).all()
     assert not grad[off:off + n].any() and torch.equal(grad[off + n:], before[0][off + n:])
+
+
+@pytest.mark.parametrize("blocks", [1, 127, 128, 129, 300, 7104 * 16 + 5])
+@pytest.mark.parametrize("double_quant", [True, False])
+def test_nf4_expansion_around_the_work_of_a_cta(blocks, double_quant):
+    """A CTA expands 128 blocks of 64 codes at a time; 888 persistent ones (second-level scales) or one a piece."""
+    from lorafusion_b200.ops import nf4
+
+    q = nf4.quantize_nf4(_rand(blocks, 64, seed=2), double_quant)
+    out = torch.full((blocks + 2, 64), 7.0, dtype=torch.bfloat16, device="cuda")
+    nf4.dequantize_nf4(q, out=out[:blocks])
+    # the product of two fp32 values, rounded to bf16; the scale may be fused (2^-24)
+    assert torch.allclose(out[:blocks].float(), nf4.dequantize_nf4_reference(q).float(), rtol=8e-3, atol=1e-6)
+    assert (out[blocks:] == 7).all()
