@@ -124,7 +124,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 // RMSNorm backward (no weight grad):
 //   g = dy * w;  dx = rstd * (g - xhat * mean(g * xhat))  (+ dres),  xhat = h * rstd
 template <int NV>
-__global__ void __launch_bounds__(NORM_THREADS, NV <= 2 ? 5 : (NV <= 4 ? 3 : 2))
+__global__ void __launch_bounds__(NORM_THREADS, NV <= 1 ? 8 : (NV <= 2 ? 5 : (NV <= 4 ? 3 : 2)))
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx, int H) {
@@ -134,7 +134,9 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   const float rstd = rstd_in[row];
   // The row is read once and waits for the dot product as the bf16 it came in, four registers per
   // vector.  (Kept as fp32 it cost 96-106 registers a thread and with them the resident CTAs that
-  // hide the DRAM latency; read a second time it cost L2 bandwidth: 173 us for 16384 x 4096.)
+  // hide the DRAM latency; read a second time it cost L2 bandwidth: 173 us for 16384 x 4096, 98 so.
+  // 8192 rows of 10240, 12288, 16384: 163, 195, 261 us with the second read, 122, 139, 178 so.  Rows of
+  // up to 2048 need room for eight CTAs: at five, 8192 x 64 took 10.7 us, 9.3 at eight.)
   uint4 gv[NV], hv[NV], rv[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {

@@ -386,3 +386,22 @@ def test_nf4_expansion_around_the_work_of_a_cta(blocks, double_quant):
     # the product of two fp32 values, rounded to bf16; the scale may be fused (2^-24)
     assert torch.allclose(out[:blocks].float(), nf4.dequantize_nf4_reference(q).float(), rtol=8e-3, atol=1e-6)
     assert (out[blocks:] == 7).all()
+
+
+@pytest.mark.parametrize("H", [8, 64, 2048, 2056, 8200, 16384])
+@pytest.mark.parametrize("with_residual", [False, True])
+def test_rmsnorm_backward_of_short_and_long_rows(H, with_residual):
+    """Every number of vectors a thread keeps (1, 2, 5 to 8), few columns and the widest rows."""
+    from lorafusion_b200.ops import elementwise as ew
+
+    M = 37
+    x, w, dy, dres = _rand(M, H, seed=1), _rand(H, seed=2), _rand(M, H, seed=3), _rand(M, H, seed=4)
+    _, h, rstd = ew.rmsnorm_fwd(x, w, 1e-5)
+    leaf = x.float().requires_grad_(True)
+    y = leaf * torch.rsqrt(leaf.pow(2).mean(1, keepdim=True) + 1e-5) * w.float()
+    ref, = torch.autograd.grad(y, [leaf], dy.float())
+    if with_residual:
+        ref = ref + dres.float()
+    got = ew.rmsnorm_bwd(dy, h, w, rstd, dres if with_residual else None)
+    # fp32 sums in another order, rounded to bf16 once (2^-9 of values around one)
+    assert torch.allclose(got.float(), ref, rtol=6e-3, atol=2e-3)
