@@ -41,42 +41,60 @@ constexpr int BWD_SMEM = ATT_TILE_BYTES * 7 + 256 + 1024;
 // quarter warp % 4).  The backward needs no row reductions, so the halves never talk.
 constexpr int BWD_THREADS = 64 + 256;
 
-// Bound by the reads of O and dO.  A CTA takes eight rows of sixteen heads: each warp reads 4 KB of one
-// row from either matrix, all thirty-two loads in flight, and the sums leave eight rows of a head
-// (32 bytes) at a time through shared memory.  (One head of a row a warp, two loads in flight and single
-// 4-byte stores: 148 us for 16384 rows of 64 heads, 3.6 TB/s.  A warp on sixteen rows of one head, so
-// that it could store them itself, took 194 us, and forming delta inside the dQ kernel cost
-// 220 us there: each head started with the loads' latency.)
-constexpr int DELTA_HEADS = 16;
+// Bound by the reads of O and dO.  A warp takes sixteen (row, head) pairs, neighbouring heads of one row
+// where there are that many (a CTA: eight rows of sixteen heads, each warp reading 4 KB of a row from
+// either matrix), else HEADS heads of 16 / HEADS rows; all thirty-two loads are in flight, and the sums
+// leave at least eight rows of a head (32 bytes) at a time through shared memory.  (One head of a row a
+// warp, two loads in flight and single 4-byte stores: 148 us for 16384 rows of 64 heads, 3.6 TB/s, and 92
+// so.  A warp on sixteen rows of one head, so that it could store them itself, took 194 us there, and
+// forming delta inside the dQ kernel cost 220 us: each head started with the loads' latency.  With
+// sixteen heads a warp also where there are two, most of its shuffles added zeros: the backward of 64
+// sequences of 256 tokens and two heads 53 us, 44.5 so, 48.5 with one head of a row a warp.)
+constexpr int DELTA_PAIRS = 16;
 
+template <int HEADS>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta,
                   long long M, int Hq, long long ld) {
-  __shared__ float sums[DELTA_HEADS][8];
-  const int groups = (Hq + DELTA_HEADS - 1) / DELTA_HEADS;
-  const int h0 = int(blockIdx.x % groups) * DELTA_HEADS;
-  const long long m0 = (long long)(blockIdx.x / groups) * 8;
+  constexpr int WROWS = DELTA_PAIRS / HEADS, ROWS = 8 * WROWS;   // of a warp, of the CTA
+  __shared__ float sums[HEADS][ROWS];
+  const int groups = (Hq + HEADS - 1) / HEADS;
+  const int h0 = int(blockIdx.x % groups) * HEADS;
+  const long long m0 = (long long)(blockIdx.x / groups) * ROWS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = m0 + warp < M ? min(DELTA_HEADS, Hq - h0) : 0;
-  const long long off = (m0 + warp) * ld + h0 * ATT_D + lane * 4;
-  uint2 a[DELTA_HEADS], b[DELTA_HEADS];
+  const int heads = min(HEADS, Hq - h0);
+  const long long left = M - (m0 + warp * WROWS);
+  const int rows = left < WROWS ? int(left) : WROWS;   // (none or fewer in the last CTA)
+  const long long off = (m0 + warp * WROWS) * ld + h0 * ATT_D + lane * 4;
+  uint2 a[DELTA_PAIRS], b[DELTA_PAIRS];
 #pragma unroll
-  for (int i = 0; i < DELTA_HEADS; ++i) {
-    a[i] = i < n ? *reinterpret_cast<const uint2*>(o + off + i * ATT_D) : make_uint2(0u, 0u);
-    b[i] = i < n ? *reinterpret_cast<const uint2*>(d_o + off + i * ATT_D) : make_uint2(0u, 0u);
+  for (int i = 0; i < DELTA_PAIRS; ++i) {
+    const bool in = i / HEADS < rows && i % HEADS < heads;
+    const long long at = off + i / HEADS * ld + i % HEADS * ATT_D;
+    a[i] = in ? *reinterpret_cast<const uint2*>(o + at) : make_uint2(0u, 0u);
+    b[i] = in ? *reinterpret_cast<const uint2*>(d_o + at) : make_uint2(0u, 0u);
   }
 #pragma unroll
-  for (int i = 0; i < DELTA_HEADS; ++i) {
+  for (int i = 0; i < DELTA_PAIRS; ++i) {
     const float2 x0 = unpack_bf16x2(a[i].x), x1 = unpack_bf16x2(a[i].y);
     const float2 y0 = unpack_bf16x2(b[i].x), y1 = unpack_bf16x2(b[i].y);
     float t = x0.x * y0.x + x0.y * y0.y + x1.x * y1.x + x1.y * y1.y;
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
-    if (lane == i) sums[i][warp] = t;
+    if (lane == i) sums[i % HEADS][warp * WROWS + i / HEADS] = t;
   }
   __syncthreads();
-  const int i = threadIdx.x >> 3, r = threadIdx.x & 7;
-  if (i < DELTA_HEADS && h0 + i < Hq && m0 + r < M) delta[(long long)(h0 + i) * M + m0 + r] = sums[i][r];
+  const int i = threadIdx.x / ROWS, r = threadIdx.x % ROWS;
+  if (i < heads && m0 + r < M) delta[(long long)(h0 + i) * M + m0 + r] = sums[i][r];
+}
+
+template <int HEADS>
+static void launch_delta(const void* out, const void* d_out, float* delta, long long M, int Hq, long long ld,
+                         cudaStream_t st) {
+  constexpr int ROWS = 8 * (DELTA_PAIRS / HEADS);
+  const long long blocks = (M + ROWS - 1) / ROWS * ((Hq + HEADS - 1) / HEADS);
+  attn_delta_kernel<HEADS><<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, delta,
+                                                             M, Hq, ld);
 }
 
 // The element-wise arithmetic of a thread's 64 columns, two at a time.
@@ -648,11 +666,10 @@ extern "C" int lf_attn_bwd(const void* qkv, const void* out, const void* d_out, 
   if (ensure_max_dynamic_smem(dq_configured, attn_dq_kernel, BWD_SMEM) != cudaSuccess ||
       ensure_max_dynamic_smem(dkdv_configured, attn_dkdv_kernel, BWD_SMEM) != cudaSuccess)
     return -10;
-  {
-    const long long blocks = (M + 7) / 8 * ((Hq + DELTA_HEADS - 1) / DELTA_HEADS);
-    attn_delta_kernel<<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, delta, M, Hq,
-                                                        ldo);
-  }
+  if (Hq > 8) launch_delta<16>(out, d_out, delta, M, Hq, ldo, st);
+  else if (Hq > 4) launch_delta<8>(out, d_out, delta, M, Hq, ldo, st);
+  else if (Hq > 2) launch_delta<4>(out, d_out, delta, M, Hq, ldo, st);
+  else launch_delta<2>(out, d_out, delta, M, Hq, ldo, st);
   AttnBwdParams p;
   p.tiles = (const int4*)tiles;
   p.num_tiles = num_tiles;
