@@ -7,7 +7,8 @@
 // is loaded once for both, and while the softmax warps of one head work on their scores the tensor
 // pipe runs the products of the other.  (One head at a time, with two threads per row that traded
 // row maxima through shared memory and P going through shared memory too, ran at 3.3K cycles
-// per key tile: the two sides took turns.)
+// per key tile: the two sides took turns.  Groups of one head have no pairs and still go that way,
+// attn_fwd_one_head.cu.)
 //   warp 0      TMA producer: Q of both heads, K and V tiles through two 2-stage rings
 //   warp 1      tcgen05.mma issuer: S = Q K^T, then O += P V with P read from tensor memory
 //   warps 2..5  softmax of the first head of the pair, one thread per query row; warps 6..9 of the second:
@@ -23,22 +24,9 @@
 #include "../common/launch.h"
 #include "../common/tensormap.h"
 #include "attn_common.cuh"
+#include "attn_fwd.h"
 
 namespace lf {
-
-struct AttnFwdParams {
-  const int4* tiles;
-  int num_tiles;
-  int Hq, Hkv;
-  int q_col0, k_col0, v_col0;
-  __nv_bfloat16* out;
-  long long ldo;
-  float* lse;
-  long long M_total;
-  float scale, scale_log2e;
-  int pairs_per_cta;  // head pairs of a group that one CTA walks (grid.y CTAs share a group)
-  int* err;
-};
 
 constexpr int FWD_THREADS = 64 + 256;  // TMA warp, MMA warp, four softmax warps per head of the pair
 constexpr int FWD_SMEM = ATT_TILE_BYTES * (2 + 4) + 256 + 1024;
@@ -333,8 +321,6 @@ extern "C" int lf_attn_fwd(const void* qkv, long long M, long long ld_qkv, int q
   CUtensorMap tm;
   int rc = make_tmap_2d_b16(&tm, qkv, (uint64_t)M, (uint64_t)ld_qkv, (uint64_t)ld_qkv, 128, 64, true);
   if (rc != 0) return -20 + rc;
-  static PerDeviceOnce configured;
-  if (ensure_max_dynamic_smem(configured, attn_fwd_kernel, FWD_SMEM) != cudaSuccess) return -10;
   AttnFwdParams p;
   p.tiles = (const int4*)tiles;
   p.num_tiles = num_tiles;
@@ -350,6 +336,9 @@ extern "C" int lf_attn_fwd(const void* qkv, long long M, long long ld_qkv, int q
   p.scale = scale;
   p.scale_log2e = scale * 1.4426950408889634f;
   p.err = err;
+  if (Hq == Hkv) return launch_attn_fwd_one_head(p, tm, (cudaStream_t)stream);   // no second head to pair with
+  static PerDeviceOnce configured;
+  if (ensure_max_dynamic_smem(configured, attn_fwd_kernel, FWD_SMEM) != cudaSuccess) return -10;
   // One CTA per (query tile, KV head) walks all head pairs of the group, which pays for its set-up
   // once, unless the launch would leave SMs idle: then the pairs of a group go to CTAs of their own.
   const int pairs = (Hq / Hkv + 1) / 2;

@@ -108,11 +108,13 @@ def test_pair_products_with_the_last_wave_cut(M, N, K, ctas, p):
 
 
 @pytest.mark.parametrize("lens,Hq,Hkv", [([1], 1, 1), ([129, 3, 128], 3, 1), ([300, 257], 10, 2), ([700, 31, 513], 8, 1),
-                                         ([128] * 150, 5, 1), ([65], 2, 2), ([200, 7], 17, 1), ([130], 4, 4)])
+                                         ([128] * 150, 5, 1), ([65], 2, 2), ([200, 7], 17, 1), ([130], 4, 4),
+                                         ([700, 31, 513], 4, 4), ([128, 1, 2000], 2, 2), ([600] * 50, 5, 5)])
 def test_attention_head_groups(lens, Hq, Hkv):
     """Odd groups (the last pair of heads has one), groups split over CTAs (few tiles) and whole
     (150 tiles), sequences around the tile size; forward, and backward with its row deltas (warps on 2, 4, 8
-    or 16 heads, 17 leave one to a group of its own)."""
+    or 16 heads, 17 leave one to a group of its own).  Groups of one head have a kernel of their own, in either order
+    of launch (fifty sequences of five heads: more than eight waves)."""
     from lorafusion_b200.ops import attention as att
 
     D, M = 128, sum(lens)
