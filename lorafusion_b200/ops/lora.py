@@ -196,7 +196,7 @@ def lora_linear_backward(dy: torch.Tensor, x: torch.Tensor, s: Optional[torch.Te
     if stack is None or info is None or s is None:
         return lk.base_lora_dx(dy, wd, None, None, tile_adapter=None) if need_dx else None
     drop = info.dropout_spec(stream_id, training)
-    if not isinstance(wd, NF4Weight):
+    if not isinstance(wd, NF4Weight) and (info.tile_adapter is None or not info.segment_table.repeats):
         return lk.linear_bwd(dy, x, s, wd if need_dx else None, stack.a, stack.b, info, drop, stack.da, stack.db, need_dx)
     ds = lk.lora_ds(dy, stack.b, tile_adapter=info.tile_adapter, adapter_scale=info.adapter_scale,
                     scale=getattr(info, "scale", 1.0))

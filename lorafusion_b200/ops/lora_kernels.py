@@ -108,7 +108,7 @@ def reduction_split(tiles: int, k_blocks: int) -> int:
 @dataclass
 class SegmentTable:
     """Token segments of one packed microbatch: ``(adapter, start, end)`` with ``start`` and
-    ``end`` multiples of 128 and at most one segment per adapter.  ``staged`` (optional):
+    ``end`` multiples of 128 and at most one segment per adapter (but see :meth:`passes`).  ``staged`` (optional):
     ``(int32 device tensor, first, end)`` where the :func:`segment_rows` of the segments already lie."""
 
     segments: Sequence[tuple[int, int, int]]
@@ -117,19 +117,26 @@ class SegmentTable:
     staged: Optional[tuple] = None
     _cache: dict = field(default_factory=dict)
 
-    def device_rows(self) -> torch.Tensor:
-        """int32 ``[n, 4]`` work list ``(adapter, start, end, 0)`` of the gradient kernels."""
+    @property
+    def repeats(self) -> bool:
+        """Whether an adapter owns more than one segment."""
+        return len(self._passes()) > 1
+
+    def _passes(self) -> list:
+        """How many rows of :func:`segment_rows` belong to each launch: first segments, second ones, ..."""
+        n = self._cache.get("passes")
+        if n is None:
+            n = [len(g) for g in _by_occurrence(self.segments)] or [0]
+            self._cache["passes"] = n
+        return n
+
+    def _rows(self) -> torch.Tensor:
+        """:func:`segment_rows` on the device."""
         t = self._cache.get("rows")
         if t is None:
-            seen = set()
             for adapter, start, end in self.segments:
-                if adapter < 0 or end <= start:
-                    continue
-                if adapter in seen:
-                    raise ValueError("an adapter may own only one token segment per microbatch")
-                seen.add(adapter)
                 last = self.total_rows is not None and end >= self.total_rows
-                if start % TILE_M or (end % TILE_M and not last):
+                if adapter >= 0 and end > start and (start % TILE_M or (end % TILE_M and not last)):
                     raise ValueError("segment bounds must be multiples of 128 tokens")
             if self.staged is not None:
                 src, first, end = self.staged
@@ -138,6 +145,21 @@ class SegmentTable:
                 t = torch.tensor(segment_rows(self.segments), dtype=torch.int32).reshape(-1, 4).to(self.device)
             self._cache["rows"] = t
         return t
+
+    def device_rows(self) -> torch.Tensor:
+        """int32 ``[n, 4]`` work list ``(adapter, start, end, 0)`` of the gradient kernels; every adapter once."""
+        if self.repeats:
+            raise ValueError("an adapter may own only one token segment per microbatch")
+        return self._rows()
+
+    def passes(self, features: int) -> list:
+        """The work lists of a gradient product of ``features`` features, to be launched one after the other: one,
+        unless an adapter owns several segments.  That is taken for long segments and few features (fewer than
+        96 pieces of segment x 128 features, a segment of 2048 tokens or more), where it has always worked."""
+        if self.repeats and (sum(self._passes()) * ((features + TILE_M - 1) // TILE_M) >= 96
+                             or max(e - s for a, s, e in self.segments if a >= 0) < 2048):
+            raise ValueError("an adapter may own only one token segment per microbatch")
+        return list(self._rows().split(self._passes()))
 
     def split_plan(self, features: int):
         """``(chunks per segment, owner)`` when the tokens of every segment are summed in several
@@ -157,12 +179,25 @@ class SegmentTable:
         return c
 
 
+def _by_occurrence(segments) -> list:
+    """``(adapter, start, end, 0)`` of every segment that has an adapter and tokens, in lists that name an adapter once:
+    the adapters' first segments, their second ones, ...  A list starts with its longest: its tiles start first, and the
+    short ones fill the gaps at the end."""
+    groups, count = [], {}
+    for a, s, e in segments:
+        if a >= 0 and e > s:
+            k = count[a] = count.get(a, -1) + 1
+            if k == len(groups):
+                groups.append([])
+            groups[k].append((a, s, e, 0))
+    for g in groups:
+        g.sort(key=lambda r: r[1] - r[2])
+    return groups
+
+
 def segment_rows(segments) -> list:
-    """``(adapter, start, end, 0)`` of every segment that has an adapter and tokens, the longest
-    first: its tiles start first, and the short ones fill the gaps at the end."""
-    rows = [(a, s, e, 0) for a, s, e in segments if a >= 0 and e > s]
-    rows.sort(key=lambda r: r[1] - r[2])
-    return rows
+    """:func:`_by_occurrence` as one list."""
+    return [r for g in _by_occurrence(segments) for r in g]
 
 
 def _flat2d(t: torch.Tensor) -> torch.Tensor:
@@ -227,11 +262,10 @@ def lora_db(dy: torch.Tensor, s: torch.Tensor, segs: SegmentTable, db_all: torch
     M, N = dy.shape
     n, N2, R = db_all.shape
     assert N2 == N and s.shape == (M, R) and db_all.dtype == torch.float32
-    rows = segs.device_rows()
-    if rows.shape[0] == 0:
-        return
-    launch_skinny(segs.chunks(N), a=dy, b=s, out=db_all, M=N, N=R, K=M, a_mn=True, b_mn=True, bn=R,
-                  epi=nv.EPI_F32_ACCUM, seg_tiles=rows, ldo=R, out_adapter_stride=N * R)
+    for rows in segs.passes(N):
+        if rows.shape[0] > 0:
+            launch_skinny(segs.chunks(N), a=dy, b=s, out=db_all, M=N, N=R, K=M, a_mn=True, b_mn=True, bn=R,
+                          epi=nv.EPI_F32_ACCUM, seg_tiles=rows, ldo=R, out_adapter_stride=N * R)
 
 
 def lora_da(x: torch.Tensor, ds: torch.Tensor, segs: SegmentTable, da_all: torch.Tensor, *,
@@ -240,12 +274,11 @@ def lora_da(x: torch.Tensor, ds: torch.Tensor, segs: SegmentTable, da_all: torch
     M, K = x.shape
     n, R, K2 = da_all.shape
     assert K2 == K and ds.shape == (M, R) and da_all.dtype == torch.float32
-    rows = segs.device_rows()
-    if rows.shape[0] == 0:
-        return
-    launch_skinny(segs.chunks(K), a=x, b=ds, out=da_all, M=K, N=R, K=M, a_mn=True, b_mn=True, bn=R,
-                  epi=nv.EPI_F32_ACCUM, mask_a=dropout.active, seg_tiles=rows, ldo=K,
-                  out_transposed=True, out_adapter_stride=R * K, **dropout.kwargs())
+    for rows in segs.passes(K):
+        if rows.shape[0] > 0:
+            launch_skinny(segs.chunks(K), a=x, b=ds, out=da_all, M=K, N=R, K=M, a_mn=True, b_mn=True, bn=R,
+                          epi=nv.EPI_F32_ACCUM, mask_a=dropout.active, seg_tiles=rows, ldo=K,
+                          out_transposed=True, out_adapter_stride=R * K, **dropout.kwargs())
 
 
 @dataclass
@@ -399,7 +432,9 @@ def linear_bwd(dy: torch.Tensor, x: Optional[torch.Tensor], s: Optional[torch.Te
         n = min(n, a_all.shape[0])
         dx = torch.empty((M, K), dtype=torch.bfloat16, device=dy.device)
         fields.update(a_all=a2d.data_ptr(), a_ld=a2d.stride(0), dx=dx.data_ptr())
-    if info.tile_adapter is None:
+    if da is None and db is None:
+        seg_rows, num_segs, split_da, split_db = None, 0, 1, 1
+    elif info.tile_adapter is None:
         seg_rows, num_segs = None, 1
         split_da, split_db = (reduction_split((f + TILE_M - 1) // TILE_M, (M + 63) // 64) for f in (K, N))
     else:

@@ -408,3 +408,47 @@ def test_rmsnorm_backward_of_short_and_long_rows(H, with_residual):
     got = ew.rmsnorm_bwd(dy, h, w, rstd, dres if with_residual else None)
     # fp32 sums in another order, rounded to bf16 once (2^-9 of values around one)
     assert torch.allclose(got.float(), ref, rtol=6e-3, atol=2e-3)
+
+
+@pytest.mark.parametrize("p", [0.0, 0.1])
+def test_multi_lora_of_an_adapter_with_several_segments(p):
+    """Three segments of adapter 0 around one of adapter 1: gradients are those of all its tokens.  Frozen adapters may
+    have short ones, too."""
+    from lorafusion_b200.ops import fused_linear_multi_lora
+    from lorafusion_b200.ops.philox import keep_mask
+
+    K, N, lens, ids, alpha = 256, 384, [2100, 128, 300, 100], [0, 1, 0, 0], {0: 2.0, 1: 0.5}
+    kw = dict(seq_len_list=lens, lora_idx_list=ids, alpha_list=[alpha[i] for i in ids], dropout_p_list=[p] * 4, seed=9,
+              stream_id=2)
+    starts = [0, 2176, 2304, 2688]
+    M = 2816
+    x, w = _rand(M, K, seed=1).requires_grad_(True), _rand(N, K, scale=0.05, seed=2)
+    ab = [(_rand(8, K, scale=0.1, seed=3 + i).requires_grad_(True), _rand(N, 8, scale=0.1, seed=5 + i).requires_grad_(True))
+          for i in range(2)]
+    for i, n in zip(starts, lens):   # (the rows between segments are padding)
+        with torch.no_grad():
+            x[i + n:(i + n + 127) // 128 * 128] = 0
+    dy = _rand(M, N, seed=9)
+    y = fused_linear_multi_lora(x, w, lora_a_list=[v[0] for v in ab], lora_b_list=[v[1] for v in ab], **kw)
+    got = torch.autograd.grad(y, [x] + [t for v in ab for t in v], dy)
+    leaves = [t.detach().float().requires_grad_(True) for t in [x] + [t for v in ab for t in v]]
+    keep = keep_mask(M, K, p, 9, 2).cuda() if p > 0 else torch.ones(M, K, dtype=torch.bool, device="cuda")
+    xh = torch.where(keep, leaves[0] / (1 - p), torch.zeros((), device="cuda"))
+    ref = leaves[0] @ w.float().t()
+    delta = torch.zeros_like(ref)
+    for i, n, ad in zip(starts, lens, ids):
+        rows = slice(i, (i + n + 127) // 128 * 128)
+        delta[rows] = alpha[ad] * (xh[rows] @ leaves[1 + 2 * ad].t()) @ leaves[2 + 2 * ad].t()
+    want = torch.autograd.grad(ref + delta, leaves, dy.float())
+    assert_close_two_rounds(y, ref + delta, msg="y")
+    for g, r, name in zip(got, want, ("dx", "dA0", "dB0", "dA1", "dB1")):
+        # S' and dS are rounded to bf16 (2^-9) on the way into sums of up to 2500 terms
+        assert_close_two_rounds(g, r, rtol=2e-2, atol=2e-2, scale_atol_by_rms=True, msg=name)
+    frozen = [t.detach() for v in ab for t in v]
+    short = dict(kw, seq_len_list=[128] * 4)
+    xs = x.detach()[:512].requires_grad_(True)
+    y = fused_linear_multi_lora(xs, w, lora_a_list=frozen[::2], lora_b_list=frozen[1::2], **short)
+    assert torch.autograd.grad(y, [xs], dy[:512])[0].shape == (512, K)
+    y = fused_linear_multi_lora(xs, w, lora_a_list=[v[0] for v in ab], lora_b_list=frozen[1::2], **short)
+    with pytest.raises(ValueError):
+        torch.autograd.grad(y, [ab[0][0]], dy[:512])

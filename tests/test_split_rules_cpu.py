@@ -40,3 +40,43 @@ def test_last_wave_is_cut_only_where_it_pays():
     assert scratch(1000, 8192, 8192, 0) == 0             # 54 of 74 pairs busy: 216 slices would cost more
     assert scratch(2048, 4096, 128256, 0) == 54 * 4 * tile + 3584     # 128 tiles of 2004 blocks
     assert scratch(0, 256, 256, 0) == 0
+
+
+def test_adapters_with_several_segments():
+    """Accepted where the tokens of a segment used to be summed in chunks (fewer than 96 pieces of segment x 128 features,
+    a segment of 2048 tokens): the n-th segments of all adapters form the n-th launch.  Refused otherwise."""
+    from lorafusion_b200.ops.lora_kernels import SegmentTable, segment_rows
+
+    segs = [(0, 0, 128), (1, 128, 384), (0, 384, 2560), (-1, 2560, 2688), (1, 2688, 2816), (0, 2816, 2944)]
+    assert segment_rows(segs) == [(1, 128, 384, 0), (0, 0, 128, 0), (0, 384, 2560, 0), (1, 2688, 2816, 0), (0, 2816, 2944, 0)]
+    for table in (SegmentTable(segs, torch.device("cpu")),
+                  SegmentTable(segs, torch.device("cpu"), staged=(torch.tensor([9] * 4 + [v for r in segment_rows(segs) for v in r],
+                                                                               dtype=torch.int32), 4, 24))):
+        assert table.repeats
+        got = [[tuple(r) for r in rows.tolist()] for rows in table.passes(128 * 19)]
+        assert got == [segment_rows(segs)[:2], segment_rows(segs)[2:4], segment_rows(segs)[4:]]
+        with pytest.raises(ValueError):
+            table.passes(128 * 19 + 1)      # 5 segments x 20 tiles
+    with pytest.raises(ValueError):
+        SegmentTable([(0, 0, 2047), (0, 2048, 2176)], torch.device("cpu")).passes(128)
+    with pytest.raises(ValueError):
+        SegmentTable([(0, 0, 1920), (0, 1920, 2176)], torch.device("cpu")).passes(128)
+    assert len(SegmentTable([(0, 0, 2048), (0, 2048, 2176)], torch.device("cpu")).passes(128)) == 2
+    one = SegmentTable([(0, 0, 128), (1, 128, 256)], torch.device("cpu"))
+    assert not one.repeats and torch.equal(one.passes(10 ** 6)[0], one.device_rows()) and len(one.passes(64)) == 1
+
+
+def test_frozen_adapters_may_have_several_segments(monkeypatch):
+    """The input's gradient alone needs no work list: such a batch is not refused, and does not take the one-call path."""
+    from lorafusion_b200.ops import lora as L
+    from lorafusion_b200.ops import lora_kernels as lk
+    from lorafusion_b200.ops.batch_info import prepare_multi_lora_batch_info
+
+    seen = []
+    for name in ("lora_ds", "lora_db", "lora_da", "base_lora_dx", "linear_bwd"):
+        monkeypatch.setattr(lk, name, lambda *a, _n=name, **k: seen.append(_n))
+    info = prepare_multi_lora_batch_info([128, 128], [0, 0], [8, 8], [0.0] * 2, [1.0] * 2, device="cpu")
+    z = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)  # noqa: E731
+    stack = L.LoRAStack(z(1, 64, 128), z(1, 128, 64))
+    L.lora_linear_backward(z(256, 128), z(256, 128), z(256, 64), z(128, 128), stack, info)
+    assert seen == ["lora_ds", "base_lora_dx"]
