@@ -284,6 +284,8 @@ def fused_linear_lora(x: torch.Tensor, linear_w: Weight, lora_a: torch.Tensor,
     if not x.is_cuda:
         return torch_ref_linear_lora(x, linear_w, lora_a, lora_b, alpha, dropout_p, seed,
                                      stream_id, linear_bias)
+    if lora_a is None or lora_b is None:
+        raise ValueError("fused_linear_lora needs A and B of its adapter")
     shape = x.shape
     x2d = x.reshape(-1, shape[-1]).contiguous()
     info = lk.OneAdapter(x2d.shape[0], float(alpha), float(dropout_p), seed)

@@ -293,6 +293,9 @@ class OneAdapter:
     tile_adapter = None
     adapter_scale = None
 
+    def __post_init__(self):
+        dropout_threshold(self.p)   # refuses what is no rate
+
     @property
     def segments(self) -> list:
         return [(0, 0, self.tokens)]

@@ -1,6 +1,7 @@
 """nn.Module wrappers (LoRALinear, MultiLoRALinear, apply_lora, merge_qkv_proj) on CPU, where the
 fused ops fall back to the plain-PyTorch oracle."""
 
+import pytest
 import torch
 from torch import nn
 
@@ -84,3 +85,22 @@ def test_apply_lora_and_merge_qkv():
     assert trainable and all("lora_" in n_ for n_ in trainable)
     streams = {m.stream_id for m in net.modules() if isinstance(m, LoRALinear)}
     assert len(streams) == sum(isinstance(m, LoRALinear) for m in net.modules())
+
+
+def test_single_adapter_call_refuses_what_the_batch_table_refused(monkeypatch):
+    """``fused_linear_lora`` builds no batch table any more; a missing adapter and a dropout rate that is no number are
+    refused all the same, before anything runs."""
+    from lorafusion_b200.ops import lora as L
+
+    class OnGpu(torch.Tensor):
+        is_cuda = True
+
+    monkeypatch.setattr(L._FusedLoRAFunction, "apply", lambda *a: pytest.fail("ran"))
+    x = torch.zeros(4, 64, dtype=torch.bfloat16).as_subclass(OnGpu)
+    w, a, b = (torch.zeros(*s, dtype=torch.bfloat16) for s in ((128, 64), (8, 64), (128, 8)))
+    with pytest.raises((AttributeError, ValueError)):
+        L.fused_linear_lora(x, w, None, b, 1.0)
+    with pytest.raises(ValueError):
+        L.fused_linear_lora(x, w, a, b, 1.0, dropout_p=float("nan"))
+    with pytest.raises(ValueError):
+        L.fused_linear_lora(x, w, a, b, 1.0, dropout_p=1.0)
