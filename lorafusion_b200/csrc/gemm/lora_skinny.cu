@@ -49,6 +49,7 @@ struct Params {
   int b_adapter_rows;          // rows mode: rows of B per adapter
   void* out;
   long long ldo, out_adapter_stride;
+  int out_vec;                 // SEG, not transposed: whether rows of the output are read and written 16 bytes at a time
   const float* adapter_scale;
   float scale;
   const uint32_t* adapter_thresh16;
@@ -302,6 +303,10 @@ lora_skinny_kernel(const Params p, const __grid_constant__ CUtensorMap tmA, cons
                            pack_bf16x2(__uint_as_float(r[g * 8 + 2]) * scale, __uint_as_float(r[g * 8 + 3]) * scale),
                            pack_bf16x2(__uint_as_float(r[g * 8 + 4]) * scale, __uint_as_float(r[g * 8 + 5]) * scale),
                            pack_bf16x2(__uint_as_float(r[g * 8 + 6]) * scale, __uint_as_float(r[g * 8 + 7]) * scale));
+          } else if (!TRANS && !p.out_vec) {
+            float* dst = out_f32 + (long long)row * p.ldo + col0;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) dst[j] = fmaf(scale, __uint_as_float(r[j]), dst[j]);
           } else if (!TRANS) {
             float4* dst = reinterpret_cast<float4*>(out_f32 + (long long)row * p.ldo + col0);
             float4 old[8];
@@ -392,6 +397,12 @@ lora_skinny_kernel(const Params p, const __grid_constant__ CUtensorMap tmA, cons
             w.x = pack_bf16x2(v.x * scale, v.y * scale);
             w.y = pack_bf16x2(v.z * scale, v.w * scale);
             *reinterpret_cast<uint2*>(out_bf16 + (long long)row * p.ldo + col) = w;
+          } else if (!TRANS && !p.out_vec) {
+            float* dst = out_f32 + (long long)row * p.ldo + col;
+            dst[0] = fmaf(scale, v.x, dst[0]);
+            dst[1] = fmaf(scale, v.y, dst[1]);
+            dst[2] = fmaf(scale, v.z, dst[2]);
+            dst[3] = fmaf(scale, v.w, dst[3]);
           } else if (!TRANS) {
             float4* dst = reinterpret_cast<float4*>(out_f32 + (long long)row * p.ldo + col);
             const float4 o = *dst;
@@ -481,8 +492,10 @@ extern "C" int lf_lora_skinny(const LfGemmArgs* a, int split) {
   if (a->a_mn ? (a->epi != LF_EPI_F32_ACCUM || (a->seg_tiles == nullptr && a->num_seg_tiles != 1) || !a->b_mn)
               : (a->epi != LF_EPI_BF16_ADAPTER_SCALE || a->seg_tiles != nullptr))
     return -4;
-  // 16-byte accesses to the output (columns of a row, or 8-byte pieces of it)
-  if (!a->out_transposed && ((reinterpret_cast<uintptr_t>(a->out) & 15) != 0 || a->ldo % 8 != 0)) return -6;
+  // 16-byte accesses to the output (columns of a row, or 8-byte pieces of it); fp32 rows that lie elsewhere are
+  // gone through value by value
+  const bool aligned = (reinterpret_cast<uintptr_t>(a->out) & 15) == 0;
+  if (!a->a_mn && (!aligned || a->ldo % 8 != 0)) return -6;
   CUtensorMap tA, tB;
   int rc = make_tmap_2d_b16(&tA, a->a, a->a_rows, a->a_cols, a->a_ld, a->a_mn ? 64 : BM, 64, true);
   if (rc != 0) return -20 + rc;
@@ -498,6 +511,7 @@ extern "C" int lf_lora_skinny(const LfGemmArgs* a, int split) {
   p.out = a->out;
   p.ldo = a->ldo;
   p.out_adapter_stride = a->out_adapter_stride;
+  p.out_vec = aligned && a->ldo % 4 == 0 && a->out_adapter_stride % 4 == 0;
   p.adapter_scale = a->adapter_scale;
   p.scale = a->scale;
   p.adapter_thresh16 = a->adapter_thresh16;

@@ -452,3 +452,21 @@ def test_multi_lora_of_an_adapter_with_several_segments(p):
     y = fused_linear_multi_lora(xs, w, lora_a_list=[v[0] for v in ab], lora_b_list=frozen[1::2], **short)
     with pytest.raises(ValueError):
         torch.autograd.grad(y, [ab[0][0]], dy[:512])
+
+
+@pytest.mark.parametrize("split", [1, 2, 8])
+@pytest.mark.parametrize("shift", [1, 2, 4])
+def test_db_into_a_buffer_of_any_alignment(split, shift, monkeypatch):
+    """fp32 accumulators that start on any float: the same bits as in an aligned buffer, nothing beside them written."""
+    from lorafusion_b200.ops import lora_kernels as lk
+
+    M, N, R, n = 700, 136, 64, 2
+    monkeypatch.setattr(lk, "reduction_split", lambda *_: split)
+    table = lk.SegmentTable([(1, 0, 384), (0, 384, 700)], torch.device("cuda"), total_rows=M)
+    dy, s = _rand(M, N, seed=1), _rand(M, R, scale=0.1, seed=2)
+    buf = torch.ones(n * N * R + 8, device="cuda")
+    db = buf[shift:shift + n * N * R].view(n, N, R)
+    lk.lora_db(dy, s, table, db)
+    ref = torch.ones(n, N, R, device="cuda")
+    lk.lora_db(dy, s, table, ref)
+    assert torch.equal(db, ref) and (buf[:shift] == 1).all() and (buf[shift + n * N * R:] == 1).all()
