@@ -143,12 +143,13 @@ nf4_absmax_sum_kernel(const float* __restrict__ absmax, long long n, double* __r
 // One warp per group of 256.
 __global__ void __launch_bounds__(256)
 nf4_double_quantize_kernel(const float* __restrict__ absmax, long long n, const double* __restrict__ partial,
-                           const float* __restrict__ mids, uint8_t* __restrict__ q, float* __restrict__ nested,
-                           float* __restrict__ offset) {
+                           const float* __restrict__ mids, const float* __restrict__ code, uint8_t* __restrict__ q,
+                           float* __restrict__ code_out, float* __restrict__ nested, float* __restrict__ offset) {
   __shared__ float s_mid[256];
   __shared__ float s_mean;
   const int lane = threadIdx.x & 31;
   s_mid[threadIdx.x] = threadIdx.x < 255 ? mids[threadIdx.x] : INFINITY;
+  if (blockIdx.x == 0) code_out[threadIdx.x] = code[threadIdx.x];   // every weight has a table of its own
   if (threadIdx.x < 32) {
     double t = 0.0;
     for (int i = lane; i < kMeanParts; i += 32) t += partial[i];
@@ -277,16 +278,16 @@ int lf_nf4_quantize(const void* w, void* packed, float* absmax, long long n_elem
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// absmax: fp32 [n]; partial: double [148] scratch; mids: fp32 [255]; q: uint8 [n]; nested: fp32
-// [ceil(n / 256)]; offset: fp32 [1], the mean that was subtracted.
-int lf_nf4_double_quantize(const float* absmax, long long n, double* partial, const float* mids, void* q,
-                           float* nested, float* offset, void* stream) {
+// absmax: fp32 [n]; partial: double [148] scratch; mids: fp32 [255]; code: fp32 [256]; q: uint8 [n]; code_out:
+// fp32 [256], a copy of code; nested: fp32 [ceil(n / 256)]; offset: fp32 [1], the mean that was subtracted.
+int lf_nf4_double_quantize(const float* absmax, long long n, double* partial, const float* mids, const float* code,
+                           void* q, float* code_out, float* nested, float* offset, void* stream) {
   if (n <= 0) return n == 0 ? 0 : -1;
   cudaStream_t st = (cudaStream_t)stream;
   nf4_absmax_sum_kernel<<<kMeanParts, 256, 0, st>>>(absmax, n, partial);
   const long long groups = (n + 255) / 256;
-  nf4_double_quantize_kernel<<<(unsigned)((groups + 7) / 8), 256, 0, st>>>(absmax, n, partial, mids, (uint8_t*)q,
-                                                                            nested, offset);
+  nf4_double_quantize_kernel<<<(unsigned)((groups + 7) / 8), 256, 0, st>>>(absmax, n, partial, mids, code,
+                                                                            (uint8_t*)q, code_out, nested, offset);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

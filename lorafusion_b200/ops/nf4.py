@@ -8,9 +8,9 @@ the even element in the high nibble; with ``double_quant`` the absmax vector is 
 8-bit indices into a 256-entry code table with one fp32 scale per 256 blocks and a global
 offset (its mean).
 
-The 4-bit quantise/dequantise passes are CUDA kernels (``csrc/nf4/nf4_codec.cu``); the
-second-level quantisation of the small absmax vector runs once at load time with torch ops.
-A pure-PyTorch implementation of both directions is the CPU oracle.
+The 4-bit quantise/dequantise passes and the second-level quantisation of the small absmax
+vector are CUDA kernels (``csrc/nf4/nf4_codec.cu``).  A pure-PyTorch implementation of both
+directions is the CPU oracle.
 """
 
 from __future__ import annotations
@@ -99,7 +99,8 @@ def _nearest_code(x: torch.Tensor, code: torch.Tensor) -> torch.Tensor:
 
 @functools.lru_cache(maxsize=None)
 def _code_table(device: torch.device):
-    """The 256 second-level code values and the 255 midpoints between them, constants of a device."""
+    """The 256 second-level code values and the 255 midpoints between them, constants of a device: weights get
+    copies of the former, nobody writes either."""
     code = dynamic_code_8bit()
     return code.to(device), ((code[:-1] + code[1:]) / 2).to(device)
 
@@ -110,11 +111,12 @@ def _double_quantize(absmax: torch.Tensor):
         n = absmax.numel()
         q = torch.empty(n, dtype=torch.uint8, device=absmax.device)
         nested = torch.empty(-(-n // NESTED_BLOCK), dtype=torch.float32, device=absmax.device)
+        own_code = torch.empty(256, dtype=torch.float32, device=absmax.device)
         scratch = torch.empty(149, dtype=torch.float64, device=absmax.device)   # 148 partial sums, the mean
         mean = scratch[148:].view(torch.float32)[:1]
-        nv.call("lf_nf4_double_quantize", absmax.data_ptr(), n, scratch.data_ptr(), mids.data_ptr(), q.data_ptr(),
-                nested.data_ptr(), mean.data_ptr(), nv.current_stream_ptr())
-        return q, code, nested, float(mean)
+        nv.call("lf_nf4_double_quantize", absmax.data_ptr(), n, scratch.data_ptr(), mids.data_ptr(), code.data_ptr(),
+                q.data_ptr(), own_code.data_ptr(), nested.data_ptr(), mean.data_ptr(), nv.current_stream_ptr())
+        return q, own_code, nested, float(mean)
     code = dynamic_code_8bit().to(absmax.device)
     offset = float(absmax.mean())
     centered = absmax - offset

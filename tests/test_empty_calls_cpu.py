@@ -11,7 +11,7 @@ CALLS = [
     "lf_swiglu_bwd(None, None, None, 4, 0, None)",
     "lf_cross_entropy(None, None, None, 0, 8, 8, 1.0, None)",
     "lf_nf4_quantize(None, None, None, 0, None)",
-    "lf_nf4_double_quantize(None, 0, None, None, None, None, None, None)",
+    "lf_nf4_double_quantize(None, 0, None, None, None, None, None, None, None, None)",
     "lf_nf4_dequantize(None, None, None, None, None, 0.0, None, 0, None)",
 ]
 

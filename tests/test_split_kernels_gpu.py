@@ -470,3 +470,18 @@ def test_db_into_a_buffer_of_any_alignment(split, shift, monkeypatch):
     ref = torch.ones(n, N, R, device="cuda")
     lk.lora_db(dy, s, table, ref)
     assert torch.equal(db, ref) and (buf[:shift] == 1).all() and (buf[shift + n * N * R:] == 1).all()
+
+
+def test_nf4_weights_share_no_code_table():
+    """Writing into the table of one weight leaves the others, and those quantised later, as they are."""
+    from lorafusion_b200.ops import nf4
+
+    w = _rand(64, 512, seed=1)
+    first, second = nf4.quantize_nf4(w), nf4.quantize_nf4(w)
+    want = nf4.dequantize_nf4(second).clone()
+    first.code256.zero_()
+    with torch.inference_mode():
+        third = nf4.quantize_nf4(w)
+    for q in (second, third, nf4.quantize_nf4(w)):
+        assert torch.equal(q.code256.cpu(), nf4.dynamic_code_8bit()) and torch.equal(nf4.dequantize_nf4(q), want)
+    assert not nf4.quantize_nf4(w).code256.is_inference()
