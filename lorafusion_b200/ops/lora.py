@@ -144,17 +144,17 @@ def _unfused_backward(dy, x, saved, wd, stack, info, need_dx):
     return dx
 
 
-def _check_batch(info, rows: int, stacks: Sequence[Optional[torch.Tensor]]) -> None:
-    """The kernels index the adapters of ``stacks`` by the ids of the batch, and its tile table by the rows they are
-    given, without looking at either's length."""
+def _check_batch(info, rows: int, *stacks: Optional[torch.Tensor]) -> None:
+    """The kernels index the adapters of ``stacks`` by the ids of the batch, and its tile table (one entry for 128 padded
+    tokens) by the rows they are given, without looking at either's length."""
     if info.tile_adapter is None:
         return
-    if rows > info.tile_adapter.shape[0] * lk.TILE_M:
+    if rows > info.total_padded_tokens:
         raise ValueError(f"{rows} rows, but the batch describes {info.total_padded_tokens}")
-    n = min(t.shape[0] for t in stacks if t is not None)
-    top = max((a for a, _, _ in info.segments), default=-1)
-    if top >= n:
-        raise ValueError(f"the batch uses adapter {top}, but only {n} are given")
+    n = min([t.shape[0] for t in stacks if t is not None])
+    for adapter, _, _ in info.segments:
+        if adapter >= n:
+            raise ValueError(f"the batch uses adapter {adapter}, but only {n} are given")
 
 
 def lora_linear_forward(x: torch.Tensor, w: Weight, stack: Optional[LoRAStack],
@@ -165,7 +165,7 @@ def lora_linear_forward(x: torch.Tensor, w: Weight, stack: Optional[LoRAStack],
     A precomputed ``s`` (kept from an earlier forward of the same call site) skips the
     down-projection."""
     if stack is not None and info is not None:
-        _check_batch(info, x.shape[0], (stack.a, stack.b))
+        _check_batch(info, x.shape[0], stack.a, stack.b)
     unfused = _UNFUSED and stack is not None and info is not None
     wd = materialize_weight(w, None if unfused else x.shape[0])
     if unfused:
@@ -189,7 +189,7 @@ def lora_linear_backward(dy: torch.Tensor, x: torch.Tensor, s: Optional[torch.Te
                          stream_id: int = 0, need_dx: bool = True, training: bool = True):
     """Accumulates dA/dB into ``stack.da`` / ``stack.db`` and returns ``dX`` (or ``None``)."""
     if stack is not None and info is not None and s is not None:
-        _check_batch(info, dy.shape[0], (stack.a, stack.b, stack.da, stack.db))
+        _check_batch(info, dy.shape[0], stack.a, stack.b, stack.da, stack.db)
     wd = materialize_weight(w, None if isinstance(s, list) else dy.shape[0]) if need_dx else None
     if isinstance(s, list):
         return _unfused_backward(dy, x, s, wd, stack, info, need_dx)

@@ -312,30 +312,36 @@ class OneAdapter:
         return DropoutSpec(seed=self.seed, stream_id=stream_id, p=self.p) if training and self.p > 0 else NO_DROPOUT
 
 
-def _matrix(t: torch.Tensor, name: str, shape: tuple) -> tuple[int, int]:
-    """Address and row pitch of a bf16 matrix of the given shape."""
-    if t.shape != shape:
-        raise ValueError(f"{name} must have the shape {shape}, got {tuple(t.shape)}")
+def _matrix(t: torch.Tensor, name: str, rows: int, cols: int) -> tuple[int, int]:
+    """Address and row pitch of a bf16 matrix ``[rows, cols]``.  (A layer looks at up to eight operands a call: the
+    usual case is one comparison of each property.)"""
+    ptr = t.data_ptr()
+    if t.shape == (rows, cols) and t.dtype is torch.bfloat16:
+        ld, unit = t.stride()
+        if unit == 1 and not (2 * ld | ptr) & 15:
+            return ptr, ld
     check2d(t, name)
-    return t.data_ptr(), t.stride(0)
+    raise ValueError(f"{name} must have the shape {(rows, cols)}, got {tuple(t.shape)}")
 
 
-def _stack(t: torch.Tensor, name: str, shape: tuple) -> torch.Tensor:
-    """``[n, *shape]`` adapters as the bf16 matrix ``[n * shape[0], shape[1]]`` that the kernels read (a copy
-    where they do not lie one behind the other)."""
-    if t.dim() != 3 or t.shape[1:] != shape:
-        raise ValueError(f"{name} must have the shape [n, {shape[0]}, {shape[1]}], got {tuple(t.shape)}")
-    flat = _flat2d(t)
-    check2d(flat, name)
-    return flat
+def _stack(t: torch.Tensor, name: str, rows: int, cols: int) -> tuple[int, int, torch.Tensor]:
+    """Address and row pitch of ``[n, rows, cols]`` adapters as the bf16 matrix ``[n * rows, cols]`` that the kernels
+    read, and the tensor that holds it: a copy where the adapters do not lie one behind the other."""
+    if t.dim() != 3 or t.shape != (t.shape[0], rows, cols):
+        raise ValueError(f"{name} must have the shape [n, {rows}, {cols}], got {tuple(t.shape)}")
+    if not t.is_contiguous() or t.dtype is not torch.bfloat16 or (2 * cols | t.data_ptr()) & 15:
+        t = _flat2d(t)
+        check2d(t, name)
+        return t.data_ptr(), t.stride(0), t
+    return t.data_ptr(), cols, t
 
 
-def _grad_stack(t: Optional[torch.Tensor], name: str, shape: tuple) -> Optional[int]:
-    """Address of the fp32 gradient accumulators ``[n, *shape]`` of all adapters."""
+def _grad_stack(t: Optional[torch.Tensor], name: str, rows: int, cols: int) -> Optional[int]:
+    """Address of the fp32 gradient accumulators ``[n, rows, cols]`` of all adapters."""
     if t is None:
         return None
-    if t.dim() != 3 or t.shape[1:] != shape or t.dtype != torch.float32 or not t.is_contiguous():
-        raise ValueError(f"{name} must be contiguous fp32 [n, {shape[0]}, {shape[1]}], got {t.dtype} {tuple(t.shape)} "
+    if t.dim() != 3 or t.shape != (t.shape[0], rows, cols) or t.dtype is not torch.float32 or not t.is_contiguous():
+        raise ValueError(f"{name} must be contiguous fp32 [n, {rows}, {cols}], got {t.dtype} {tuple(t.shape)} "
                          f"strides {t.stride()}")
     return t.data_ptr()
 
@@ -387,19 +393,21 @@ def linear_fwd(x: torch.Tensor, w: torch.Tensor, a_all: Optional[torch.Tensor], 
     M, K = x.shape
     n, N, R = b_all.shape
     have_s = s is not None
-    x_ptr, x_ld = _matrix(x, "x", (M, K))
-    w_ptr, w_ld = _matrix(w, "w", (N, K))
-    b2d = _stack(b_all, "B", (N, R))
-    fields = dict(x=x_ptr, x_ld=x_ld, w=w_ptr, w_ld=w_ld, b_all=b2d.data_ptr(), b_ld=b2d.stride(0))
-    if not have_s:
-        a2d = _stack(a_all, "A", (R, K))
+    x_ptr, x_ld = _matrix(x, "x", M, K)
+    w_ptr, w_ld = _matrix(w, "w", N, K)
+    b_ptr, b_ld, b_all = _stack(b_all, "B", N, R)
+    a_ptr, a_ld = None, 0
+    if have_s:
+        s_ptr, s_ld = _matrix(s, "S'", M, R)
+    else:
         n = min(n, a_all.shape[0])
-        fields.update(a_all=a2d.data_ptr(), a_ld=a2d.stride(0))
-        s = torch.empty((M, R), dtype=torch.bfloat16, device=x.device)
-    fields["s"], fields["s_ld"] = _matrix(s, "S'", (M, R))
-    y = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
-    args = _linear_args(M, K, N, R, n, info, drop, x.device, y=y.data_ptr(), have_s=int(have_s),
-                        bias=None if bias is None else bias.data_ptr(), split_s=_rows_split(M, K), **fields)
+        a_ptr, a_ld, a_all = _stack(a_all, "A", R, K)
+        s = x.new_empty(M, R)
+        s_ptr, s_ld = s.data_ptr(), R
+    y = x.new_empty(M, N)
+    args = _linear_args(M, K, N, R, n, info, drop, x.device, y=y.data_ptr(), have_s=int(have_s), x=x_ptr, x_ld=x_ld,
+                        w=w_ptr, w_ld=w_ld, a_all=a_ptr, a_ld=a_ld, b_all=b_ptr, b_ld=b_ld, s=s_ptr, s_ld=s_ld,
+                        bias=None if bias is None else bias.data_ptr(), split_s=_rows_split(M, K))
     scratch = _pair_setup(args, M, N, K, args.fwd_max_ctas, x.device)
     nv.note_launch(1 if have_s else 2)
     rc = nv.cuda_lib().lf_lora_linear_fwd(C.byref(args))
@@ -417,24 +425,20 @@ def linear_bwd(dy: torch.Tensor, x: Optional[torch.Tensor], s: Optional[torch.Te
     n, N, R = b_all.shape
     M = dy.shape[0]
     K = w.shape[1] if need_dx else (0 if da is None else x.shape[1])
-    dy_ptr, dy_ld = _matrix(dy, "dy", (M, N))
-    b2d = _stack(b_all, "B", (N, R))
-    fields = dict(dy=dy_ptr, dy_ld=dy_ld, b_all=b2d.data_ptr(), b_ld=b2d.stride(0),
-                  da=_grad_stack(da, "dA", (R, K)), db=_grad_stack(db, "dB", (N, R)))
-    if da is not None:
-        fields["x"], fields["x_ld"] = _matrix(x, "x", (M, K))
-        n = min(n, da.shape[0])
-    if db is not None:
-        fields["s"], fields["s_ld"] = _matrix(s, "S'", (M, R))
-        n = min(n, db.shape[0])
-    ds = torch.empty((M, R), dtype=torch.bfloat16, device=dy.device)
-    dx = None
+    dy_ptr, dy_ld = _matrix(dy, "dy", M, N)
+    b_ptr, b_ld, b_all = _stack(b_all, "B", N, R)
+    da_ptr, db_ptr = _grad_stack(da, "dA", R, K), _grad_stack(db, "dB", N, R)
+    x_ptr, x_ld = (None, 0) if da is None else _matrix(x, "x", M, K)
+    s_ptr, s_ld = (None, 0) if db is None else _matrix(s, "S'", M, R)
+    ds = dy.new_empty(M, R)
+    dx = dx_ptr = w_ptr = a_ptr = None
+    w_ld = a_ld = 0
     if need_dx:
-        fields["w"], fields["w_ld"] = _matrix(w, "w", (N, K))
-        a2d = _stack(a_all, "A", (R, K))
         n = min(n, a_all.shape[0])
-        dx = torch.empty((M, K), dtype=torch.bfloat16, device=dy.device)
-        fields.update(a_all=a2d.data_ptr(), a_ld=a2d.stride(0), dx=dx.data_ptr())
+        w_ptr, w_ld = _matrix(w, "w", N, K)
+        a_ptr, a_ld, a_all = _stack(a_all, "A", R, K)
+        dx = dy.new_empty(M, K)
+        dx_ptr = dx.data_ptr()
     if da is None and db is None:
         seg_rows, num_segs, split_da, split_db = None, 0, 1, 1
     elif info.tile_adapter is None:
@@ -444,8 +448,10 @@ def linear_bwd(dy: torch.Tensor, x: Optional[torch.Tensor], s: Optional[torch.Te
         rows = info.segment_table.device_rows()
         seg_rows, num_segs = rows.data_ptr(), rows.shape[0]
         split_da, split_db = info.segment_table.chunks(K), info.segment_table.chunks(N)
-    args = _linear_args(M, K, N, R, n, info, drop, dy.device, ds=ds.data_ptr(), seg_rows=seg_rows, num_segs=num_segs,
-                        split_ds=_rows_split(M, N), split_db=split_db, split_da=split_da, **fields)
+    args = _linear_args(M, K, N, R, n, info, drop, dy.device, dy=dy_ptr, dy_ld=dy_ld, ds=ds.data_ptr(), x=x_ptr, x_ld=x_ld,
+                        s=s_ptr, s_ld=s_ld, w=w_ptr, w_ld=w_ld, a_all=a_ptr, a_ld=a_ld, b_all=b_ptr, b_ld=b_ld, dx=dx_ptr,
+                        da=da_ptr, db=db_ptr, seg_rows=seg_rows, num_segs=num_segs, split_ds=_rows_split(M, N),
+                        split_db=split_db, split_da=split_da)
     scratch = _pair_setup(args, M, K, N, args.dx_max_ctas, dy.device) if need_dx else None
     nv.note_launch(1 + (da is not None) + (db is not None) + need_dx)
     rc = nv.cuda_lib().lf_lora_linear_bwd(C.byref(args))

@@ -93,7 +93,8 @@ def get_kernel_config(kernel: str, m: int, k: int, n: int) -> KernelConfig:
     """Tuned launch parameters for ``kernel`` on an ``m x k x n`` problem, or the defaults."""
     if kernel not in DEFAULTS:
         raise KeyError(f"unknown kernel {kernel!r}; known: {KERNELS}")
-    return _load().get(entry_key(kernel, m, k, n), DEFAULTS[kernel])
+    table = _load()
+    return table.get(entry_key(kernel, m, k, n), DEFAULTS[kernel]) if table else DEFAULTS[kernel]
 
 
 def write_table(entries: dict, path: Optional[str | Path] = None, gpu: Optional[str] = None) -> Path:
