@@ -58,6 +58,8 @@ typedef struct LfGemmArgs {
 
 // Scratch a product of the CTA-pair kernels wants (0 = none).
 long long lf_gemm_pair_scratch(int M, int N, int K, int max_ctas);
+// Blocks of the main loop that such a product takes a pair, one after the other.
+double lf_gemm_pair_blocks(int M, int N, int K, int max_ctas);
 
 // Returns 0 on success, negative on argument/launch errors.
 int lf_gemm(const LfGemmArgs* args);

@@ -733,12 +733,12 @@ static int launch(const Params& p, const CUtensorMap& tA, const CUtensorMap& tB,
 // stored and read back; slices are at least 8 blocks long.  Measured, us: dX of 300 x 4096 <- 14336
 // (32 tiles of 224 blocks) 78 -> 55; dX of 2048 x 4096 <- 128256 (128 tiles) 1770 -> 1460; with a
 // cost of 8 + 4 s blocks also products that lost were cut: 1000 x 8192 x 8192 107 -> 117.
-static int pick_split(int tiles, int pairs, int nkb) {
+// `saved` (if wanted): the blocks that this saves.
+static int pick_split(int tiles, int pairs, int nkb, double* saved = nullptr) {
   const int tail = tiles % pairs;
-  if (tail == 0) return 1;
   int best = 1;
   double best_gain = 8.0;   // blocks; less is not worth a second look
-  for (int s = 2; s <= 8 && nkb / s >= 8; ++s) {
+  for (int s = 2; tail != 0 && s <= 8 && nkb / s >= 8; ++s) {
     const int waves = (tail * s + pairs - 1) / pairs;
     const double gain = nkb * (1.0 - double(waves) / s) - (30.0 + 0.27 * tail * s);
     if (gain > best_gain) {
@@ -746,6 +746,7 @@ static int pick_split(int tiles, int pairs, int nkb) {
       best = s;
     }
   }
+  if (saved != nullptr) *saved = best > 1 ? best_gain : 0.0;
   return best;
 }
 
@@ -774,6 +775,16 @@ extern "C" long long lf_gemm_pair_scratch(int M, int N, int K, int max_ctas) {
   const int s = pick_split(tiles, pairs, (K + lf::pair::BK - 1) / lf::pair::BK);
   const int tail = tiles % pairs;
   return s > 1 ? arrival_bytes(tail) + (long long)tail * s * kPartialBytes : 0;
+}
+
+// 64-deep blocks of the main loop that a pair walks for such a product, one tile after the other, with
+// what a cut of the last wave costs and saves: what its time goes by.
+extern "C" double lf_gemm_pair_blocks(int M, int N, int K, int max_ctas) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0.0;
+  const int tiles = tile_count(M, N), pairs = pair_count(max_ctas), nkb = (K + lf::pair::BK - 1) / lf::pair::BK;
+  double saved;
+  pick_split(tiles, pairs, nkb, &saved);
+  return double((tiles + pairs - 1) / pairs) * nkb - saved;
 }
 
 // Same argument struct as lf_gemm.  Supported: a / a2 K-major; b and b2 both K-major or both

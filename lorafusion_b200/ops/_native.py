@@ -160,6 +160,8 @@ def _declare_cuda(lib: C.CDLL) -> None:
     lib.lf_lora_skinny.restype = C.c_int
     lib.lf_gemm_pair_scratch.argtypes = [C.c_int] * 4
     lib.lf_gemm_pair_scratch.restype = C.c_longlong
+    lib.lf_gemm_pair_blocks.argtypes = [C.c_int] * 4
+    lib.lf_gemm_pair_blocks.restype = C.c_double
     lib.lf_gemm_nf4.argtypes = [C.POINTER(LfGemmArgs), C.POINTER(LfNf4Args)]
     lib.lf_gemm_nf4.restype = C.c_int
     for name, sig in _SIGNATURES.items():

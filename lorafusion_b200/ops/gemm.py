@@ -148,17 +148,17 @@ def set_pair_kernels(enabled: bool) -> None:
 
 @functools.lru_cache(maxsize=4096)
 def _pair_is_faster(M: int, N: int, K: int, max_ctas: int, device: int) -> bool:
-    """Which kernel takes a product of fewer than ``_PAIR_MIN_ROWS`` rows with 256-wide tiles.  Both
-    walk the reduction in 64-deep blocks, the single-CTA one in 0.44 us a block (it loads a whole
-    B tile per SM), a pair in 0.37 us, but over half as many, twice as high tiles at a time and with
-    3 us more around them; a last wave cut along the reduction is the pairs' alone."""
-    if _pair_scratch_bytes(M, N, K, max_ctas, device):
-        return True
+    """Which kernel takes a product of fewer than ``_PAIR_MIN_ROWS`` rows with 256-wide tiles.  Both walk the
+    reduction in 64-deep blocks: an SM alone takes the less for one and starts sooner, a pair reads the weight
+    faster (SMs that read it: twice as many) and does with fewer waves, or a last one that is cut, where tiles are
+    many.  The figures are fitted to 340 products of 64 to 511 rows, forward and dX; us alone / in pairs: 128 x 19456
+    x 4096 43 / 58, 128 x 22016 x 8192 72 / 86, 384 x 10240 x 8192 61 / 74, 128 x 4096 x 4096 24.2 / 25.9; 128 x 14336
+    x 4096 36.4 / 32.4, 257 x 8192 x 8192 57 / 48, 511 x 8192 x 28672 194 / 175.  What the rule gets wrong costs 1.5 us
+    at most in a single wave (forward, 385 x 7168 x 5120 32.3 / 34.8) and 0.1 % on average."""
     sms = 148 if max_ctas <= 0 else min(148, max_ctas)
-    n_tiles, blocks = -(-N // 256), -(-K // 64)
-    single = -(-(-(-M // 128) * n_tiles) // sms) * blocks * 0.44
-    pairs = -(-(-(-M // 256) * n_tiles) // max(1, sms // 2)) * blocks * 0.37
-    return pairs + 3.0 < single
+    waves = -(-(-(-M // 128) * -(-N // 256)) // sms)
+    weight_mb = N * K * 2e-6
+    return 0.30 * nv.cuda_lib().lf_gemm_pair_blocks(M, N, K, max_ctas) + 2.0 < 0.28 * waves * -(-K // 64) + 0.06 * weight_mb
 
 
 def use_pair(M: int, N: int, K: int, max_ctas: int, device: torch.device) -> bool:

@@ -80,3 +80,27 @@ def test_frozen_adapters_may_have_several_segments(monkeypatch):
     stack = L.LoRAStack(z(1, 64, 128), z(1, 128, 64))
     L.lora_linear_backward(z(256, 128), z(256, 128), z(256, 64), z(128, 128), stack, info)
     assert seen == ["lora_ds", "base_lora_dx"]
+
+
+@pytest.mark.parametrize("M,N,K,pairs", [
+    # measured, alone against in pairs: 43 / 58, 48 / 63, 72 / 86, 61 / 74, 165 / 185, 24.2 / 25.9, 8.5 / 9.9 us
+    (128, 19456, 4096, False), (100, 21504, 5120, False), (100, 22016, 8192, False), (384, 10240, 8192, False),
+    (128, 57344, 8192, False), (128, 4096, 4096, False), (257, 512, 512, False),
+    # 36.4 / 32.4, 57 / 48, 194 / 175, 62 / 50, 78 / 55 (cut), 85 / 71 us
+    (128, 14336, 4096, True), (257, 8192, 8192, True), (511, 8192, 28672, True), (128, 10240, 8192, True),
+    (300, 4096, 14336, True), (511, 19456, 4096, True),
+])
+def test_which_kernel_takes_a_product_of_few_rows(M, N, K, pairs):
+    from lorafusion_b200.ops import gemm
+
+    assert gemm._pair_is_faster(M, N, K, 0, 0) == pairs
+
+
+def test_blocks_of_a_pair_count_waves_and_the_cut():
+    from lorafusion_b200.ops import _native as nv
+
+    blocks = nv.cuda_lib().lf_gemm_pair_blocks
+    assert blocks(256 * 74, 256, 8192, 0) == 128 and blocks(256 * 75, 256, 640, 0) == 20    # one and two waves
+    # 54 of 74 pairs busy with 2004 blocks in the second wave, cut in four: 3 / 4 of it, 30 + 0.27 * 54 * 4 on top
+    assert blocks(2048, 4096, 128256, 0) == pytest.approx(2004 + 2004 * 0.75 + 30 + 0.27 * 216)
+    assert blocks(0, 256, 256, 0) == 0
