@@ -93,7 +93,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // time limit are looked at every 256 polls, 5 ms.  Under the large products, at the power cap, ten warps
 // of every CTA wait for most of a main loop, and sleeping instead of polling at the default rate is worth
 // 1 to 5 % (a layer of 8192 x 4096 x 4096: 582 -> 555 us).  In the attention kernels the waits are short
-// and on the critical path, and the same hint cost 2 to 4 % (8192 tokens: 2109 -> 2152 us): they poll.
+// and on the critical path, and the same hint cost 2 to 4 % (8192 tokens: 2109 -> 2152 us): they poll.  So
+// do the tensor-parallel products, whose waits for peers the hint has not been measured with.
 constexpr uint32_t kSuspendHintNs = 20000;
 
 template <bool SLEEP = true>

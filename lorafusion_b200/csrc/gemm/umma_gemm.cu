@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(192 + (NF4B ? 32 * kNumExpandWarps : 0) +
         for (int kb = 0; kb < total; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&empty[s], ph ^ 1, ctx, ERR_WAIT_EMPTY)) {
+          if (!mbar_wait<TP == 0>(&empty[s], ph ^ 1, ctx, ERR_WAIT_EMPTY)) {
             ok = false;
             break;
           }
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(192 + (NF4B ? 32 * kNumExpandWarps : 0) +
         const int total = nkb + nkb2;
         const int buf = tile_iter % NBUF;
         const uint32_t bph = (tile_iter / NBUF) & 1;
-        if (!mbar_wait(&tempty[buf], bph ^ 1, ctx, ERR_WAIT_TMEM_EMPTY)) {
+        if (!mbar_wait<TP == 0>(&tempty[buf], bph ^ 1, ctx, ERR_WAIT_TMEM_EMPTY)) {
           ok = false;
           break;
         }
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(192 + (NF4B ? 32 * kNumExpandWarps : 0) +
         for (int kb = 0; kb < total; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(NF4B ? &ready[s] : &full[s], ph, ctx,
+          if (!mbar_wait<TP == 0>(NF4B ? &ready[s] : &full[s], ph, ctx,
                          NF4B ? ERR_WAIT_READY : ERR_WAIT_FULL)) {
             ok = false;
             break;
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(192 + (NF4B ? 32 * kNumExpandWarps : 0) +
       const bool has_slab = nkb2 > 0;
       const int buf = tile_iter % NBUF;
       const uint32_t bph = (tile_iter / NBUF) & 1;
-      bool got = mbar_wait(&tfull[buf], bph, ctx, ERR_WAIT_TMEM_FULL);
+      bool got = mbar_wait<TP == 0>(&tfull[buf], bph, ctx, ERR_WAIT_TMEM_FULL);
       // The reduce-scatter epilogue ends in a named barrier of its 128 threads: they must all
       // take the same branch here, or one that saw an abort earlier would leave the others
       // waiting for its arrival.
@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(192 + (NF4B ? 32 * kNumExpandWarps : 0) +
             scale = __ldg(p.nf4_scales + wrow * p.nf4_blocks_per_row + wblk);
         }
         // one answer per warp: its lanes meet again in __syncwarp below
-        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, ctx, ERR_WAIT_FULL))) {
+        if (!__all_sync(0xffffffffu, mbar_wait<TP == 0>(&full[s], ph, ctx, ERR_WAIT_FULL))) {
           ok = false;
           break;
         }

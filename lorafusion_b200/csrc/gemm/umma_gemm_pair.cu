@@ -214,7 +214,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
       auto load_block = [&](const Tile& t, const int (&ad)[2], int kb, int slab_idx) -> bool {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1;
-        if (!mbar_wait(&empty[s], ph ^ 1, ctx, ERR_WAIT_EMPTY)) return false;
+        if (!mbar_wait<TP == 0>(&empty[s], ph ^ 1, ctx, ERR_WAIT_EMPTY)) return false;
         ++it;
         const int m0 = (2 * t.pm + int(cta)) * BM;
         const int n0 = t.n_tile * BN + int(cta) * BNH;
@@ -309,7 +309,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
       auto issue_block = [&](uint32_t d, bool fresh) -> bool {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1;
-        if (!mbar_wait(&full[s], ph, ctx, ERR_WAIT_FULL)) return false;
+        if (!mbar_wait<TP == 0>(&full[s], ph, ctx, ERR_WAIT_FULL)) return false;
         ++it;
         tc_fence_after_sync();
         const uint32_t sA = smem_u32(smem + s * STAGE_BYTES);
@@ -344,7 +344,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
       bool more = get_unit(p, pair_id, num_pairs, 0, w);
       if (SLAB_FIRST && more) {
         const Tile t = decode(p, w.tile);
-        ok = mbar_wait(&tempty[0], 1, ctx, ERR_WAIT_TMEM_EMPTY);   // fresh barrier: passes at once
+        ok = mbar_wait<TP == 0>(&tempty[0], 1, ctx, ERR_WAIT_TMEM_EMPTY);   // fresh barrier: passes at once
         if (ok && has_slab(w)) {
           tc_fence_after_sync();
           ok = issue_slabs(t, tmem_base);
@@ -365,9 +365,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
         if (SLAB_FIRST) {
           int ad[2];
           opens = !has_slab(w) || slab_passes(t, ad) * p.nkb2 == 0;
-          ok = mbar_wait(&masked[buf], bph, ctx, ERR_WAIT_READY);
+          ok = mbar_wait<TP == 0>(&masked[buf], bph, ctx, ERR_WAIT_READY);
         } else {
-          ok = mbar_wait(&tempty[buf], bph ^ 1, ctx, ERR_WAIT_TMEM_EMPTY);
+          ok = mbar_wait<TP == 0>(&tempty[buf], bph ^ 1, ctx, ERR_WAIT_TMEM_EMPTY);
         }
         if (!ok) break;
         tc_fence_after_sync();
@@ -377,7 +377,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
             const Tile tn = decode(p, wn.tile);
             const int nbuf = (u + 1) % NBUF;
             const uint32_t nph = ((u + 1) / NBUF) & 1;
-            ok = mbar_wait(&tempty[nbuf], nph ^ 1, ctx, ERR_WAIT_TMEM_EMPTY);
+            ok = mbar_wait<TP == 0>(&tempty[nbuf], nph ^ 1, ctx, ERR_WAIT_TMEM_EMPTY);
             if (ok && has_slab(wn)) {
               tc_fence_after_sync();
               ok = issue_slabs(tn, tmem_base + uint32_t(nbuf * BN));
@@ -414,7 +414,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
       const Tile t = decode(p, w.tile);
       const int buf = iter % NBUF;
       // warp-uniform: the tcgen05.ld/st below are .sync.aligned, and the warp reports in as one
-      bool got = __all_sync(0xffffffffu, mbar_wait(&sfull[buf], uint32_t(iter / NBUF) & 1, ctx, ERR_WAIT_TMEM_FULL));
+      bool got = __all_sync(0xffffffffu, mbar_wait<TP == 0>(&sfull[buf], uint32_t(iter / NBUF) & 1, ctx, ERR_WAIT_TMEM_FULL));
       // the reduce-scatter epilogue meets in named barriers: one answer for all 256 threads
       if (TP == 2) got = named_bar_and<1, 32 * PAIR_EPI_WARPS>(got);
       if (!got) return false;
@@ -507,7 +507,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + (TP !
       }
       const int buf = u % NBUF;
       const uint32_t bph = (u / NBUF) & 1;
-      bool got = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], bph, ctx, ERR_WAIT_TMEM_FULL));
+      bool got = __all_sync(0xffffffffu, mbar_wait<TP == 0>(&tfull[buf], bph, ctx, ERR_WAIT_TMEM_FULL));
       // the reduce-scatter epilogue ends in a named barrier of its 256 threads: one answer for all
       if (TP == 2) got = named_bar_and<1, 32 * PAIR_EPI_WARPS>(got);
       if (!got) {
