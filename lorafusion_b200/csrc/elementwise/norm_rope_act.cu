@@ -192,11 +192,11 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 // QKV activation [M, (Hq + 2 Hkv) * D].  cos/sin come from a table [max_pos, D/2] gathered
 // by position id.  `sign` = +1 forward, -1 backward (the transpose of a rotation).
 // ---------------------------------------------------------------------------------
-// One CTA per token, or as many tokens as fill it where there are few heads; threadIdx.x = 16-byte vector
+// One CTA per token, or several where there are few heads and many tokens; threadIdx.x = 16-byte vector
 // of a half head, threadIdx.y = head, threadIdx.z = token.  A thread keeps its piece of the cos / sin row
 // for all the heads it rotates, two at a time and as many as every other thread (lf_rope_inplace), and
 // the first heads are on their way before the position that selects the row is known.  16384 tokens of 1,
-// 40 and 72 heads of 128: 6.2, 66, 105 us; 6.8, 74, 126 with a flat index over all vectors, two
+// 40 and 72 heads of 128: 5.7, 66, 105 us; 6.7, 74, 126 with a flat index over all vectors, two
 // 64-bit divisions and a cos / sin load each; 11, 75, 118 with one token a CTA and 32 heads at a time,
 // where a quarter of the threads rotated two of 40 heads and the others one.
 constexpr int ROPE_THREADS = 256;
@@ -360,6 +360,13 @@ static inline int grid_for(long long total, int threads) {
 }
 
 
+// How many of M short rows share a CTA: at most `most` (and 64), and so that two CTAs an SM remain.
+static inline int rows_per_cta(long long M, int most) {
+  int n = most < 64 ? most : 64;
+  while (n > 1 && (M + n - 1) / n < 2 * 148) n /= 2;
+  return n < 1 ? 1 : n;
+}
+
 }  // namespace lf
 
 using namespace lf;
@@ -414,8 +421,7 @@ int lf_rope_inplace(void* qkv, const int* pos, const float* cos_t, const float* 
   } else {
     by = n_rot_heads;
   }
-  int bz = ROPE_THREADS / (bx * by);
-  if (bz > 64) bz = 64;   // the most a block may have in z
+  const int bz = rows_per_cta(M, 128 / (bx * by));   // (z has room for 64)
   rope_inplace_kernel<<<((unsigned)M + bz - 1) / bz, dim3(bx, by, bz), 0, (cudaStream_t)stream>>>(
       (__nv_bfloat16*)qkv, pos, cos_t, sin_t, M, n_rot_heads, D, row_stride, backward ? -1.f : 1.f);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -433,7 +439,7 @@ int lf_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long M, int 
   if (I % 8 != 0) return -1;
   if (M == 0 || I == 0) return 0;
   const int vec = I / 8, half = (vec + SWIGLU_VECS - 1) / SWIGLU_VECS;
-  const int bx = half < SWIGLU_THREADS ? half : SWIGLU_THREADS, by = SWIGLU_THREADS / bx;
+  const int bx = half < SWIGLU_THREADS ? half : SWIGLU_THREADS, by = rows_per_cta(M, SWIGLU_THREADS / bx);
   const int pieces = (half + bx - 1) / bx;
   swiglu_bwd_kernel<<<(unsigned)((M + by - 1) / by * pieces), dim3(bx, by), 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)dout, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, M, I, pieces);

@@ -242,7 +242,8 @@ def test_one_call_layer_of_several_adapters_equals_its_building_blocks(K, N, ps)
     info = prepare_multi_lora_batch_info([100, 128, 128, 200], [1, -1, 0, 2], [16, 0, 16, 16],
                                          [ps[1], 0.0, ps[0], ps[2]], [2.0, 0.0, 0.5, 1.0], device="cuda", seed=(3 << 32) | 5)
     assert info.total_padded_tokens == M
-    assert (_pair_scratch_bytes(M, N, K, 0, 0) > 0) == (K == 5000) and (_pair_scratch_bytes(M, K, N, 0, 0) > 0) == (N == 5000)
+    assert (_pair_scratch_bytes(M, N, K, 0, 0) > 0) == (K == 5000)
+    assert (_pair_scratch_bytes(M, K, N, 0, 0) > 0) == (N == 5000)
     drop = replace(info.dropout_spec(5), row_offset=256, col_offset=512)
     x, dy, w = _rand(M, K, seed=1), _rand(M, N, seed=2), _rand(N, K, scale=0.05, seed=3)
     a, b = _rand(n, 2 * R, K, scale=0.05, seed=5)[:, R:], _rand(n, N, R + 64, scale=0.05, seed=6)[:, :, 64:]
@@ -316,8 +317,8 @@ def test_cross_entropy_stays_inside_its_row(V):
             assert torch.equal(alone[0], buf[i]), label
 
 
-@pytest.mark.parametrize("M,heads,D", [(1, 1, 128), (129, 1, 16), (67, 1, 128), (100, 5, 128), (33, 40, 128), (7, 3, 256),
-                                       (65, 2, 64)])
+@pytest.mark.parametrize("M,heads,D", [(1, 1, 128), (19001, 1, 16), (4777, 1, 128), (1201, 5, 128), (33, 40, 128),
+                                       (599, 2, 64), (7, 3, 256), (65, 2, 64)])
 def test_rope_with_several_tokens_a_block(M, heads, D):
     """Token counts that leave the last block ragged; the heads behind the rotated ones and the rows behind the batch
     stay as they were."""
@@ -336,9 +337,11 @@ def test_rope_with_several_tokens_a_block(M, heads, D):
     assert torch.equal(qkv[:M, heads * D:], before[:M, heads * D:]) and torch.equal(qkv[M:], before[M:])
 
 
-@pytest.mark.parametrize("M,I", [(1, 8), (300, 8), (65, 24), (257, 64), (100, 1000), (33, 2056), (3, 4104), (5, 8200)])
+@pytest.mark.parametrize("M,I", [(1, 8), (300, 8), (19001, 8), (9001, 24), (2501, 64), (1187, 1000), (33, 2056), (3, 4104),
+                                 (5, 8200)])
 def test_swiglu_backward_of_short_and_long_rows(M, I):
-    """Rows that share a CTA, one row a CTA (2056 to 4096) and rows in pieces; ragged last CTAs and odd vector counts."""
+    """Several rows a CTA (long batches of short rows), one row a CTA and rows in pieces; ragged last CTAs and odd vector
+    counts."""
     from lorafusion_b200.ops import elementwise as ew
 
     gu, d = _rand(M, 2 * I, seed=1), _rand(M, I, seed=2)
@@ -362,7 +365,8 @@ def test_adam_regions_of_any_size(rows, ld, col0, cols):
     want = [t[st:st + rows * cols].clone() for t in (mas, m, v)]
     before = [t.clone() for t in (grad, mas, m, v)]
     table = torch.tensor([[off, rows, ld, col0, cols, st]], dtype=torch.int64, device="cuda")
-    ew.adam_chunks(table, grad, mas, m, v, work, lr=0.01, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=1, grad_scale=0.5)
+    ew.adam_chunks(table, grad, mas, m, v, work, lr=0.01, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=1,
+                   grad_scale=0.5)
     g = 0.5 * before[0][off:off + n].view(rows, ld)[:, col0:col0 + cols].reshape(-1)
     want[1] = 0.9 * want[1] + 0.1 * g
     want[2] = 0.95 * want[2] + 0.05 * g * g
