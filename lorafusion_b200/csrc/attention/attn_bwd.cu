@@ -420,7 +420,7 @@ attn_dkdv_kernel(const AttnBwdParams p, const __grid_constant__ CUtensorMap tmQK
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   AbortCtx ctx{p.err, abort_flag};
-  const int4 tile = p.tiles[p.num_tiles - 1 - blockIdx.x / p.Hkv];   // first key tiles first: they see the most queries
+  const int4 tile = p.tiles[p.num_tiles - 1 - blockIdx.x / p.Hkv];   // a sequence's first key tiles first: they see the most queries
   const int row0 = tile.x, rows = tile.y, seq_row0 = tile.z, seq_rows = tile.w;
   const int g = blockIdx.x % p.Hkv;
   const int group = p.Hq / p.Hkv;
@@ -687,7 +687,9 @@ extern "C" int lf_attn_bwd(const void* qkv, const void* out, const void* d_out, 
   p.scale_log2e = scale * 1.4426950408889634f;
   p.err = err;
   // KV heads vary fastest, so that a launch starts with its longest CTAs (the tile list starts with the
-  // longest key ranges): with the tiles fastest the long tiles of the last heads started last.
+  // longest key ranges): with the tiles fastest the long tiles of the last heads started last.  dK/dV
+  // walks the list from its other end, which is longest first within a sequence, but not over sequences
+  // of different lengths: a short one's first key tile comes before a long one's second.
   // One CTA walks all query heads of a group, which pays for its set-up once, unless the launch
   // would leave SMs idle: then the heads of a group go to several CTAs.
   const int group = Hq / Hkv;

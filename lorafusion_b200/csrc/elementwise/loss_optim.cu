@@ -197,8 +197,8 @@ __device__ __forceinline__ void adam_one(float g, float& w, float& mi, float& vi
   w -= h.lr * (mi * inv_c1) / (sqrtf(vi) * inv_sqrt_c2 + h.eps);
 }
 
-// One CTA per work item {chunk, first element, element count}: regions differ in size by two
-// orders of magnitude (a 16 x 8192 A block next to a 57344 x 64 B block), so the host cuts
+// A work item {chunk, first element, element count} is what kAdamShares CTAs share: regions differ in
+// size by two orders of magnitude (a 16 x 8192 A block next to a 57344 x 64 B block), so the host cuts
 // them into equal pieces instead of giving every region the same number of CTAs.  Regions
 // whose offsets and sizes are all multiples of four elements (every region the adapter arenas
 // produce) go through 16-byte accesses with 32-bit index arithmetic; anything else takes the
@@ -208,7 +208,6 @@ struct AdamWorkItem {
   unsigned first, count;  // elements; multiples of 4 inside vectorisable regions
 };
 
-//
 // Bound by latency unless every load of a thread is issued before its first use: an item is shared by
 // kAdamShares neighbouring CTAs, and a thread loads gradient, weight and moments of its two pieces
 // first (padding is not read at all).  The 86 MB of a two-layer 8B adapter take 34 us (2.5 TB/s); one

@@ -272,9 +272,10 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
 }
 
 // dgu[M, 2I] from dout[M, I] and the saved gu.  One CTA per piece of a row, the pieces of a row side by
-// side: one small division a CTA and all loads of two vectors in flight a thread, 421 -> 330 us for
-// 16384 x 14336 (a flat index over all vectors takes two 64-bit divisions each).  The forward kernel,
-// which has a third fewer loads to wait for, is the faster one with the flat index: 243 against 286.
+// side: one small division a CTA and all loads of two vectors in flight a thread, 190 -> 172 us for
+// 8192 x 14336 (a flat index over all vectors takes two 64-bit divisions each).  The forward kernel,
+// which has a third fewer loads to wait for, is the faster one with the flat index: 243 against 286 for
+// 16384 x 14336.
 // Rows too short for a CTA share one (threadIdx.y = row): 8192 x 64 took 3.5 us with the flat index, 8.7
 // with eight threads of a CTA at work, 4.2 so (8192 x 256: 5.6, 9.0, 5.0).
 constexpr int SWIGLU_THREADS = 256;

@@ -91,7 +91,7 @@ def cross_entropy_inplace(logits: torch.Tensor, labels: torch.Tensor, grad_scale
     return loss_out
 
 
-ADAM_WORK_UNIT = 32768  # elements per CTA (a multiple of 4)
+ADAM_WORK_UNIT = 32768  # elements per work item, which sixteen CTAs share (a multiple of 4)
 
 
 def dp_slice(total: int, rank: int, world: int) -> tuple[int, int]:

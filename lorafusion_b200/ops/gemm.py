@@ -157,8 +157,8 @@ def _pair_is_faster(M: int, N: int, K: int, max_ctas: int, device: int) -> bool:
     at most in a single wave (forward, 385 x 7168 x 5120 32.3 / 34.8) and 0.1 % on average."""
     sms = 148 if max_ctas <= 0 else min(148, max_ctas)
     waves = -(-(-(-M // 128) * -(-N // 256)) // sms)
-    weight_mb = N * K * 2e-6
-    return 0.30 * nv.cuda_lib().lf_gemm_pair_blocks(M, N, K, max_ctas) + 2.0 < 0.28 * waves * -(-K // 64) + 0.06 * weight_mb
+    alone = 0.28 * waves * -(-K // 64) + 0.06 * N * K * 2e-6   # (both short of what they share, in us)
+    return 0.30 * nv.cuda_lib().lf_gemm_pair_blocks(M, N, K, max_ctas) + 2.0 < alone
 
 
 def use_pair(M: int, N: int, K: int, max_ctas: int, device: torch.device) -> bool:

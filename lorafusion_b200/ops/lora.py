@@ -145,8 +145,8 @@ def _unfused_backward(dy, x, saved, wd, stack, info, need_dx):
 
 
 def _check_batch(info, rows: int, *stacks: Optional[torch.Tensor]) -> None:
-    """The kernels index the adapters of ``stacks`` by the ids of the batch, and its tile table (one entry for 128 padded
-    tokens) by the rows they are given, without looking at either's length."""
+    """The kernels index the adapters of ``stacks`` by the ids of the batch, and its tile table (one entry for 128
+    padded tokens) by the rows they are given, without looking at either's length."""
     if info.tile_adapter is None:
         return
     if rows > info.total_padded_tokens:
@@ -197,7 +197,8 @@ def lora_linear_backward(dy: torch.Tensor, x: torch.Tensor, s: Optional[torch.Te
         return lk.base_lora_dx(dy, wd, None, None, tile_adapter=None) if need_dx else None
     drop = info.dropout_spec(stream_id, training)
     if not isinstance(wd, NF4Weight) and (info.tile_adapter is None or not info.segment_table.repeats):
-        return lk.linear_bwd(dy, x, s, wd if need_dx else None, stack.a, stack.b, info, drop, stack.da, stack.db, need_dx)
+        return lk.linear_bwd(dy, x, s, wd if need_dx else None, stack.a, stack.b, info, drop, stack.da, stack.db,
+                             need_dx)
     ds = lk.lora_ds(dy, stack.b, tile_adapter=info.tile_adapter, adapter_scale=info.adapter_scale,
                     scale=getattr(info, "scale", 1.0))
     segs = info.segment_table if info.tile_adapter is not None else \

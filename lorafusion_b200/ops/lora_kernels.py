@@ -161,13 +161,6 @@ class SegmentTable:
             raise ValueError("an adapter may own only one token segment per microbatch")
         return list(self._rows().split(self._passes()))
 
-    def split_plan(self, features: int):
-        """``(chunks per segment, owner)`` when the tokens of every segment are summed in several
-        chunks, whose partial results are added in token order, or ``None`` when each (segment,
-        128-feature tile) is one chunk.  ``owner[chunk]`` = the adapter of each segment's chunks."""
-        chunks = self.chunks(features)
-        return None if chunks == 1 else (chunks, [r[0] for r in segment_rows(self.segments) for _ in range(chunks)])
-
     def chunks(self, features: int) -> int:
         """In how many chunks the tokens of a segment are summed."""
         c = self._cache.get(features)
@@ -346,7 +339,8 @@ def _grad_stack(t: Optional[torch.Tensor], name: str, rows: int, cols: int) -> O
     return t.data_ptr()
 
 
-def _linear_args(M: int, K: int, N: int, R: int, n: int, info, drop: DropoutSpec, device, **fields) -> nv.LfLoraLinearArgs:
+def _linear_args(M: int, K: int, N: int, R: int, n: int, info, drop: DropoutSpec, device,
+                 **fields) -> nv.LfLoraLinearArgs:
     """Describe one LoRA linear layer (``lf_lora_linear_fwd`` / ``_bwd``) for the current stream.  The operands come as
     addresses: the callers have checked them, since the kernels read and write what the sizes say."""
     if R not in RANK_PADS and not fields.get("have_s"):
@@ -389,7 +383,7 @@ def _pair_setup(args: nv.LfLoraLinearArgs, M: int, N: int, K: int, max_ctas: int
 
 def linear_fwd(x: torch.Tensor, w: torch.Tensor, a_all: Optional[torch.Tensor], b_all: torch.Tensor, info,
                drop: DropoutSpec, bias: Optional[torch.Tensor] = None, s: Optional[torch.Tensor] = None):
-    """``lora_down`` (unless ``s`` is given: then ``a_all`` is not read) and ``base_lora_fwd`` in one call: ``(y, s)``."""
+    """``lora_down`` and ``base_lora_fwd`` in one call: ``(y, s)``.  With ``s`` given, ``a_all`` is not read."""
     M, K = x.shape
     n, N, R = b_all.shape
     have_s = s is not None
@@ -420,8 +414,8 @@ def linear_fwd(x: torch.Tensor, w: torch.Tensor, a_all: Optional[torch.Tensor], 
 def linear_bwd(dy: torch.Tensor, x: Optional[torch.Tensor], s: Optional[torch.Tensor], w: Optional[torch.Tensor],
                a_all: Optional[torch.Tensor], b_all: torch.Tensor, info, drop: DropoutSpec, da: Optional[torch.Tensor],
                db: Optional[torch.Tensor], need_dx: bool) -> Optional[torch.Tensor]:
-    """``lora_ds``, ``lora_db`` into ``db``, ``lora_da`` into ``da`` and ``base_lora_dx`` in one call.  ``x`` is read for
-    ``da``, ``s`` for ``db``, ``w`` and ``a_all`` for dX."""
+    """``lora_ds``, ``lora_db`` into ``db``, ``lora_da`` into ``da`` and ``base_lora_dx`` in one call.  ``x`` is read
+    for ``da``, ``s`` for ``db``, ``w`` and ``a_all`` for dX."""
     n, N, R = b_all.shape
     M = dy.shape[0]
     K = w.shape[1] if need_dx else (0 if da is None else x.shape[1])
@@ -448,10 +442,10 @@ def linear_bwd(dy: torch.Tensor, x: Optional[torch.Tensor], s: Optional[torch.Te
         rows = info.segment_table.device_rows()
         seg_rows, num_segs = rows.data_ptr(), rows.shape[0]
         split_da, split_db = info.segment_table.chunks(K), info.segment_table.chunks(N)
-    args = _linear_args(M, K, N, R, n, info, drop, dy.device, dy=dy_ptr, dy_ld=dy_ld, ds=ds.data_ptr(), x=x_ptr, x_ld=x_ld,
-                        s=s_ptr, s_ld=s_ld, w=w_ptr, w_ld=w_ld, a_all=a_ptr, a_ld=a_ld, b_all=b_ptr, b_ld=b_ld, dx=dx_ptr,
-                        da=da_ptr, db=db_ptr, seg_rows=seg_rows, num_segs=num_segs, split_ds=_rows_split(M, N),
-                        split_db=split_db, split_da=split_da)
+    args = _linear_args(M, K, N, R, n, info, drop, dy.device, dy=dy_ptr, dy_ld=dy_ld, ds=ds.data_ptr(), x=x_ptr,
+                        x_ld=x_ld, s=s_ptr, s_ld=s_ld, w=w_ptr, w_ld=w_ld, a_all=a_ptr, a_ld=a_ld, b_all=b_ptr,
+                        b_ld=b_ld, dx=dx_ptr, da=da_ptr, db=db_ptr, seg_rows=seg_rows, num_segs=num_segs,
+                        split_ds=_rows_split(M, N), split_db=split_db, split_da=split_da)
     scratch = _pair_setup(args, M, K, N, args.dx_max_ctas, dy.device) if need_dx else None
     nv.note_launch(1 + (da is not None) + (db is not None) + need_dx)
     rc = nv.cuda_lib().lf_lora_linear_bwd(C.byref(args))

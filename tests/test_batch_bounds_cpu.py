@@ -71,7 +71,8 @@ def test_backward_alone_is_checked_too(launched):
 @pytest.mark.gpu
 def test_fused_multi_lora_refuses_before_it_launches():
     z = lambda *s: torch.zeros(*s, dtype=torch.bfloat16, device="cuda")  # noqa: E731
-    info = prepare_multi_lora_batch_info([100, 200], [0, 2], [8, 8], [0.0, 0.0], [1.0, 1.0], device="cuda", num_adapters=3)
+    info = prepare_multi_lora_batch_info([100, 200], [0, 2], [8, 8], [0.0, 0.0], [1.0, 1.0], device="cuda",
+                                         num_adapters=3)
     ab = dict(lora_a_list=[z(8, K)] * 3, lora_b_list=[z(N, 8)] * 3, batch_info=info)
     with pytest.raises(ValueError, match="adapter"):
         L.fused_linear_multi_lora(z(384, K), z(N, K), **dict(ab, lora_b_list=[z(N, 8)] * 2))

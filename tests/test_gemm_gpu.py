@@ -124,9 +124,9 @@ def test_lora_linear_blocks(p):
 
 @pytest.mark.parametrize("mixed_p", [False, True])
 def test_gradient_kernels_split_long_segments_into_chunks(mixed_p):
-    """Two long segments and few feature tiles: the work list is cut into token chunks that write
-    partial sums, folded in a fixed order.  Same results as fp32 math, and bitwise the same from
-    run to run."""
+    """Two long segments and few feature tiles: the tokens of a segment are summed in chunks by several
+    CTAs, whose partial sums are added in a fixed order.  Same results as fp32 math, and bitwise the
+    same from run to run."""
     from lorafusion_b200.ops import lora_kernels as lk
     from lorafusion_b200.ops.philox import keep_mask
 
@@ -136,8 +136,7 @@ def test_gradient_kernels_split_long_segments_into_chunks(mixed_p):
     x, dy = _rand(M, K, seed=40), _rand(M, N, seed=41)
     s, ds = _rand(M, R, scale=0.1, seed=42), _rand(M, R, scale=0.1, seed=43)
     table = lk.SegmentTable(segs, torch.device("cuda"), total_rows=M)
-    plan = table.split_plan(K)
-    assert plan is not None and len(plan[1]) > 2 and plan[1] == sorted(plan[1], reverse=True)
+    assert table.chunks(K) > 1 and table.chunks(N) > 1
     ps = [0.1, 0.2] if mixed_p else [0.1, 0.1]
     if mixed_p:
         from lorafusion_b200.ops.philox import dropout_threshold

@@ -47,7 +47,8 @@ def _operands(**change):
 
 
 def _fwd(o, s=True):
-    return lk.linear_fwd(o["x"], o["w"], o["a"], o["b"], lk.OneAdapter(M, 1.0, 0.0, 0), o["drop"], s=o["s"] if s else None)
+    return lk.linear_fwd(o["x"], o["w"], o["a"], o["b"], lk.OneAdapter(M, 1.0, 0.0, 0), o["drop"],
+                         s=o["s"] if s else None)
 
 
 def _bwd(o, need_dx=True):

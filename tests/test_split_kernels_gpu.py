@@ -240,7 +240,8 @@ def test_one_call_layer_of_several_adapters_equals_its_building_blocks(K, N, ps)
 
     R, n, M = 64, 3, 640
     info = prepare_multi_lora_batch_info([100, 128, 128, 200], [1, -1, 0, 2], [16, 0, 16, 16],
-                                         [ps[1], 0.0, ps[0], ps[2]], [2.0, 0.0, 0.5, 1.0], device="cuda", seed=(3 << 32) | 5)
+                                         [ps[1], 0.0, ps[0], ps[2]], [2.0, 0.0, 0.5, 1.0], device="cuda",
+                                         seed=(3 << 32) | 5)
     assert info.total_padded_tokens == M
     assert (_pair_scratch_bytes(M, N, K, 0, 0) > 0) == (K == 5000)
     assert (_pair_scratch_bytes(M, K, N, 0, 0) > 0) == (N == 5000)
@@ -337,11 +338,11 @@ def test_rope_with_several_tokens_a_block(M, heads, D):
     assert torch.equal(qkv[:M, heads * D:], before[:M, heads * D:]) and torch.equal(qkv[M:], before[M:])
 
 
-@pytest.mark.parametrize("M,I", [(1, 8), (300, 8), (19001, 8), (9001, 24), (2501, 64), (1187, 1000), (33, 2056), (3, 4104),
-                                 (5, 8200)])
+@pytest.mark.parametrize("M,I", [(1, 8), (300, 8), (19001, 8), (9001, 24), (2501, 64), (1187, 1000), (33, 2056),
+                                 (3, 4104), (5, 8200)])
 def test_swiglu_backward_of_short_and_long_rows(M, I):
-    """Several rows a CTA (long batches of short rows), one row a CTA and rows in pieces; ragged last CTAs and odd vector
-    counts."""
+    """Several rows a CTA (long batches of short rows), one row a CTA and rows in pieces; ragged last CTAs and odd
+    vector counts."""
     from lorafusion_b200.ops import elementwise as ew
 
     gu, d = _rand(M, 2 * I, seed=1), _rand(M, I, seed=2)
@@ -352,10 +353,11 @@ def test_swiglu_backward_of_short_and_long_rows(M, I):
     assert torch.allclose(ew.swiglu_bwd(d, gu).float(), ref, rtol=5e-3, atol=1e-5)
 
 
-@pytest.mark.parametrize("rows,ld,col0,cols", [(700, 30, 3, 24), (1, 12289, 0, 12289), (333, 7, 0, 7), (300, 64, 16, 16)])
+@pytest.mark.parametrize("rows,ld,col0,cols", [(700, 30, 3, 24), (1, 12289, 0, 12289), (333, 7, 0, 7),
+                                               (300, 64, 16, 16)])
 def test_adam_regions_of_any_size(rows, ld, col0, cols):
-    """One update of regions with odd sizes (the last one vectorisable), longer than what the CTAs of a work item take in
-    one go: weights, moments, bf16 copy and cleared gradient; memory around the region untouched."""
+    """One update of regions with odd sizes (the last one vectorisable), longer than what the CTAs of a work item take
+    in one go: weights, moments, bf16 copy and cleared gradient; memory around the region untouched."""
     from lorafusion_b200.ops import elementwise as ew
 
     n, off, st = rows * ld, 12, 8
@@ -427,8 +429,8 @@ def test_multi_lora_of_an_adapter_with_several_segments(p):
     starts = [0, 2176, 2304, 2688]
     M = 2816
     x, w = _rand(M, K, seed=1).requires_grad_(True), _rand(N, K, scale=0.05, seed=2)
-    ab = [(_rand(8, K, scale=0.1, seed=3 + i).requires_grad_(True), _rand(N, 8, scale=0.1, seed=5 + i).requires_grad_(True))
-          for i in range(2)]
+    ab = [(_rand(8, K, scale=0.1, seed=3 + i).requires_grad_(True),
+           _rand(N, 8, scale=0.1, seed=5 + i).requires_grad_(True)) for i in range(2)]
     for i, n in zip(starts, lens):   # (the rows between segments are padding)
         with torch.no_grad():
             x[i + n:(i + n + 127) // 128 * 128] = 0

@@ -43,15 +43,16 @@ def test_last_wave_is_cut_only_where_it_pays():
 
 
 def test_adapters_with_several_segments():
-    """Accepted where the tokens of a segment used to be summed in chunks (fewer than 96 pieces of segment x 128 features,
-    a segment of 2048 tokens): the n-th segments of all adapters form the n-th launch.  Refused otherwise."""
+    """Accepted where the tokens of a segment used to be summed in chunks (fewer than 96 pieces of segment x 128
+    features, a segment of 2048 tokens): the n-th segments of all adapters form the n-th launch.  Refused otherwise."""
     from lorafusion_b200.ops.lora_kernels import SegmentTable, segment_rows
 
     segs = [(0, 0, 128), (1, 128, 384), (0, 384, 2560), (-1, 2560, 2688), (1, 2688, 2816), (0, 2816, 2944)]
-    assert segment_rows(segs) == [(1, 128, 384, 0), (0, 0, 128, 0), (0, 384, 2560, 0), (1, 2688, 2816, 0), (0, 2816, 2944, 0)]
+    assert segment_rows(segs) == [(1, 128, 384, 0), (0, 0, 128, 0), (0, 384, 2560, 0), (1, 2688, 2816, 0),
+                                  (0, 2816, 2944, 0)]
+    staged = torch.tensor([9] * 4 + [v for r in segment_rows(segs) for v in r], dtype=torch.int32)
     for table in (SegmentTable(segs, torch.device("cpu")),
-                  SegmentTable(segs, torch.device("cpu"), staged=(torch.tensor([9] * 4 + [v for r in segment_rows(segs) for v in r],
-                                                                               dtype=torch.int32), 4, 24))):
+                  SegmentTable(segs, torch.device("cpu"), staged=(staged, 4, 24))):
         assert table.repeats
         got = [[tuple(r) for r in rows.tolist()] for rows in table.passes(128 * 19)]
         assert got == [segment_rows(segs)[:2], segment_rows(segs)[2:4], segment_rows(segs)[4:]]
@@ -67,7 +68,8 @@ def test_adapters_with_several_segments():
 
 
 def test_frozen_adapters_may_have_several_segments(monkeypatch):
-    """The input's gradient alone needs no work list: such a batch is not refused, and does not take the one-call path."""
+    """The input's gradient alone needs no work list: such a batch is not refused, and does not take the one-call
+    path."""
     from lorafusion_b200.ops import lora as L
     from lorafusion_b200.ops import lora_kernels as lk
     from lorafusion_b200.ops.batch_info import prepare_multi_lora_batch_info
