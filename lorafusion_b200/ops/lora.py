@@ -149,8 +149,9 @@ def _check_batch(info, rows: int, *stacks: Optional[torch.Tensor]) -> None:
     padded tokens) by the rows they are given, without looking at either's length."""
     if info.tile_adapter is None:
         return
-    if rows > info.total_padded_tokens:
-        raise ValueError(f"{rows} rows, but the batch describes {info.total_padded_tokens}")
+    described = info.tile_adapter.shape[0] * lk.TILE_M
+    if rows > described:
+        raise ValueError(f"{rows} rows, but the batch describes {described}")
     n = min([t.shape[0] for t in stacks if t is not None])
     for adapter, _, _ in info.segments:
         if adapter >= n:

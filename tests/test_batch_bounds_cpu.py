@@ -1,5 +1,7 @@
 """Adapter ids and rows of a batch are checked against the adapters and rows given, before anything is launched."""
 
+from dataclasses import replace
+
 import pytest
 import torch
 
@@ -38,7 +40,8 @@ def test_batches_that_fit_pass(launched, rows):
     _call(_batch(), 3, rows)
     _call(_batch(), 5, rows)
     _call(_batch(ids=(-1, 0)), 1, rows)
-    assert launched == ["fwd", "bwd"] * 3
+    _call(replace(_batch(), total_padded_tokens=0), 3, rows)   # a batch put together by hand: the table counts
+    assert launched == ["fwd", "bwd"] * 4
 
 
 def test_an_adapter_that_is_not_given_is_refused(launched):
