@@ -14,6 +14,7 @@
 // benchmarks_paper/bench_multi_gpu.py:225-230.)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <float.h>
 #include <stdint.h>
 
 #include "../common/ptx.cuh"
@@ -77,7 +78,9 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
   }
 
   const unsigned long long log2e2 = f32x2(1.4426950408889634f, 1.4426950408889634f);
-  float m = -INFINITY, s = 0.f;
+  // The maximum starts below every finite bf16, not at -inf: a logit of -inf (masked) then weighs
+  // 2^-inf = 0, also in front of the first finite one of its thread, where -inf - -inf would be NaN.
+  float m = -FLT_MAX, s = 0.f;
   for (int c0 = threadIdx.x; c0 < nvec; c0 += CE_VECS * THREADS) {
     uint4 raw[CE_VECS];
 #pragma unroll
@@ -114,7 +117,7 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
   }
   // block reduce (max, then rescaled sums)
   float wm = warp_max(m);
-  s = (m == -INFINITY) ? 0.f : s * __expf(m - wm);  // threads that saw no element
+  s *= __expf(m - wm);   // (no finite logit seen: s is 0)
   s = warp_sum2(s);
   if (lane == 0) {
     red_m[warp] = wm;
@@ -125,7 +128,7 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
   for (int i = 1; i < THREADS / 32; ++i) bm = fmaxf(bm, red_m[i]);
   float bs = 0.f;
   for (int i = 0; i < THREADS / 32; ++i)
-    bs += (red_m[i] == -INFINITY) ? 0.f : red_s[i] * __expf(red_m[i] - bm);
+    bs += red_s[i] * __expf(red_m[i] - bm);
   const float lse = bm + __logf(bs);
   const float inv_sum = 1.f / bs, scale = inv_sum * grad_scale;
   const float label_logit = __bfloat162float(lr[min(label, V - 1)]);

@@ -491,3 +491,28 @@ def test_nf4_weights_share_no_code_table():
     for q in (second, third, nf4.quantize_nf4(w)):
         assert torch.equal(q.code256.cpu(), nf4.dynamic_code_8bit()) and torch.equal(nf4.dequantize_nf4(q), want)
     assert not nf4.quantize_nf4(w).code256.is_inference()
+
+
+@pytest.mark.parametrize("V", [9, 1000, 4096, 4100, 32000, 50257])
+@pytest.mark.parametrize("masked", [0.3, 0.97])
+def test_cross_entropy_of_masked_logits(V, masked):
+    """Logits of minus infinity, whole vectors of them in front of the finite ones too, and of the lowest finite value:
+    they have no weight, and no NaN comes of them."""
+    from lorafusion_b200.ops import elementwise as ew
+
+    M, ld = 40, (V + 7) // 8 * 8
+    buf = _rand(M, ld, seed=1, scale=3.0)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    hide = torch.rand(M, ld, generator=g, device="cuda") < masked
+    hide[:, 8:V // 2] = True          # the first vectors of most threads
+    hide[:, 0] = False
+    buf[hide] = float("-inf")
+    buf[M // 2:] = torch.nan_to_num(buf[M // 2:], neginf=torch.finfo(torch.bfloat16).min)
+    lab = torch.zeros(M, dtype=torch.int32, device="cuda")
+    logits = buf[:, :V].float()
+    loss = ew.cross_entropy_inplace(buf[:, :V], lab, 0.5)
+    want = logits.softmax(1)
+    want[:, 0] -= 1
+    # fp32 sums with an approximate exponential (2^-22), gradients rounded to bf16 once
+    assert torch.allclose(loss, logits.logsumexp(1) - logits[:, 0], rtol=1e-5, atol=1e-4)
+    assert torch.allclose(buf[:, :V].float(), want * 0.5, rtol=6e-3, atol=1e-6)
