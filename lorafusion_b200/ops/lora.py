@@ -147,11 +147,10 @@ def _unfused_backward(dy, x, saved, wd, stack, info, need_dx):
 def _check_batch(info, rows: int, *stacks: Optional[torch.Tensor]) -> None:
     """The kernels index the adapters of ``stacks`` by the ids of the batch, and its tile table (one entry for 128
     padded tokens) by the rows they are given, without looking at either's length."""
-    if info.tile_adapter is None:
+    if info.tile_adapter is None and info.segment_table is None:
         return
-    described = info.tile_adapter.shape[0] * lk.TILE_M
-    if rows > described:
-        raise ValueError(f"{rows} rows, but the batch describes {described}")
+    if info.tile_adapter is not None and rows > info.tile_adapter.shape[0] * lk.TILE_M:
+        raise ValueError(f"{rows} rows, but the batch describes {info.tile_adapter.shape[0] * lk.TILE_M}")
     n = min([t.shape[0] for t in stacks if t is not None])
     for adapter, _, _ in info.segments:
         if adapter >= n:
@@ -197,12 +196,12 @@ def lora_linear_backward(dy: torch.Tensor, x: torch.Tensor, s: Optional[torch.Te
     if stack is None or info is None or s is None:
         return lk.base_lora_dx(dy, wd, None, None, tile_adapter=None) if need_dx else None
     drop = info.dropout_spec(stream_id, training)
-    if not isinstance(wd, NF4Weight) and (info.tile_adapter is None or not info.segment_table.repeats):
+    if not isinstance(wd, NF4Weight) and (info.segment_table is None or not info.segment_table.repeats):
         return lk.linear_bwd(dy, x, s, wd if need_dx else None, stack.a, stack.b, info, drop, stack.da, stack.db,
                              need_dx)
     ds = lk.lora_ds(dy, stack.b, tile_adapter=info.tile_adapter, adapter_scale=info.adapter_scale,
                     scale=getattr(info, "scale", 1.0))
-    segs = info.segment_table if info.tile_adapter is not None else \
+    segs = info.segment_table if info.segment_table is not None else \
         lk.SegmentTable(info.segments, dy.device, total_rows=dy.shape[0])
     if stack.db is not None:
         lk.lora_db(dy, s, segs, stack.db)

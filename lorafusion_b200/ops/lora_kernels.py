@@ -285,6 +285,7 @@ class OneAdapter:
     seed: int
     tile_adapter = None
     adapter_scale = None
+    segment_table = None
 
     def __post_init__(self):
         dropout_threshold(self.p)   # refuses what is no rate
@@ -356,6 +357,7 @@ def _linear_args(M: int, K: int, N: int, R: int, n: int, info, drop: DropoutSpec
         dropmix_bn=DROPMIX_BN, scale=getattr(info, "scale", 1.0), **fields)
     if info.tile_adapter is not None:
         args.tile_adapter = info.tile_adapter.data_ptr()
+    if info.adapter_scale is not None:
         args.adapter_scale = info.adapter_scale.data_ptr()
     if drop.active:
         args.dropout = 1
@@ -435,7 +437,7 @@ def linear_bwd(dy: torch.Tensor, x: Optional[torch.Tensor], s: Optional[torch.Te
         dx_ptr = dx.data_ptr()
     if da is None and db is None:
         seg_rows, num_segs, split_da, split_db = None, 0, 1, 1
-    elif info.tile_adapter is None:
+    elif info.segment_table is None:
         seg_rows, num_segs = None, 1
         split_da, split_db = (reduction_split((f + TILE_M - 1) // TILE_M, (M + 63) // 64) for f in (K, N))
     else:

@@ -50,6 +50,8 @@ def test_an_adapter_that_is_not_given_is_refused(launched):
             _call(_batch(), 2, 384)
     with pytest.raises(ValueError, match="adapter"):
         _call(_batch(), 3, 384, da=torch.zeros(2, R, K))
+    with pytest.raises(ValueError, match="adapter"):   # no tile table: the work list of the gradients names it
+        _call(replace(_batch(), tile_adapter=None), 2, 384)
     # its segment holds no tokens: no kernel meets the id
     _call(_batch(ids=(0, 2), lens=(100, 0)), 1, 128)
     assert launched == ["fwd"] + ["fwd", "bwd"]

@@ -145,3 +145,24 @@ def test_offsets_of_a_sharded_mask_reach_the_kernels(calls):
     _fwd(_operands(drop=drop), s=False)
     _bwd(_operands(drop=drop))
     assert [(c.row_offset, c.col_offset) for c in calls] == [(384, 4096)] * 2
+
+
+def test_batches_put_together_by_hand(calls):
+    """Without a tile table every token belongs to adapter 0, whose scale and segments count all the same; without scales
+    they are one."""
+    from dataclasses import replace
+
+    from lorafusion_b200.ops.batch_info import prepare_multi_lora_batch_info
+
+    info = prepare_multi_lora_batch_info([M], [0], [16], [0.0], [2.0], device="cpu")
+    o = _operands()
+    for batch in (replace(info, tile_adapter=None), replace(info, adapter_scale=None)):
+        lk.linear_fwd(o["x"], o["w"], o["a"], o["b"], batch, o["drop"])
+        lk.linear_bwd(o["dy"], o["x"], o["s"], o["w"], o["a"], o["b"], batch, o["drop"], o["da"], o["db"], True)
+    ptr = lambda t: t.data_ptr()  # noqa: E731
+    for c in calls[:2]:
+        assert c.tile_adapter is None and c.adapter_scale == ptr(info.adapter_scale)
+    for c in calls[2:]:
+        assert c.tile_adapter == ptr(info.tile_adapter) and c.adapter_scale is None and c.scale == 1.0
+    for c in calls[1::2]:
+        assert c.seg_rows == ptr(info.segment_table.device_rows()) and c.num_segs == 1
