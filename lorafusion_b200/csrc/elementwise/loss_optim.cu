@@ -117,7 +117,7 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
   }
   // block reduce (max, then rescaled sums)
   float wm = warp_max(m);
-  s *= __expf(m - wm);   // (no finite logit seen: s is 0)
+  s = m == -FLT_MAX ? 0.f : s * __expf(m - wm);  // threads that saw no finite logit
   s = warp_sum2(s);
   if (lane == 0) {
     red_m[warp] = wm;

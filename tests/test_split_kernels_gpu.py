@@ -516,3 +516,13 @@ def test_cross_entropy_of_masked_logits(V, masked):
     # fp32 sums with an approximate exponential (2^-22), gradients rounded to bf16 once
     assert torch.allclose(loss, logits.logsumexp(1) - logits[:, 0], rtol=1e-5, atol=1e-4)
     assert torch.allclose(buf[:, :V].float(), want * 0.5, rtol=6e-3, atol=1e-6)
+
+
+def test_cross_entropy_of_a_single_nan_in_a_thread():
+    """A thread that sees nothing but a NaN logit adds nothing to the row's sum, as ever: only its own column is NaN."""
+    from lorafusion_b200.ops import elementwise as ew
+
+    buf = _rand(3, 8, seed=2)
+    buf[1, 4] = float("nan")
+    loss = ew.cross_entropy_inplace(buf[:, :7], torch.zeros(3, dtype=torch.int32, device="cuda"), 1.0)
+    assert loss.isfinite().all() and buf.isnan().nonzero().tolist() == [[1, 4]]
