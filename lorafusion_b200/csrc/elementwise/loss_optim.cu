@@ -128,7 +128,7 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__
   for (int i = 1; i < THREADS / 32; ++i) bm = fmaxf(bm, red_m[i]);
   float bs = 0.f;
   for (int i = 0; i < THREADS / 32; ++i)
-    bs += red_s[i] * __expf(red_m[i] - bm);
+    bs += (red_m[i] == -FLT_MAX) ? 0.f : red_s[i] * __expf(red_m[i] - bm);
   const float lse = bm + __logf(bs);
   const float inv_sum = 1.f / bs, scale = inv_sum * grad_scale;
   const float label_logit = __bfloat162float(lr[min(label, V - 1)]);
